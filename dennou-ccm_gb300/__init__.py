@@ -482,7 +482,8 @@ def spec_apply_dev(nmax, op, spec_in, spec_out, batch, stream=None):
 class ShtPlan:
     """w_Initial(nMax, iMax, jMax) equivalent: a transform plan on the GPU.
 
-    precision SHT_FP64 (CUDA cores) or SHT_MIXED (tcgen05 BF16x3 Legendre,
+    precision SHT_FP64 (FP64 accuracy; Legendre by exact digit products on the
+    tensor cores) or SHT_MIXED (tcgen05 BF16x3 Legendre,
     FP32 FFT).  Spectra are complex128 [batch, ncoef] (m-major), grids
     float64 [batch, jmax, imax]."""
 

@@ -1,0 +1,653 @@
+// FP64 Legendre transforms on the 5th-generation tensor cores (tcgen05),
+// exact products of integer digits with the accuracy of FP64 arithmetic.
+//
+// The FP64 pipe of this GPU does one FMA for every 64 of the FP32 pipe
+// (1.05 TFLOP/s measured), and the contraction took 80 % of the plain FP64
+// transforms as an FP64 FMA loop (T341 x 192 field-levels: synthesis 10.4
+// ms, analysis 13.5 ms; T85 x 128: 209 and 340 us; with the kernels below
+// 0.78, 0.76 ms, 50 and 43 us, packs included).  Here every operand is
+// split into seven 9-bit digits (digits.cuh: the scheme of K. Ozaki, T.
+// Ogita, S. Oishi, S. Rump, "Error-free transformations of matrix
+// multiplication", Numer. Algorithms 59 (2012), with integer digits), and
+// the products d_i(a) d_j(b) of equal weight, s = i + j = 2 .. 8, are
+// summed in one FP32 accumulator per s: integers below 2^24, so the sums
+// are exact.  28 MMAs take the place of an FP64 FMA; the products left out
+// (s >= 9) are below 2^-60 of (largest |a|) (largest |b|), well under the
+// rounding errors of an FP64 sum.
+//
+// Exactness: an accumulator takes at most DG_KB = 128 values of K before it
+// is drained, so levels s = 2, 3 (one and two products of at most 2^16 a
+// value) stay within 2^24 whatever the data; levels 4 and 5 do for any data
+// because the table's lower digits average 128 in magnitude; from level 6
+// on (below 2^-52 of the largest product) a rounding would not be seen.
+//
+// As the mixed path (legendre_tc.cu) the contractions run per zonal
+// wavenumber m and parity p (n - m even / odd), folded by equatorial symmetry:
+//   inverse  D_p[c][jj] = sum_k S_p[c][k] Pbar_p[jj][k],
+//            F(jn) = D_0 + D_1, F(js) = D_0 - D_1 (added as integers);
+//   forward  D_p[c][k]  = sum_jj X_p[c][jj] ((w/2) Pbar)_p[k][jj].
+//
+// Both operands lie in global memory as the shared-memory image of a tile
+// (K-major rows of 32 values = 64 bytes, 64-byte swizzle), so that a stage
+// is filled by a few untiled bulk copies:
+//   A  [ct][chunk][7][128 rows c][32], written by the pack kernels, chunk =
+//      32 values of K of one (m, p);
+//   B  [m][p][nt][q][7][rows][32], built once per plan.
+// The digit slices of B lie one after the other in the image, so one MMA
+// multiplies slice i of A with several consecutive slices j of B (N = rows
+// x slices, up to 256 columns), whose results fall into consecutive
+// accumulators s = i + j: a slice of A is read from shared memory once for
+// all of them.
+//
+// A work item is (m, 128 columns c, TN rows of N).  Warp 0 copies, warp 1
+// allocates TMEM and issues the MMAs, warps 2-9 drain the accumulators
+// (7 TMEM columns an output, integer arithmetic, one store).  Every wait is
+// bounded, as in legendre_tc.cu.
+#include <math.h>
+#include <string.h>
+
+#include "digits.cuh"
+#include "sht_plan.cuh"
+#include "tcgen05.cuh"
+
+namespace dccm {
+namespace sht {
+
+constexpr int DG_CHUNK = 32;                                   // K of a stage
+constexpr int DG_KB = 4;                                       // chunks an accumulator takes (128 values of K)
+constexpr int DG_ROW = 2 * DG_CHUNK;                           // bytes of a K-major row of a chunk
+constexpr int DG_A_SLICE = 128 * DG_ROW;                       // 8 KB
+constexpr int DG_A_BYTES = DG_SLICES * DG_A_SLICE;             // 56 KB
+constexpr int DG_EPI_WARPS = 8;
+constexpr int DG_THREADS = 64 + 32 * DG_EPI_WARPS;
+constexpr size_t DG_WORK_CAP = (size_t)4 << 30;                // A images of one launch
+template <int TN> struct DgShape {
+  static constexpr int B_BYTES = DG_SLICES * TN * DG_ROW;
+  static constexpr int STAGE = DG_A_BYTES + B_BYTES;
+  static constexpr int NSTAGE = TN == 32 ? 3 : 2;
+  static constexpr int NACC = TN == 32 ? 2 : 1;                // accumulator sets (7 TN columns each)
+  static constexpr int ACC_COLS = TN == 32 ? 256 : 512;
+  static constexpr int SMEM = 1024 + NSTAGE * STAGE + 256;
+};
+
+struct DgMInfo {
+  long long tab[2];  // first table tile of (m, p), bytes
+  int ch[2];         // first A chunk of (m, p)
+  int nq[2];         // K chunks
+  int kv[2];         // valid K
+  int nv[2];         // valid N
+  int nr[2];         // N rounded up to 16
+  long long eb[2];   // first row-scale entry: inverse eb[0] + jj; forward idx(m, m) (entry idx(m, n))
+};
+
+struct DgArgs {
+  int N, Jh, batch;
+  int c0;            // first column of this launch
+  int nct;           // column tiles
+  int nitems;        // items per column tile
+  int nchunk;        // A chunks per column tile
+  int ldea;          // row length of ea
+  long long ncoef;
+  const DgMInfo *mi;
+  const int2 *items;           // (m, nt)
+  const unsigned char *A, *B;
+  const int *ea;               // scale exponents of A: inverse [m][c], forward [2m+p][c]
+  const short *eb;             // scale exponents of the table rows
+  double *out;                 // F or spectra
+  int *err;
+  unsigned long long wait_ns;
+  int withhold;
+};
+
+__device__ __forceinline__ uint64_t dg_desc(uint32_t addr) {
+  // K-major, 64-byte swizzle, 8-row groups 512 bytes apart
+  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) | ((uint64_t)1 << 46) |
+         ((uint64_t)4 << 61);
+}
+
+// byte offset of 16-byte unit u (8 values of K) of row r in a swizzled slice
+__host__ __device__ __forceinline__ int dg_unit(int r, int u) { return r * DG_ROW + ((u ^ ((r >> 1) & 3)) << 4); }
+
+__device__ __forceinline__ int dg_item(int k) {  // as cta_item: rounds in alternating directions
+  const int G = (int)gridDim.x, b = (int)blockIdx.x;
+  return (k & 1) ? (k + 1) * G - 1 - b : k * G + b;
+}
+
+template <int TN, int DIR>
+__global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid_constant__ DgArgs a) {
+  using Sh = DgShape<TN>;
+  constexpr int NSTAGE = Sh::NSTAGE, NACC = Sh::NACC;
+  extern __shared__ __align__(1024) unsigned char smem_dyn[];
+  unsigned char *stage = reinterpret_cast<unsigned char *>(
+      (reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(stage + NSTAGE * Sh::STAGE);
+  uint64_t *full = bars, *empty = bars + NSTAGE, *accf = bars + 2 * NSTAGE, *acce = accf + NACC;
+  uint64_t *drain = bars + 15;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 16);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 17);
+
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NSTAGE; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int s = 0; s < NACC; ++s) {
+      mbar_init(&accf[s], 1);
+      mbar_init(&acce[s], 32 * DG_EPI_WARPS);
+    }
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    mbar_init_fence();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const int nitems = a.nct * a.nitems;
+  pdl_wait();
+  pdl_trigger();
+
+  if (warp == 0) {
+    // -------------------------------------------------------- copies
+    if (lane == 0 && !a.withhold) {
+      int g = 0;
+      bool ok = true;
+      for (int k = 0, it = dg_item(0); it < nitems && ok; it = dg_item(++k)) {
+        const int2 w = a.items[it / a.nct];
+        const int ct = it % a.nct, m = w.x, nt = w.y;
+        const DgMInfo &mi = a.mi[m];
+        // rows of the column tile that hold data (whole groups of 8)
+        const int rows = min(128, ((2 * a.batch - a.c0 - ct * 128) + 7) & ~7);
+        for (int p = 0; p < 2 && ok; ++p) {
+          if (nt * TN >= mi.nr[p]) continue;
+          const int ntw = min(TN, mi.nr[p] - nt * TN);
+          const unsigned char *Bt =
+              a.B + mi.tab[p] + (long long)nt * TN * mi.nq[p] * (DG_SLICES * DG_ROW);
+          for (int q = 0; q < mi.nq[p]; ++q, ++g) {
+            const int s = g % NSTAGE;
+            if (!mbar_wait(&empty[s], ((g / NSTAGE) & 1) ^ 1, a.err, abort_flag, 1, a.wait_ns)) { ok = false; break; }
+            unsigned char *As = stage + s * Sh::STAGE;
+            const unsigned char *Ag = a.A + ((long long)ct * a.nchunk + mi.ch[p] + q) * DG_A_BYTES;
+            const uint32_t bb = (uint32_t)(DG_SLICES * DG_ROW * ntw);
+            mbar_arrive_tx(&full[s], (uint32_t)(DG_SLICES * DG_ROW * rows) + bb);
+            bulk_load(As + DG_A_BYTES, Bt + (long long)q * bb, bb, &full[s]);
+            if (rows == 128) {
+              bulk_load(As, Ag, DG_A_BYTES, &full[s]);
+            } else {
+              for (int i = 0; i < DG_SLICES; ++i)
+                bulk_load(As + i * DG_A_SLICE, Ag + i * DG_A_SLICE, (uint32_t)(rows * DG_ROW), &full[s]);
+            }
+          }
+        }
+      }
+      if (!ok) {  // let the copies in flight land before the CTA's shared memory goes
+        for (int h = g > NSTAGE ? g - NSTAGE : 0; h < g; ++h)
+          mbar_wait_bounded(&full[h % NSTAGE], (h / NSTAGE) & 1, nullptr, 0);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ---------------------------------------------------------- MMA
+    if (lane == 0) {
+      int g = 0, seg = 0;
+      bool ok = true;
+      for (int k = 0, it = dg_item(0); it < nitems && ok; it = dg_item(++k)) {
+        const int2 w = a.items[it / a.nct];
+        const int m = w.x, nt = w.y;
+        const DgMInfo &mi = a.mi[m];
+        for (int p = 0; p < 2 && ok; ++p) {
+          if (nt * TN >= mi.nr[p]) continue;
+          const int ntw = min(TN, mi.nr[p] - nt * TN);
+          const int per = 256 / ntw;  // slices of B an MMA can take
+          for (int q0 = 0; q0 < mi.nq[p] && ok; q0 += DG_KB, ++seg) {
+            const int set = seg % NACC;
+            if (!mbar_wait(&acce[set], ((seg / NACC) & 1) ^ 1, a.err, abort_flag, 2, a.wait_ns)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t acc = tmem + set * Sh::ACC_COLS;
+            int first = 0;  // 0 until the accumulators have been written
+            for (int q = q0; q < min(mi.nq[p], q0 + DG_KB); ++q, ++g) {
+              const int s = g % NSTAGE;
+              if (!mbar_wait(&full[s], (g / NSTAGE) & 1, a.err, abort_flag, 3, a.wait_ns)) { ok = false; break; }
+              tc_fence_after();
+              const uint32_t As = smem_u32(stage + s * Sh::STAGE), Bs = As + DG_A_BYTES;
+              const int ks = min(2, (mi.kv[p] - q * DG_CHUNK + 15) / 16);
+              for (int kk = 0; kk < ks; ++kk) {
+#pragma unroll
+                for (int i = 0; i < DG_SLICES; ++i) {
+                  const uint64_t da = dg_desc(As + i * DG_A_SLICE + kk * 32);
+                  // slices j = 0 .. 6 - i of B into accumulators i + j
+                  for (int j = 0; j < DG_SLICES - i; j += per) {
+                    const int n = min(per, DG_SLICES - i - j);
+                    mma_bf16(acc + (i + j) * ntw, da, dg_desc(Bs + j * ntw * DG_ROW + kk * 32),
+                             idesc_f16kind(n * ntw, 0, 1), first | i);
+                  }
+                }
+                first = 1;
+              }
+              mma_commit(&empty[s]);
+            }
+            if (ok) mma_commit(&accf[set]);
+          }
+        }
+      }
+      if (!ok) {  // MMAs in flight end before the TMEM is freed
+        mma_commit(drain);
+        mbar_wait_bounded(drain, 0, nullptr, 0);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ----------------------------------------------------- epilogue
+    constexpr int HC = TN / 16;               // groups of 8 columns a thread drains
+    const int quad = warp & 3, half = (warp - 2) >> 2;
+    const int row = quad * 32 + lane;
+    const int C2B = 2 * a.batch;
+    int seg = 0;
+    bool dead = false;
+    for (int k = 0, it = dg_item(0); it < nitems && !dead; it = dg_item(++k)) {
+      const int2 w = a.items[it / a.nct];
+      const int ct = it % a.nct, m = w.x, nt = w.y;
+      const DgMInfo &mi = a.mi[m];
+      const int c = a.c0 + ct * 128 + row;
+      const bool live = c < C2B;
+      // inverse: both parities' sums; forward: the current parity's
+      Dg96 sum[DIR == 0 ? 2 : 1][HC][8];
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        Dg96(&S)[HC][8] = sum[DIR == 0 ? p : 0];
+#pragma unroll
+        for (int h = 0; h < HC; ++h)
+#pragma unroll
+          for (int x = 0; x < 8; ++x) S[h][x] = Dg96{0, 0, 0};
+        if (nt * TN >= mi.nr[p]) continue;
+        const int ntw = min(TN, mi.nr[p] - nt * TN);
+        for (int q0 = 0; q0 < mi.nq[p]; q0 += DG_KB, ++seg) {
+          const int set = seg % NACC;
+          if (!mbar_wait(&accf[set], (seg / NACC) & 1, a.err, abort_flag, 4, a.wait_ns)) {
+            dead = true;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t tb = tmem + ((uint32_t)(quad * 32) << 16) + set * Sh::ACC_COLS;
+#pragma unroll
+          for (int h = 0; h < HC; ++h) {
+            const int j0 = 16 * h + 8 * half;
+            if (j0 < ntw) {
+              uint32_t r[DG_SLICES][8];
+#pragma unroll
+              for (int s = 0; s < DG_SLICES; ++s) tmem_ld8_nw(tb + s * ntw + j0, r[s]);
+              tmem_wait_ld();
+#pragma unroll
+              for (int x = 0; x < 8; ++x) {
+                int v[DG_SLICES];
+#pragma unroll
+                for (int s = 0; s < DG_SLICES; ++s) v[s] = __float2int_rn(__uint_as_float(r[s][x]));
+                dg_add(S[h][x], (long long)v[0] * 262144 + ((long long)v[1] * 512 + v[2]),
+                       ((long long)v[3] * 512 + v[4]) * 262144 + ((long long)v[5] * 512 + v[6]));
+              }
+            }
+          }
+          tc_fence_before();
+          mbar_arrive(&acce[set]);
+        }
+        if (dead) break;
+        if (DIR == 1 && live) {
+          // column k of the tile is n = m + p + 2 (nt TN + k)
+          const int E = a.ea[(long long)(2 * m + p) * a.ldea + c];
+#pragma unroll
+          for (int h = 0; h < HC; ++h)
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+              const int kk = nt * TN + 16 * h + 8 * half + x;
+              if (kk < mi.nv[p] && 16 * h + 8 * half < ntw) {
+                const long long id = mi.eb[p] + p + 2 * kk;
+                double v = dg_to_double(S[h][x], E - 1022 + a.eb[id] - 70);
+                if (E >= 2047) v = __longlong_as_double(0x7FF8000000000000ll);
+                a.out[((long long)(c >> 1) * a.ncoef + id) * 2 + (c & 1)] = (m == 0 && (c & 1)) ? 0.0 : v;
+              }
+            }
+        }
+      }
+      if (DIR == 0 && !dead && live) {
+        const int ntw = min(TN, mi.nr[0] - nt * TN);
+        const int E = a.ea[(long long)m * a.ldea + c];
+        double *Fm = a.out + (long long)m * 2 * a.Jh * C2B + c;
+#pragma unroll
+        for (int h = 0; h < HC; ++h)
+#pragma unroll
+          for (int x = 0; x < 8; ++x) {
+            const int jj = nt * TN + 16 * h + 8 * half + x;
+            if (jj < a.Jh && 16 * h + 8 * half < ntw) {
+              const int ex = E - 1022 + a.eb[mi.eb[0] + jj] - 70;
+              double fn = dg_to_double(dg_sum(sum[0][h][x], sum[DIR == 0][h][x]), ex);
+              double fs = dg_to_double(dg_diff(sum[0][h][x], sum[DIR == 0][h][x]), ex);
+              if (E >= 2047) fn = fs = __longlong_as_double(0x7FF8000000000000ll);
+              Fm[(long long)(a.Jh + jj) * C2B] = fn;
+              Fm[(long long)(a.Jh - 1 - jj) * C2B] = fs;
+            }
+          }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ packs
+// Spectra -> A images.  G lanes handle one (m, field-level b): they find the
+// largest magnitude of its coefficients n = m .. N (one scale for both
+// parities and for re and im), then write the digits; a lane takes 8
+// coefficients of one parity (n0 + p, n0 + p + 2, ...).  Whole chunks are
+// written, zeros past the last coefficient.
+template <int G>
+__global__ void __launch_bounds__(256)
+dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const double2 *__restrict__ spec, int b0, int nb,
+             int nchunk, unsigned char *__restrict__ A, int *__restrict__ ea, int ldea) {
+  pdl_wait();
+  pdl_trigger();
+  const int m = blockIdx.y;
+  const int gl = threadIdx.x % G;
+  const int bl = blockIdx.x * (256 / G) + threadIdx.x / G;  // field-level of this launch
+  const bool live = bl < nb;
+  const int b = b0 + (live ? bl : 0);
+  const DgMInfo &mi = mi_[m];
+  const double2 *src = spec + (long long)b * ncoef + idx_mn(N, m, m);
+  const int nu = 4 * max(mi.nq[0], mi.nq[1]);  // units of 8 a parity, both parities side by side
+  unsigned mx = 0;
+  double2 v[8];
+  for (int t = gl; t < 2 * nu; t += G) {
+    const int n0 = m + 16 * (t >> 1) + (t & 1);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      v[e] = live && n0 + 2 * e <= N ? __ldg(src + (n0 - m) + 2 * e) : make_double2(0.0, 0.0);
+      mx = max(mx, max(dg_mag(v[e].x), dg_mag(v[e].y)));
+    }
+  }
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (!live) return;
+  const int E = dg_exp(mx);
+  const int c = 2 * bl;  // column within this launch
+  const int ct = c / 128, row = c % 128;
+  if (gl == 0) *reinterpret_cast<int2 *>(ea + (long long)m * ldea + 2 * b) = make_int2(E, E);
+  const bool keep = 2 * nu <= G;  // the values are still in registers
+  for (int t = gl; t < 2 * nu; t += G) {
+    const int p = t & 1, u = t >> 1;
+    if (u >= 4 * mi.nq[p]) continue;
+    const int n0 = m + 16 * u + p;
+    if (!keep) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = n0 + 2 * e <= N ? __ldg(src + (n0 - m) + 2 * e) : make_double2(0.0, 0.0);
+    }
+    unsigned char *img = A + ((long long)ct * nchunk + mi.ch[p] + (u >> 2)) * DG_A_BYTES;
+    unsigned long long q[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) q[e] = dg_fixed(v[e].x, E);
+    dg_store8(img + dg_unit(row, u & 3), DG_A_SLICE, q);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) q[e] = dg_fixed(v[e].y, E);
+    dg_store8(img + dg_unit(row + 1, u & 3), DG_A_SLICE, q);
+  }
+}
+
+// Folded Fourier coefficients G[m][p][jj][c] -> A images, one scale per
+// (m, p, c).  A warp takes 8 columns x 4 units of 8 latitudes (one chunk):
+// its loads are 64-byte runs along c, its stores whole rows of an image.
+// WQ warps share the chunks of 8 columns.
+template <int WQ>
+__global__ void __launch_bounds__(256)
+dg_pack_four(const DgMInfo *__restrict__ mi_, int Jh, int C2B, int c0, int nc, const double *__restrict__ Gf, int nchunk,
+             unsigned char *__restrict__ A, int *__restrict__ ea, int ldea) {
+  __shared__ unsigned smx[8][8];
+  pdl_wait();
+  pdl_trigger();
+  const int mp = blockIdx.y, m = mp >> 1, p = mp & 1;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int c8 = lane & 7, u = lane >> 3;
+  const int cl = (blockIdx.x * (8 / WQ) + warp / WQ) * 8 + c8;
+  const bool live = cl < nc;
+  const DgMInfo &mi = mi_[m];
+  if (mi.nv[p] <= 0) return;  // this parity has no coefficient (uniform over the block)
+  const int nq = mi.nq[p];
+  const double *src = Gf + (long long)mp * Jh * C2B + c0 + (live ? cl : 0);
+  double v[8];
+  unsigned mx = 0;
+  for (int q = warp % WQ; q < nq; q += WQ) {
+    const int j0 = q * DG_CHUNK + 8 * u;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = live && j0 + e < Jh ? __ldg(src + (long long)(j0 + e) * C2B) : 0.0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) mx = max(mx, dg_mag(v[e]));
+  }
+  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+  if (WQ > 1) {
+    if (u == 0) smx[warp][c8] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < WQ; ++k) mx = max(mx, smx[warp / WQ * WQ + k][c8]);
+  }
+  if (!live) return;
+  const int E = dg_exp(mx);
+  if (u == 0 && warp % WQ == 0) ea[(long long)mp * ldea + c0 + cl] = E;
+  const int ct = cl / 128, row = cl % 128;
+  const bool keep = nq <= WQ;
+  for (int q = warp % WQ; q < nq; q += WQ) {
+    const int j0 = q * DG_CHUNK + 8 * u;
+    if (!keep) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = j0 + e < Jh ? __ldg(src + (long long)(j0 + e) * C2B) : 0.0;
+    }
+    unsigned char *img = A + ((long long)ct * nchunk + mi.ch[p] + q) * DG_A_BYTES;
+    unsigned long long qv[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) qv[e] = dg_fixed(v[e], E);
+    dg_store8(img + dg_unit(row, u), DG_A_SLICE, qv);
+  }
+}
+
+// ------------------------------------------------------------------ tables
+// Scale exponent of every table row: inverse rows (m, jj) over all n;
+// forward rows (m, n) over all latitudes of (w/2) Pbar.  The stored value is
+// E - 1022: the row's entries are below 2^eb.  One warp per row.
+__global__ void dg_row_scale(int dir, int N, int Jh, const double *__restrict__ pnm, const double *__restrict__ w,
+                             long long nrows, short *__restrict__ eb) {
+  const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (r >= nrows) return;
+  unsigned mx = 0;
+  if (dir == 0) {
+    const int m = (int)(r / Jh), jj = (int)(r % Jh);
+    for (int n = m + lane; n <= N; n += 32) mx = max(mx, dg_mag(pnm[idx_mn(N, m, n) * Jh + jj]));
+  } else {
+    for (int jj = lane; jj < Jh; jj += 32) mx = max(mx, dg_mag((0.5 * w[Jh + jj]) * pnm[r * Jh + jj]));
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) eb[r] = (short)(dg_exp(mx) - 1022);
+}
+
+// Table tiles: thread = (m, p, row of N, unit of 8 along K).
+__global__ void __launch_bounds__(256)
+dg_build(int dir, int N, int Jh, int TN, const DgMInfo *__restrict__ mi_, const double *__restrict__ pnm,
+         const double *__restrict__ w, const short *__restrict__ eb, unsigned char *__restrict__ B) {
+  const int m = blockIdx.y, p = blockIdx.z;
+  const DgMInfo &mi = mi_[m];
+  const int nu = 4 * mi.nq[p];
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < mi.nr[p] * nu; t += gridDim.x * blockDim.x) {
+    // neighbouring threads along the table's contiguous latitude index
+    const int r = dir == 0 ? t % mi.nr[p] : t / nu, ug = dir == 0 ? t / mi.nr[p] : t % nu;
+    unsigned long long q[8];
+    int E = 1;
+    if (r < mi.nv[p]) E = eb[dir == 0 ? mi.eb[0] + r : mi.eb[p] + p + 2 * r] + 1022;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int k = 8 * ug + e;
+      double x = 0.0;
+      if (r < mi.nv[p] && k < mi.kv[p]) {
+        if (dir == 0) x = pnm[idx_mn(N, m, m + p + 2 * k) * Jh + r];
+        else x = (0.5 * w[Jh + k]) * pnm[idx_mn(N, m, m + p + 2 * r) * Jh + k];
+      }
+      q[e] = dg_fixed(x, E);
+    }
+    const int nt = r / TN, ntw = min(TN, mi.nr[p] - nt * TN);
+    unsigned char *tile = B + mi.tab[p] +
+                          ((long long)nt * TN * mi.nq[p] + (long long)(ug >> 2) * ntw) * (DG_SLICES * DG_ROW);
+    dg_store8(tile + dg_unit(r % TN, ug & 3), (size_t)ntw * DG_ROW, q);
+  }
+}
+
+// ------------------------------------------------------------------ host
+constexpr int DG_TN = 32;
+
+static int build_dir(Plan &P, int dir, DgTable &T) {
+  const int N = P.N, Jh = P.Jh;
+  std::vector<DgMInfo> mi(N + 1);
+  std::vector<int2> items;
+  long long tab = 0;
+  int ch = 0;
+  for (int m = 0; m <= N; ++m) {
+    DgMInfo &M = mi[m];
+    int nrmax = 0;
+    for (int p = 0; p < 2; ++p) {
+      const int cnt = count_np(N, m, p);
+      M.kv[p] = cnt > 0 ? (dir == 0 ? cnt : Jh) : 0;
+      M.nv[p] = cnt > 0 ? (dir == 0 ? Jh : cnt) : 0;
+      M.nq[p] = (M.kv[p] + DG_CHUNK - 1) / DG_CHUNK;
+      M.nr[p] = (M.nv[p] + 15) / 16 * 16;
+      M.tab[p] = tab;
+      M.ch[p] = ch;
+      M.eb[p] = dir == 0 ? (long long)m * Jh : idx_mn(N, m, m);
+      tab += (long long)M.nr[p] * M.nq[p] * (DG_SLICES * DG_ROW);
+      ch += M.nq[p];
+      nrmax = M.nr[p] > nrmax ? M.nr[p] : nrmax;
+    }
+    for (int nt = 0; nt * DG_TN < nrmax; ++nt) items.push_back(make_int2(m, nt));
+  }
+  T.nchunk = ch;
+  T.nitems = (int)items.size();
+  const long long nrows = dir == 0 ? (long long)(N + 1) * Jh : P.ncoef;
+  // one allocation a direction: metadata and items (one copy), row scales, tiles
+  const size_t mi_b = mi.size() * sizeof(DgMInfo), it_b = items.size() * sizeof(int2);
+  const size_t head = (mi_b + it_b + 255) / 256 * 256, eb_b = ((size_t)nrows * sizeof(short) + 255) / 256 * 256;
+  std::vector<unsigned char> h(head, 0);
+  memcpy(h.data(), mi.data(), mi_b);
+  memcpy(h.data() + mi_b, items.data(), it_b);
+  DCCM_CUDA(cudaMalloc(&T.d_mem, head + eb_b + (size_t)tab));
+  DCCM_CUDA(cudaMemcpy(T.d_mem, h.data(), head, cudaMemcpyHostToDevice));
+  unsigned char *base = (unsigned char *)T.d_mem;
+  T.d_mi = base;
+  T.d_items = (int2 *)(base + mi_b);
+  T.d_eb = (short *)(base + head);
+  T.d_tab = base + head + eb_b;
+  dg_row_scale<<<(unsigned)((nrows + 7) / 8), 256>>>(dir, N, Jh, P.d_pnm, P.d_w, nrows, T.d_eb);
+  DCCM_LAUNCH_CHECK();
+  dg_build<<<dim3(16, N + 1, 2), 256>>>(dir, N, Jh, DG_TN, (const DgMInfo *)T.d_mi, P.d_pnm, P.d_w, T.d_eb,
+                                        (unsigned char *)T.d_tab);
+  DCCM_LAUNCH_CHECK();
+  return DCCM_OK;
+}
+
+// Tables of both directions and the A images.  The images of one launch are
+// bounded (DG_WORK_CAP); a larger batch takes several launches.
+int build_digits(Plan &P) {
+  DCCM_TRY(build_dir(P, 0, P.dinv));
+  DCCM_TRY(build_dir(P, 1, P.dfwd));
+  const int nch = P.dinv.nchunk > P.dfwd.nchunk ? P.dinv.nchunk : P.dfwd.nchunk;
+  const size_t per = (size_t)nch * DG_A_BYTES;
+  const int nct = (2 * P.max_batch + 127) / 128;
+  size_t cap = DG_WORK_CAP / per;
+  if (cap < 1) cap = 1;
+  P.dg_ct = (size_t)nct < cap ? nct : (int)cap;
+  P.dg_ldea = 2 * P.max_batch;
+  const size_t dig = per * P.dg_ct;
+  DCCM_CUDA(cudaMalloc(&P.d_dig, dig + (size_t)2 * (P.N + 1) * P.dg_ldea * sizeof(int)));
+  P.d_ea = (int *)((unsigned char *)P.d_dig + dig);
+  return DCCM_OK;
+}
+
+static int launch_dg(Plan &P, int dir, int batch, int c0, int nct, double *out, cudaStream_t s) {
+  static bool attr_done = false;
+  if (!attr_done) {
+    DCCM_CUDA(cudaFuncSetAttribute(legendre_dg_kernel<DG_TN, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   DgShape<DG_TN>::SMEM));
+    DCCM_CUDA(cudaFuncSetAttribute(legendre_dg_kernel<DG_TN, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   DgShape<DG_TN>::SMEM));
+    attr_done = true;
+  }
+  const DgTable &T = dir == 0 ? P.dinv : P.dfwd;
+  DgArgs a;
+  a.N = P.N;
+  a.Jh = P.Jh;
+  a.batch = batch;
+  a.c0 = c0;
+  a.nct = nct;
+  a.nitems = T.nitems;
+  a.nchunk = T.nchunk;
+  a.ldea = P.dg_ldea;
+  a.ncoef = P.ncoef;
+  a.mi = (const DgMInfo *)T.d_mi;
+  a.items = T.d_items;
+  a.A = (const unsigned char *)P.d_dig;
+  a.B = (const unsigned char *)T.d_tab;
+  a.ea = P.d_ea;
+  a.eb = T.d_eb;
+  a.out = out;
+  a.err = P.d_err;
+  a.wait_ns = tunables().wait_limit_ms > 0 ? 1000000ull * (unsigned long long)tunables().wait_limit_ms : WAIT_LIMIT_NS;
+  a.withhold = tunables().tc_withhold_loads;
+  const int items = nct * T.nitems, ctas = sm_count();
+  DCCM_CUDA(launch_pdl(dir == 0 ? legendre_dg_kernel<DG_TN, 0> : legendre_dg_kernel<DG_TN, 1>, dim3(items < ctas ? items : ctas), dim3(DG_THREADS),
+                       (size_t)DgShape<DG_TN>::SMEM, s, a));
+  return DCCM_OK;
+}
+
+int legendre_inv_f64(Plan &P, int batch, const double *spec, double *F, cudaStream_t s) {
+  const int nct = (2 * batch + 127) / 128;
+  const DgMInfo *mi = (const DgMInfo *)P.dinv.d_mi;
+  for (int t = 0; t < nct; t += P.dg_ct) {
+    const int k = nct - t < P.dg_ct ? nct - t : P.dg_ct;
+    const int b0 = 64 * t, nb = batch - b0 < 64 * k ? batch - b0 : 64 * k;
+    // lanes a (m, field-level): 2 units of 8 for every 16 coefficients
+    if (P.N < 128)
+      DCCM_CUDA(launch_pdl(dg_pack_spec<8>, dim3((nb + 31) / 32, P.N + 1), dim3(256), 0, s, mi, P.N, (long long)P.ncoef,
+                           (const double2 *)spec, b0, nb, P.dinv.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea));
+    else
+      DCCM_CUDA(launch_pdl(dg_pack_spec<32>, dim3((nb + 7) / 8, P.N + 1), dim3(256), 0, s, mi, P.N, (long long)P.ncoef,
+                           (const double2 *)spec, b0, nb, P.dinv.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea));
+    DCCM_TRY(launch_dg(P, 0, batch, 128 * t, k, F, s));
+  }
+  return DCCM_OK;
+}
+
+int legendre_fwd_f64(Plan &P, int batch, const double *G, double *spec, cudaStream_t s) {
+  const int nct = (2 * batch + 127) / 128;
+  const int nq = (P.Jh + DG_CHUNK - 1) / DG_CHUNK;
+  const DgMInfo *mi = (const DgMInfo *)P.dfwd.d_mi;
+  for (int t = 0; t < nct; t += P.dg_ct) {
+    const int k = nct - t < P.dg_ct ? nct - t : P.dg_ct;
+    const int c0 = 128 * t, nc = 2 * batch - c0 < 128 * k ? 2 * batch - c0 : 128 * k;
+    auto pack = [&](auto kernel, int wq) {
+      const int per = 8 * (8 / wq);
+      return launch_pdl(kernel, dim3((nc + per - 1) / per, 2 * (P.N + 1)), dim3(256), 0, s, mi, P.Jh, 2 * batch, c0, nc, G,
+                        P.dfwd.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea);
+    };
+    DCCM_CUDA(nq <= 1 ? pack(dg_pack_four<1>, 1) : nq <= 2 ? pack(dg_pack_four<2>, 2)
+              : nq <= 4 ? pack(dg_pack_four<4>, 4) : pack(dg_pack_four<8>, 8));
+    DCCM_TRY(launch_dg(P, 1, batch, c0, k, spec, s));
+  }
+  return DCCM_OK;
+}
+
+}  // namespace sht
+}  // namespace dccm

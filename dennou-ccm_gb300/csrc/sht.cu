@@ -9,7 +9,8 @@
 // split into BF16 x 3 tensor-core tiles.
 //
 // Transform paths (precision chosen at plan creation):
-//   DCCM_SHT_FP64   Legendre on the FP64 CUDA cores, FP64 FFT;
+//   DCCM_SHT_FP64   Legendre by exact digit products on the tensor cores (the
+//                   accuracy of FP64 arithmetic, legendre_dg.cu), FP64 FFT;
 //   DCCM_SHT_MIXED  Legendre on tcgen05 tensor cores (BF16 x 3, FP32
 //                   accumulation), FP32 FFT; spectra and grids stay FP64;
 //   DCCM_SHT_MIXED_FP16  the same with FP16 hi + lo operands (3 products
@@ -95,7 +96,7 @@ static void destroy(Plan &P) {
   void *ptrs[] = {P.d_mu,      P.d_w,        P.d_pnm,       P.d_tw64,  P.d_tw32,  P.d_twl32,
                   P.tinv.d,    P.tfwd.d,     P.tinv.d_mi,   P.tfwd.d_mi, P.tinv.d_items,
                   P.tfwd.d_items, P.d_work,  P.d_err,       P.d_apack, P.d_punits, P.d_cexp,
-                  P.d_wa_pos, P.d_wa_src};
+                  P.d_wa_pos, P.d_wa_src, P.d_dig,     P.dinv.d_mem, P.dfwd.d_mem};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   P.stage.release();
@@ -160,6 +161,7 @@ static int create(Plan &P, int N, int I, int J, int precision, int max_batch) {
   DCCM_CUDA(cudaMalloc(&P.d_work, P.work_bytes));
   if (precision == DCCM_SHT_MIXED_FP16) DCCM_CUDA(cudaMalloc(&P.d_cexp, 2 * (size_t)max_batch * sizeof(int)));
   if (precision != DCCM_SHT_FP64) DCCM_TRY(build_tiles(P));
+  else DCCM_TRY(build_digits(P));
   DCCM_CUDA(cudaDeviceSynchronize());
   return DCCM_OK;
 }

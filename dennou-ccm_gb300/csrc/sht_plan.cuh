@@ -51,6 +51,17 @@ struct TileTable {
   int ntmax = 64;             // TMEM columns per accumulator (N tile bound)
 };
 
+// FP64 path: one direction's digit tables (legendre_dg.cu).
+struct DgTable {
+  void *d_mem = nullptr;      // the allocation that holds the four arrays below
+  void *d_mi = nullptr;       // per-m tile metadata
+  int2 *d_items = nullptr;    // work items (m, nt) of one 128-column tile
+  short *d_eb = nullptr;      // scale exponent of every table row
+  void *d_tab = nullptr;      // shared-memory images of the table tiles
+  int nchunk = 0;             // A chunks per 128-column tile
+  int nitems = 0;
+};
+
 struct Plan {
   int N = 0, I = 0, J = 0, Jh = 0;
   int precision = 0;
@@ -76,6 +87,10 @@ struct Plan {
   int *d_err = nullptr;        // device error flag of bounded waits
   int nsplit = 3;              // tensor-path operand splits: 3 (BF16 x 3) or 2 (FP16 hi + lo)
   int *d_cexp = nullptr;       // FP16: per field-level scale exponents, [inverse | forward][max_batch]
+  DgTable dinv, dfwd;          // FP64 path: digit tables
+  void *d_dig = nullptr;       // FP64 path: A operand images of up to dg_ct column tiles
+  int *d_ea = nullptr;         // FP64 path: scale exponents of the A operand, rows of dg_ldea (in d_dig)
+  int dg_ct = 0, dg_ldea = 0;
   DevBuf stage;                // host entry point staging
   cudaStream_t stream = nullptr;
   // SPML real layout (spml.cu), set up by the first call that uses it:
@@ -100,8 +115,8 @@ int fft_inverse_f64(const Plan &P, int batch, const double *F, double *grid, cud
 int fft_forward_f64(const Plan &P, int batch, const double *grid, double *G, cudaStream_t s);
 int fft_inverse(const Plan &P, int batch, bool fp32, const void *F, double *grid, cudaStream_t s);
 int fft_forward(const Plan &P, int batch, bool fp32, const double *grid, void *G, cudaStream_t s);
-int legendre_inv_f64(const Plan &P, int batch, const double *spec, double *F, cudaStream_t s);
-int legendre_fwd_f64(const Plan &P, int batch, const double *G, double *spec, cudaStream_t s);
+int legendre_inv_f64(Plan &P, int batch, const double *spec, double *F, cudaStream_t s);
+int legendre_fwd_f64(Plan &P, int batch, const double *G, double *spec, cudaStream_t s);
 int legendre_inv_tc(Plan &P, int batch, const double *spec, float *F, cudaStream_t s);
 int legendre_fwd_tc(Plan &P, int batch, const void *G3, double *spec, cudaStream_t s);
 int legendre_tc_multi(Plan *const *plans, const int *batch, const void *const *in, void *const *out,
@@ -113,6 +128,7 @@ int fft_multi(Plan *const *plans, const int *batch, const void *const *in, void 
 int inverse(Plan &P, const double *spec, double *grid, int batch, cudaStream_t s);
 int forward(Plan &P, const double *grid, double *spec, int batch, cudaStream_t s);
 int build_tiles(Plan &P);
+int build_digits(Plan &P);
 
 }  // namespace sht
 }  // namespace dccm

@@ -291,7 +291,8 @@ int dccm_area_integral_noalloc_dev(const double *f, const double *area, int64_t 
  *   - inverse: g = Re F_0 + 2 Re sum_{m>=1} F_m e^{i m lon},
  *     F_m(mu) = sum_n s_n^m Pbar_n^m(mu);
  *   - forward: s_n^m = (1/2) sum_j w_j Pbar_n^m(mu_j) (1/I) sum_i g_ij e^{-i m lon_i}.
- * precision DCCM_SHT_FP64: FP64 throughout (CUDA cores).
+ * precision DCCM_SHT_FP64: FP64 accuracy throughout (the Legendre sums as
+ * exact digit products on the tensor cores, FP64 FFT).
  * precision DCCM_SHT_MIXED: Legendre sums on the tensor cores in split
  * BF16 x 3 with FP32 accumulation, FFT in FP32; relative L2 error of a
  * forward(inverse(s)) round trip below 1e-6.  Requires jmax/2 % 16 == 0.

@@ -958,8 +958,7 @@ bool fft_length_supported(int I) {
   }
 }
 
-// The FP64 path uses the shared-memory Stockham transform (fft_f64.cu),
-// which needs fewer FP64 operations than the register/shuffle one.
+// The FP64 path has its own transform, in fixed point (fft_f64.cu).
 int fft_inverse(const Plan &P, int batch, bool fp32, const void *F, double *grid, cudaStream_t s) {
   if (batch <= 0) return DCCM_OK;
   if (!fp32) return fft_inverse_f64(P, batch, (const double *)F, grid, s);

@@ -1,238 +1,565 @@
-// Longitude FFT of the plain FP64 path: self-sorting Stockham radix-4/3/2
-// in shared memory, one warp per pair of latitude rows.
+// Longitude FFT of the FP64 path, in 64-bit block fixed point on the
+// integer pipes.
 //
-// On GB300 the FP64 pipe is the limit of this path, so it uses the
-// transform with the fewest FP64 operations per point: radix-4 stages
-// (multiplications by +-i are swaps) with table twiddles, about half the
-// multiplications of the register/shuffle factorisation that the FP32 path
-// uses (fft.cu).  Rows pair up as in fft.cu (z = g(jn) + i g(js)), and the
-// data layouts (F[m][j][c] in, G[m][p][jj][c] out) are the same.
+// The FP64 pipe of this GPU issues one warp instruction in 64 cycles, and a
+// 1024-point transform of a row pair takes about 36,000 FP64 operations (a
+// shared-memory Stockham transform in FP64 ran T341 x 192 field-levels in
+// 5.2 ms either way, T85 x 128 in 131 / 147 us).  In fixed point an addition
+// is two integer instructions and is exact, and a product with a 62-bit
+// twiddle takes three 32 x 32 -> 64 bit multiply-adds, all on full-rate
+// pipes.
+//
+// Rows pair up as in fft.cu: z = g(jn) + i g(js), one complex transform of
+// length I = R1 R2 (R3) by T = I / R1 threads.  A row pair has one scale:
+//   forward  the largest magnitude of the pair sits at 2^CB; every pass
+//            of radix R is followed by its twiddles times 2^-ceil(log2 R),
+//            so nothing overflows (|Z| <= sum |z|) and a pass rounds once,
+//            below 2^-53 of the row's r.m.s. for noise-like rows;
+//   inverse  every partial sum of the transform is bounded by the sum S of
+//            the input magnitudes, so the inputs are scaled with S at 2^61
+//            and no pass scales: roundings are a few 2^-61 S.
+// Both are below the rounding errors of an FP64 transform (about 2.5e-16 of
+// the r.m.s.; measured errors of the whole transforms fell, see the tests).
+// A row pair that holds an infinity or NaN comes out NaN.
+//
+// Passes are in place: forward decimation in frequency (radix-R DFT in
+// registers over stride N / R, twiddles), leaving frequency f = p1 + R1 p2 +
+// R1 R2 p3 at position p1 N1 + p2 N2 + p3; inverse the same passes
+// mirrored, from that order to natural order.  Positions are padded by one
+// in every last radix and one in every N1, so that the passes' 16-byte
+// accesses and the reads by frequency are free of bank conflicts.  A CTA
+// takes BB field-levels of one latitude pair, so that F and G are read and
+// written in runs of 16 BB bytes.
+#include <math.h>
+#include <string.h>
+
 #include "sht_plan.cuh"
 
 namespace dccm {
 namespace sht {
 namespace f64 {
 
-constexpr int MAX_STAGES = 12;
+struct C64 {
+  long long x, y;
+};
+__device__ __forceinline__ C64 operator+(C64 a, C64 b) { return {a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ C64 operator-(C64 a, C64 b) { return {a.x - b.x, a.y - b.y}; }
+// a times SG i
+template <int SG> __device__ __forceinline__ C64 muli(C64 a) {
+  return SG > 0 ? C64{-a.y, a.x} : C64{a.y, -a.x};
+}
 
-struct Radix {
-  int I, nst;
-  int r[MAX_STAGES];
+// z w for a twiddle in 64-bit fixed point, w = (x 2^32 + y, z 2^32 + w) with
+// signed low words: (z W) >> (32 + SH), rounded to nearest.  The product of
+// the two low words (below 2^-2 of the result's last place) is left out.
+template <int SH> __device__ __forceinline__ C64 twmul(C64 a, int4 w) {
+  const int xl = (int)a.x, xh = (int)(a.x >> 32) + ((unsigned)xl >> 31);
+  const int yl = (int)a.y, yh = (int)(a.y >> 32) + ((unsigned)yl >> 31);
+  const int ns = -w.z, nt = -w.w;
+  constexpr long long HALF = 1ll << (SH - 1);
+  long long m = (long long)xh * w.y + HALF;
+  m += (long long)xl * w.x;
+  m += (long long)yh * nt;
+  m += (long long)yl * ns;
+  long long r = (m >> 32) + (long long)xh * w.x;
+  r += (long long)yh * ns;
+  long long n = (long long)xh * w.w + HALF;
+  n += (long long)xl * w.z;
+  n += (long long)yh * w.y;
+  n += (long long)yl * w.x;
+  long long s = (n >> 32) + (long long)xh * w.z;
+  s += (long long)yh * w.x;
+  if constexpr (SH == 32) return {r, s};
+  else return {(r << (32 - SH)) | ((unsigned)m >> SH), (s << (32 - SH)) | ((unsigned)n >> SH)};
+}
+// x c for a constant |c| <= 1 given as (hi, lo) words of c 2^62
+__device__ __forceinline__ long long cmulr(long long x, int ch, int cl) {
+  const int xl = (int)x, xh = (int)(x >> 32) + ((unsigned)xl >> 31);
+  long long m = (long long)xh * cl + (1ll << 29);
+  m += (long long)xl * ch;
+  const long long r = (m >> 32) + (long long)xh * ch;
+  return (r << 2) | ((unsigned)m >> 30);
+}
+
+// cos(pi/4), cos(pi/8), sin(pi/8), sin(pi/3) times 2^62 as a signed low word
+// and the rest
+#define DCCM_FX(name, v)                                            \
+  constexpr int name##_L = (int)(unsigned)((unsigned long long)(v)); \
+  constexpr int name##_H = (int)(((v) + 0x80000000ll) >> 32)
+DCCM_FX(RH, 3260954456333195553ll);
+DCCM_FX(C8, 4260642322793532497ll);
+DCCM_FX(S8, 1764815834521887442ll);
+DCCM_FX(Q3, 3993837246235628775ll);
+#undef DCCM_FX
+
+__device__ __forceinline__ C64 mulc(C64 a, int ch, int cl, int sh, int sl) { return twmul<30>(a, make_int4(ch, cl, sh, sl)); }
+// a e^{SG i pi/4}, a e^{SG 3 i pi/4}
+template <int SG> __device__ __forceinline__ C64 rot1(C64 a) {
+  const C64 b = SG > 0 ? C64{a.x - a.y, a.x + a.y} : C64{a.x + a.y, a.y - a.x};
+  return {cmulr(b.x, RH_H, RH_L), cmulr(b.y, RH_H, RH_L)};
+}
+template <int SG> __device__ __forceinline__ C64 rot3(C64 a) { return muli<SG>(rot1<SG>(a)); }
+
+template <int SG> __device__ __forceinline__ void dft4(C64 &a, C64 &b, C64 &c, C64 &d) {
+  const C64 s0 = a + c, d0 = a - c, s1 = b + d, d1 = muli<SG>(b - d);
+  a = s0 + s1;
+  b = d0 + d1;
+  c = s0 - s1;
+  d = d0 - d1;
+}
+template <int SG> __device__ __forceinline__ void dft3(C64 &a, C64 &b, C64 &c) {
+  const C64 t = b + c, u = muli<SG>(b - c);
+  const C64 m = {a.x - (t.x >> 1), a.y - (t.y >> 1)};
+  const C64 q = {cmulr(u.x, Q3_H, Q3_L), cmulr(u.y, Q3_H, Q3_L)};
+  a = a + t;
+  b = m + q;
+  c = m - q;
+}
+
+// v[p] = sum_q v[q] e^{SG 2 pi i p q / R}
+template <int SG, int R> __device__ __forceinline__ void dft(C64 (&v)[R]) {
+  if constexpr (R == 4) {
+    dft4<SG>(v[0], v[1], v[2], v[3]);
+  } else if constexpr (R == 8) {  // 2 x 4: even and odd q, then radix 2 over them
+    dft4<SG>(v[0], v[2], v[4], v[6]);
+    dft4<SG>(v[1], v[3], v[5], v[7]);
+    const C64 o1 = rot1<SG>(v[3]), o2 = muli<SG>(v[5]), o3 = rot3<SG>(v[7]);
+    const C64 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1];
+    v[0] = e0 + o0;
+    v[4] = e0 - o0;
+    v[1] = e1 + o1;
+    v[5] = e1 - o1;
+    v[2] = e2 + o2;
+    v[6] = e2 - o2;
+    v[3] = e3 + o3;
+    v[7] = e3 - o3;
+  } else if constexpr (R == 16) {  // 4 x 4
+#pragma unroll
+    for (int q = 0; q < 4; ++q) dft4<SG>(v[q], v[q + 4], v[q + 8], v[q + 12]);
+    // v[q + 4 a]: twiddle e^{SG 2 pi i a q / 16}
+    const int S = SG;
+    v[5] = mulc(v[5], C8_H, C8_L, S * S8_H, S * S8_L);
+    v[6] = rot1<SG>(v[6]);
+    v[7] = mulc(v[7], S8_H, S8_L, S * C8_H, S * C8_L);
+    v[9] = rot1<SG>(v[9]);
+    v[10] = muli<SG>(v[10]);
+    v[11] = rot3<SG>(v[11]);
+    v[13] = mulc(v[13], S8_H, S8_L, S * C8_H, S * C8_L);
+    v[14] = rot3<SG>(v[14]);
+    v[15] = mulc(v[15], -C8_H, -C8_L, -S * S8_H, -S * S8_L);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) dft4<SG>(v[4 * a], v[4 * a + 1], v[4 * a + 2], v[4 * a + 3]);
+    // output p = a + 4 b is at v[4 a + b]
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = a + 1; b < 4; ++b) {
+        const C64 t = v[4 * a + b];
+        v[4 * a + b] = v[4 * b + a];
+        v[4 * b + a] = t;
+      }
+  } else {  // R == 12: coprime factors 3 x 4 (Good's mapping), no twiddles
+    static_assert(R == 12);
+    C64 u[3][4];
+    // q = 4 a + 3 b (mod 12)
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) u[a][b] = v[(4 * a + 3 * b) % 12];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) dft3<SG>(u[0][b], u[1][b], u[2][b]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) dft4<SG>(u[a][0], u[a][1], u[a][2], u[a][3]);
+    // p = A (mod 3), B (mod 4) with e^{2 pi i p (4 a + 3 b) / 12} = e^{2 pi i p a / 3} e^{2 pi i p b / 4}
+#pragma unroll
+    for (int p = 0; p < 12; ++p) v[p] = u[p % 3][p % 4];
+  }
+}
+
+constexpr int clog2(int r) { return r <= 1 ? 0 : r <= 2 ? 1 : r <= 4 ? 2 : r <= 8 ? 3 : 4; }
+
+template <int I_, int R1_, int R2_, int R3_> struct Shape {
+  static constexpr int I = I_, R1 = R1_, R2 = R2_, R3 = R3_;
+  static constexpr int N1 = I / R1, N2 = N1 / R2;  // N2 = R3
+  static constexpr int T = N1;                     // threads a row pair
+  static constexpr int RL = R3 > 1 ? R3 : R2;      // last radix
+  static constexpr int S1 = clog2(R1), S2 = R3 > 1 ? clog2(R2) : 0;
+  // forward: components of the input below 2^CB, so that R1 2^(CB + 1/2) and
+  // the fold of four results of the last pass stay below 2^63
+  static constexpr int CB = 60 - clog2(RL) < 58 ? 60 - clog2(RL) : 58;
+  static constexpr int THREADS = T >= 64 ? 256 : 128;
+  static constexpr int BB = THREADS / T;
+  static __host__ __device__ constexpr int at(int a) { return a + a / RL + (R3 > 1 ? a / N1 : 0); }
+  // stride of the row pairs' buffers, 2 (mod 8) 16-byte units
+  static constexpr int LD = (at(I - 1) + 1 + 7) / 8 * 8 + 2;
+  static constexpr int TW = (R1 - 1) * N1 + (R3 > 1 ? (R2 - 1) * N2 : 0);  // twiddles of a direction
+  static __device__ __forceinline__ int pos(int f) {                       // position of frequency f
+    const int p1 = f % R1, r = f / R1;
+    return at(p1 * N1 + (r % R2) * N2 + r / R2);
+  }
 };
 
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// lanes of this thread's row pair (T <= 32)
+template <int T> __device__ __forceinline__ unsigned group_mask() {
+  if constexpr (T >= 32) return 0xffffffffu;
+  else return ((1u << T) - 1u) << (threadIdx.x % 32 / T * T);
 }
-__device__ __forceinline__ double2 cmuli(double2 a, int s) { return make_double2(-a.y * s, a.x * s); }
+template <int T> __device__ __forceinline__ void group_sync(int g) {
+  if constexpr (T <= 32) __syncwarp(group_mask<T>());
+  else asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(T) : "memory");
+}
 
-// Stockham autosort FFT of one complex row by one warp.  sign = -1 forward,
-// +1 inverse (unnormalised).  Returns the buffer holding the result.
-__device__ double2 *warp_stockham(double2 *x, double2 *y, const double2 *__restrict__ tw, const Radix &a,
-                                  int sign, int lane) {
-  const int I = a.I;
-  int Ns = 1;
-  for (int st = 0; st < a.nst; ++st) {
-    const int R = a.r[st];
-    const int nb = I / R;
-    const int tstep = I / (Ns * R);
-    for (int j = lane; j < nb; j += 32) {
-      const int k = j % Ns;
-      const int base = (j / Ns) * Ns * R + k;
-      double2 v[4];
+__device__ __forceinline__ unsigned mag(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
+
+// x 2^k as an integer, k = sh + 1075 - (exponent of the row), given as
+// r = 10 - (shift of the 53-bit mantissa): (mantissa 2^10) >> (r - ef), rounded.
+__device__ __forceinline__ long long to_fixed(double x, int rbase) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int ef = (int)(b >> 52) & 0x7FF;
+  const unsigned long long m = ((b << 10) & 0x3FFFFFFFFFFFFC00ull) | (ef ? 1ull << 62 : 0ull);
+  int r = rbase - (ef ? ef : 1);
+  r = r > 63 ? 63 : r;
+  const long long q = (long long)(((m >> (r - 1)) + 1) >> 1);
+  return (long long)b < 0 ? -q : q;
+}
+
+// q 2^ex as the nearest double (ties away from zero).
+__device__ __forceinline__ double to_double(long long q, int ex) {
+  const long long s = q >> 63;
+  unsigned long long m = (unsigned long long)((q ^ s) - s);
+  const int z = __clzll((long long)m);
+  if (m == 0) return 0.0;
+  m <<= z;
+  const unsigned long long mant = (m >> 11) + ((unsigned)m >> 10 & 1u);
+  const int be = ex + 63 - z + 1023;
+  if ((unsigned)(be - 1) >= 2045u) {  // subnormal result or overflow
+    const double r = ldexp((double)mant, be - 1075);
+    return s ? -r : r;
+  }
+  return __longlong_as_double((long long)((((unsigned long long)(unsigned)(be - 1) << 52) + mant) |
+                                          ((unsigned long long)s << 63)));
+}
+
+// One in-place pass over the buffer of a row pair: DFTs of radix R over
+// stride NS within blocks of R NS.  SG < 0: DFT, then twiddles (scaled);
+// SG > 0: twiddles, then DFT.
+template <class Sh, int SG, int R, int NS, int SHIFT>
+__device__ __forceinline__ void pass(C64 *z, const int4 *__restrict__ tw, int t) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-        if (r < R) {
-          double2 t = x[j + r * nb];
-          if (r > 0 && k > 0) {
-            double2 w = tw[k * r * tstep];
-            if (sign > 0) w.y = -w.y;
-            t = cmul(t, w);
-          }
-          v[r] = t;
-        }
-      if (R == 4) {
-        const double2 s0 = cadd(v[0], v[2]), d0 = csub(v[0], v[2]);
-        const double2 s1 = cadd(v[1], v[3]), d1 = cmuli(csub(v[1], v[3]), sign);
-        y[base] = cadd(s0, s1);
-        y[base + Ns] = cadd(d0, d1);
-        y[base + 2 * Ns] = csub(s0, s1);
-        y[base + 3 * Ns] = csub(d0, d1);
-      } else if (R == 2) {
-        y[base] = cadd(v[0], v[1]);
-        y[base + Ns] = csub(v[0], v[1]);
-      } else {  // R == 3
-        const double2 t1 = cadd(v[1], v[2]);
-        const double2 t2 = cmuli(csub(v[1], v[2]), sign);
-        const double h = 0.86602540378443864676;  // sqrt(3)/2
-        const double2 m = make_double2(v[0].x - 0.5 * t1.x, v[0].y - 0.5 * t1.y);
-        const double2 q = make_double2(t2.x * h, t2.y * h);
-        y[base] = cadd(v[0], t1);
-        y[base + Ns] = cadd(m, q);
-        y[base + 2 * Ns] = csub(m, q);
-      }
+  for (int d0 = 0; d0 < Sh::I / R; d0 += Sh::T) {
+    const int d = d0 + t;
+    if ((Sh::I / R) % Sh::T != 0 && d >= Sh::I / R) break;
+    const int k = d % NS, base = (d / NS) * (R * NS) + k;
+    C64 v[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = z[Sh::at(base + q * NS)];
+    if (NS > 1 && SG > 0) {
+#pragma unroll
+      for (int q = 1; q < R; ++q) v[q] = twmul<SHIFT>(v[q], __ldg(tw + (q - 1) * NS + k));
     }
-    __syncwarp();
-    double2 *t = x;
-    x = y;
-    y = t;
-    Ns *= R;
+    dft<SG, R>(v);
+    if (NS > 1 && SG < 0) {
+      // the p = 0 output has twiddle 1: the same scaling by a rounded shift
+      constexpr int s = clog2(R);
+      v[0] = {(v[0].x + (1ll << (s - 1))) >> s, (v[0].y + (1ll << (s - 1))) >> s};
+#pragma unroll
+      for (int p = 1; p < R; ++p) v[p] = twmul<SHIFT>(v[p], __ldg(tw + (p - 1) * NS + k));
+    }
+#pragma unroll
+    for (int p = 0; p < R; ++p) z[Sh::at(base + p * NS)] = v[p];
   }
-  return x;
 }
 
-__global__ void __launch_bounds__(512)
-fft64_inverse_kernel(Radix a, int N, int J, int batch, int BB, const double *__restrict__ F,
-                     double *__restrict__ grid, const double2 *__restrict__ twg) {
+template <class Sh>
+__global__ void __launch_bounds__(Sh::THREADS, 512 / Sh::THREADS)
+fft_forward_kernel(int N, int J, int batch, const double *__restrict__ grid, double *__restrict__ G,
+                   const int4 *__restrict__ tw, int4 w0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int I = a.I, Jh = J / 2;
-  const int jj = blockIdx.x;
-  const int jn = Jh + jj, js = Jh - 1 - jj;
-  const int b0 = blockIdx.y * BB;
-  const int nb = min(BB, batch - b0);
-  const int64_t C2B = 2LL * batch;
-  const int cw = 2 * BB;
-  double *stA = reinterpret_cast<double *>(smem_raw);
-  double *stB = stA + (size_t)(N + 1) * cw;
-  double2 *tw = reinterpret_cast<double2 *>(stB + (size_t)(N + 1) * cw);
-  double2 *bufs = tw + I;
-  for (int t = threadIdx.x; t < I; t += blockDim.x) tw[t] = twg[t];
-  for (int t = threadIdx.x; t < (N + 1) * cw; t += blockDim.x) {
-    const int m = t / cw, c = t % cw;
-    double va = 0, vb = 0;
-    if (c < 2 * nb) {
-      va = F[((int64_t)m * J + jn) * C2B + 2LL * b0 + c];
-      vb = F[((int64_t)m * J + js) * C2B + 2LL * b0 + c];
+  C64 *buf = reinterpret_cast<C64 *>(smem_raw);
+  __shared__ unsigned smx[Sh::BB][2];
+  __shared__ int sE[Sh::BB];
+  const int Jh = J / 2, jj = blockIdx.x % Jh, jn = Jh + jj, js = Jh - 1 - jj;
+  const int b0 = blockIdx.x / Jh * Sh::BB, nb = min(Sh::BB, batch - b0);
+  const int g = threadIdx.x / Sh::T, t = threadIdx.x % Sh::T;  // row pair, thread of it
+  C64 *z = buf + (size_t)g * Sh::LD;
+  pdl_wait();
+  pdl_trigger();
+  if (g < nb) {
+    const double *gn = grid + ((int64_t)(b0 + g) * J + jn) * Sh::I + t;
+    const double *gs = grid + ((int64_t)(b0 + g) * J + js) * Sh::I + t;
+    double a[Sh::R1], b[Sh::R1];
+#pragma unroll
+    for (int q = 0; q < Sh::R1; ++q) {
+      a[q] = __ldg(gn + q * Sh::N1);
+      b[q] = __ldg(gs + q * Sh::N1);
     }
-    stA[t] = va;
-    stB[t] = vb;
+    unsigned mx = 0;
+#pragma unroll
+    for (int q = 0; q < Sh::R1; ++q) mx = max(mx, max(mag(a[q]), mag(b[q])));
+#pragma unroll
+    for (int o = (Sh::T < 32 ? Sh::T : 32) / 2; o > 0; o >>= 1)
+      mx = max(mx, __shfl_xor_sync(group_mask<Sh::T>(), mx, o));
+    if constexpr (Sh::T > 32) {
+      if (t % 32 == 0) smx[g][t / 32] = mx;
+      group_sync<Sh::T>(g);
+      mx = max(smx[g][0], smx[g][1]);
+    }
+    const int E = max((int)(mx >> 20), 1);
+    if (t == 0) sE[g] = E;
+    // |x| < 2^(E - 1022) -> 2^CB: the mantissa moves by CB - 53 + ef - E
+    const int rb = 10 - (Sh::CB - 53) + E;
+    C64 v[Sh::R1];
+#pragma unroll
+    for (int q = 0; q < Sh::R1; ++q) v[q] = {to_fixed(a[q], rb), to_fixed(b[q], rb)};
+    dft<-1, Sh::R1>(v);
+    v[0] = twmul<32>(v[0], w0);
+#pragma unroll
+    for (int p = 1; p < Sh::R1; ++p) v[p] = twmul<32>(v[p], __ldg(tw + (p - 1) * Sh::N1 + t));
+#pragma unroll
+    for (int p = 0; p < Sh::R1; ++p) z[Sh::at(p * Sh::N1 + t)] = v[p];
+    group_sync<Sh::T>(g);
+    pass<Sh, -1, Sh::R2, Sh::N2, 32>(z, tw + (Sh::R1 - 1) * Sh::N1, t);
+    if constexpr (Sh::R3 > 1) {
+      group_sync<Sh::T>(g);
+      pass<Sh, -1, Sh::R3, 1, 32>(z, nullptr, t);
+    }
   }
   __syncthreads();
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int nw = blockDim.x / 32;
-  double2 *x = bufs + (size_t)warp * 2 * I;
-  double2 *y = x + I;
-  for (int bl = warp; bl < nb; bl += nw) {
-    for (int k = lane; k < I; k += 32) x[k] = make_double2(0.0, 0.0);
-    __syncwarp();
-    for (int m = lane; m <= N; m += 32) {
-      const double ar = stA[m * cw + 2 * bl], ai = m ? stA[m * cw + 2 * bl + 1] : 0.0;
-      const double br = stB[m * cw + 2 * bl], bi = m ? stB[m * cw + 2 * bl + 1] : 0.0;
-      x[m] = make_double2(ar - bi, ai + br);
-      if (m > 0) x[I - m] = make_double2(ar + bi, br - ai);
-    }
-    __syncwarp();
-    double2 *z = warp_stockham(x, y, tw, a, +1, lane);
-    double *gn = grid + ((int64_t)(b0 + bl) * J + jn) * I;
-    double *gs = grid + ((int64_t)(b0 + bl) * J + js) * I;
-    for (int i = lane; i < I; i += 32) {
-      gn[i] = z[i].x;
-      gs[i] = z[i].y;
-    }
-    __syncwarp();
+  // results: E = A + B, O = A - B of the rows' spectra A, B, field-levels fastest
+  constexpr bool THREE = Sh::I % 3 == 0;  // the twiddles carry 2/3
+  const int bl = threadIdx.x % Sh::BB;
+  if (bl >= nb) return;
+  const C64 *zb = buf + (size_t)bl * Sh::LD;
+  const int E = sE[bl];
+  // value = q 2^ex: row scale, pass scalings, the halves of A and B, and 1/I
+  constexpr int LI = THREE ? clog2(Sh::I / 96) + 5 + 1 : clog2(Sh::I / 64) + 6;
+  const int ex = E - 1022 - Sh::CB + Sh::S1 + Sh::S2 - 1 - LI;
+  const int64_t C2B = 2LL * batch;
+  double2 *out = reinterpret_cast<double2 *>(G + (int64_t)jj * C2B + 2 * (b0 + bl));
+  const int64_t pst = (int64_t)Jh * batch;  // one parity of one m, in double2
+  const double nan = __longlong_as_double(0x7FF8000000000000ll);
+  for (int m = threadIdx.x / Sh::BB; m <= N; m += Sh::T) {
+    const C64 a = zb[Sh::pos(m)], c = zb[Sh::pos(m ? Sh::I - m : 0)];
+    // 2A = (a.x + c.x, a.y - c.y), 2B = (a.y + c.y, c.x - a.x)
+    const long long ar = a.x + c.x, ai = a.y - c.y, br = a.y + c.y, bi = c.x - a.x;
+    double2 e = make_double2(to_double(ar + br, ex), to_double(ai + bi, ex));
+    double2 o = make_double2(to_double(ar - br, ex), to_double(ai - bi, ex));
+    if (m == 0) e.y = o.y = 0.0;
+    if (E >= 2047) e = o = make_double2(nan, m ? nan : 0.0);
+    out[(int64_t)(2 * m) * pst] = e;
+    out[(int64_t)(2 * m + 1) * pst] = o;
   }
 }
 
-__global__ void __launch_bounds__(512)
-fft64_forward_kernel(Radix a, int N, int J, int batch, int BB, const double *__restrict__ grid,
-                     double *__restrict__ G, const double2 *__restrict__ twg) {
+template <class Sh>
+__global__ void __launch_bounds__(Sh::THREADS, 512 / Sh::THREADS)
+fft_inverse_kernel(int N, int J, int batch, const double *__restrict__ F, double *__restrict__ grid,
+                   const int4 *__restrict__ tw) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int I = a.I, Jh = J / 2;
-  const int jj = blockIdx.x;
-  const int jn = Jh + jj, js = Jh - 1 - jj;
-  const int b0 = blockIdx.y * BB;
-  const int nb = min(BB, batch - b0);
+  C64 *buf = reinterpret_cast<C64 *>(smem_raw);
+  __shared__ unsigned smx[Sh::BB], ssum[Sh::BB];
+  const int Jh = J / 2, jj = blockIdx.x % Jh, jn = Jh + jj, js = Jh - 1 - jj;
+  const int b0 = blockIdx.x / Jh * Sh::BB, nb = min(Sh::BB, batch - b0);
+  if (threadIdx.x < Sh::BB) smx[threadIdx.x] = ssum[threadIdx.x] = 0;
+  __syncthreads();
+  pdl_wait();
+  pdl_trigger();
+  // Fourier coefficients (m, field-level), field-levels fastest
+  constexpr int KI = Sh::R1 / 2;  // N + 1 <= I / 2
+  const int bl = threadIdx.x % Sh::BB, m0 = threadIdx.x / Sh::BB;
   const int64_t C2B = 2LL * batch;
-  const int cw = 2 * BB;
-  double *stE = reinterpret_cast<double *>(smem_raw);
-  double *stO = stE + (size_t)(N + 1) * cw;
-  double2 *tw = reinterpret_cast<double2 *>(stO + (size_t)(N + 1) * cw);
-  double2 *bufs = tw + I;
-  for (int t = threadIdx.x; t < I; t += blockDim.x) tw[t] = twg[t];
-  __syncthreads();
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int nw = blockDim.x / 32;
-  double2 *x = bufs + (size_t)warp * 2 * I;
-  double2 *y = x + I;
-  const double invI = 1.0 / (double)I;
-  for (int bl = warp; bl < nb; bl += nw) {
-    const double *gn = grid + ((int64_t)(b0 + bl) * J + jn) * I;
-    const double *gs = grid + ((int64_t)(b0 + bl) * J + js) * I;
-    for (int i = lane; i < I; i += 32) x[i] = make_double2(gn[i], gs[i]);
-    __syncwarp();
-    double2 *Z = warp_stockham(x, y, tw, a, -1, lane);
-    for (int m = lane; m <= N; m += 32) {
-      const double2 zm = Z[m], zc = Z[(I - m) % I];
-      const double ar = 0.5 * (zm.x + zc.x), ai = 0.5 * (zm.y - zc.y);
-      const double br = 0.5 * (zm.y + zc.y), bi = -0.5 * (zm.x - zc.x);
-      stE[m * cw + 2 * bl] = (ar + br) * invI;
-      stE[m * cw + 2 * bl + 1] = m ? (ai + bi) * invI : 0.0;
-      stO[m * cw + 2 * bl] = (ar - br) * invI;
-      stO[m * cw + 2 * bl + 1] = m ? (ai - bi) * invI : 0.0;
-    }
-    __syncwarp();
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < (N + 1) * cw; t += blockDim.x) {
-    const int m = t / cw, c = t % cw;
-    if (c < 2 * nb) {
-      G[(((int64_t)m * 2 + 0) * Jh + jj) * C2B + 2LL * b0 + c] = stE[t];
-      G[(((int64_t)m * 2 + 1) * Jh + jj) * C2B + 2LL * b0 + c] = stO[t];
+  double2 a[KI], b[KI];
+  unsigned mx = 0;
+#pragma unroll
+  for (int i = 0; i < KI; ++i) {
+    const int m = m0 + i * Sh::T;
+    a[i] = b[i] = make_double2(0.0, 0.0);
+    if (bl < nb && m <= N) {
+      const double *f = F + (int64_t)m * J * C2B + 2 * (b0 + bl);
+      a[i] = __ldg(reinterpret_cast<const double2 *>(f + jn * C2B));
+      b[i] = __ldg(reinterpret_cast<const double2 *>(f + js * C2B));
+      if (m == 0) a[i].y = b[i].y = 0.0;
     }
   }
-}
-
-static bool radix_plan(int I, Radix &a) {
-  a.I = I;
-  a.nst = 0;
-  int n = I;
-  while (n % 4 == 0 && a.nst < MAX_STAGES) { a.r[a.nst++] = 4; n /= 4; }
-  while (n % 2 == 0 && a.nst < MAX_STAGES) { a.r[a.nst++] = 2; n /= 2; }
-  while (n % 3 == 0 && a.nst < MAX_STAGES) { a.r[a.nst++] = 3; n /= 3; }
-  return n == 1;
-}
-
-static int pick_bb(const Plan &P, int batch, size_t *smem) {
-  const size_t budget = 160 * 1024;
-  int BB = 16;
-  auto need = [&](int bb) {
-    return (size_t)(P.N + 1) * 2 * bb * 2 * sizeof(double) + (size_t)P.I * sizeof(double2) * (1 + 2 * (size_t)bb);
+#pragma unroll
+  for (int i = 0; i < KI; ++i) mx = max(max(mx, max(mag(a[i].x), mag(a[i].y))), max(mag(b[i].x), mag(b[i].y)));
+  atomicMax(&smx[bl], mx);
+  __syncthreads();
+  const int E = max((int)(smx[bl] >> 20), 1);
+  // sum of the magnitudes in units of 2^(E - 1022 - 20), each rounded up
+  unsigned sum = 0;
+  auto units = [&](double x) {
+    const unsigned h = mag(x);
+    const int ef = (int)(h >> 20);
+    const unsigned m20 = ((h & 0xFFFFFu) | (ef ? 0x100000u : 0u)) >> 1;
+    return (m20 >> min(E - max(ef, 1), 31)) + 1u;
   };
-  while (BB > 1 && need(BB) > budget) BB /= 2;
-  if (BB > batch) BB = batch < 1 ? 1 : batch;
-  *smem = need(BB);
-  return BB;
+#pragma unroll
+  for (int i = 0; i < KI; ++i) sum += units(a[i].x) + units(a[i].y) + units(b[i].x) + units(b[i].y);
+  atomicAdd(&ssum[bl], sum);
+  __syncthreads();
+  // sum of |Re Z| + |Im Z| over all frequencies < 2^(nbit + 1) units -> 2^61:
+  // the mantissa moves by ef - E + 27 - nbit
+  const int nbit = 32 - __clz((int)ssum[bl]);
+  const int rb = 10 - (27 - nbit) + E;
+  C64 *zb = buf + (size_t)bl * Sh::LD;
+#pragma unroll
+  for (int i = 0; i < KI; ++i) {
+    const int m = m0 + i * Sh::T;
+    const long long ar = to_fixed(a[i].x, rb), ai = to_fixed(a[i].y, rb);
+    const long long br = to_fixed(b[i].x, rb), bi = to_fixed(b[i].y, rb);
+    // frequencies above N hold zeros; I / 2 is never used (N < I / 2)
+    zb[Sh::pos(m)] = {ar - bi, ai + br};
+    zb[Sh::pos(m ? Sh::I - m : Sh::I / 2)] = m ? C64{ar + bi, br - ai} : C64{0, 0};
+  }
+  __syncthreads();
+  const int g = threadIdx.x / Sh::T, t = threadIdx.x % Sh::T;
+  if (g >= nb) return;
+  C64 *z = buf + (size_t)g * Sh::LD;
+  if constexpr (Sh::R3 > 1) {
+    pass<Sh, 1, Sh::R3, 1, 30>(z, nullptr, t);
+    group_sync<Sh::T>(g);
+  }
+  pass<Sh, 1, Sh::R2, Sh::N2, 30>(z, tw + (Sh::R1 - 1) * Sh::N1, t);
+  group_sync<Sh::T>(g);
+  C64 v[Sh::R1];
+#pragma unroll
+  for (int q = 0; q < Sh::R1; ++q) v[q] = z[Sh::at(q * Sh::N1 + t)];
+#pragma unroll
+  for (int q = 1; q < Sh::R1; ++q) v[q] = twmul<30>(v[q], __ldg(tw + (q - 1) * Sh::N1 + t));
+  dft<1, Sh::R1>(v);
+  const int Eg = max((int)(smx[g] >> 20), 1);
+  const int ex = Eg - 1075 - (27 - (32 - __clz((int)ssum[g])));
+  const double nan = __longlong_as_double(0x7FF8000000000000ll);
+  double *gn = grid + ((int64_t)(b0 + g) * J + jn) * Sh::I + t;
+  double *gs = grid + ((int64_t)(b0 + g) * J + js) * Sh::I + t;
+#pragma unroll
+  for (int p = 0; p < Sh::R1; ++p) {
+    gn[p * Sh::N1] = Eg >= 2047 ? nan : to_double(v[p].x, ex);
+    gs[p * Sh::N1] = Eg >= 2047 ? nan : to_double(v[p].y, ex);
+  }
+}
+
+// ------------------------------------------------------------------ host
+// cos and sin of pi x / 4, 0 <= x <= 1 (x = num / den), as integers times
+// 2^62, by Taylor series in 128-bit integers (error below 2^-61: the same
+// table on every host).
+static void octant(unsigned num, unsigned den, long long &c, long long &s) {
+  typedef unsigned __int128 u128;
+  // pi / 4 in 2^-96 units
+  const u128 PI4 = ((u128)0xC90FDAA2ull << 64) | 0x2168C234C4C6628Bull;
+  const u128 th = PI4 * num / den;  // num < 2^11: no overflow below 2^128
+  const unsigned long long x = (unsigned long long)(th >> 32) + (unsigned long long)((th >> 31) & 1);  // 2^-64 units
+  auto mul = [](unsigned long long a, unsigned long long b) { return (unsigned long long)(((u128)a * b + (1ull << 63)) >> 64); };
+  const unsigned long long x2 = mul(x, x);
+  // terms 1 - x^2/2 + ... and x - x^3/6 + ..., summed signed in 128 bits
+  __int128 cs = (__int128)1 << 64, sn = x;
+  unsigned long long tc = 0, ts = x;
+  for (int k = 1; k <= 14; ++k) {
+    tc = k == 1 ? x2 / 2 : mul(tc, x2) / (unsigned)((2 * k - 1) * (2 * k));
+    ts = mul(ts, x2) / (unsigned)((2 * k) * (2 * k + 1));
+    cs += (k & 1) ? -(__int128)tc : (__int128)tc;
+    sn += (k & 1) ? -(__int128)ts : (__int128)ts;
+  }
+  c = (long long)((cs + 2) >> 2);
+  s = (long long)((sn + 2) >> 2);
+}
+// e^{2 pi i t / I} times 2^62
+static void unit_root(int t, int I, long long &c, long long &s) {
+  const int o = 8 * t / I, r = 8 * t - o * I;  // octant, remainder in 1/I of it
+  long long a, b;
+  if (o & 1) octant((unsigned)(I - r), (unsigned)I, b, a);  // the octant's mirror image
+  else octant((unsigned)r, (unsigned)I, a, b);
+  switch (o / 2) {  // quadrant
+    case 0: c = a; s = b; break;
+    case 1: c = -b; s = a; break;
+    case 2: c = -a; s = -b; break;
+    default: c = b; s = -a; break;
+  }
+}
+static int4 words(long long c, long long s) {
+  auto hi = [](long long v) { return (int)((v + 0x80000000ll) >> 32); };
+  auto lo = [](long long v) {
+    const int l = (int)(unsigned)(unsigned long long)v;
+    return l == (int)0x80000000 ? l + 1 : l;  // its negative has to fit
+  };
+  return make_int4(hi(c), lo(c), hi(s), lo(s));
+}
+// v 2^-k, times 2/3 if three, rounded
+static long long scaled(long long v, int k, bool three) {
+  __int128 x = (__int128)v * (three ? 2 : 1);
+  const __int128 d = ((__int128)1 << k) * (three ? 3 : 1);
+  return (long long)(x >= 0 ? (x + d / 2) / d : -((-x + d / 2) / d));
+}
+
+template <class F> static int with_shape(int I, F &&f) {
+  switch (I) {
+    case 64: return f(Shape<64, 8, 8, 1>());
+    case 96: return f(Shape<96, 12, 8, 1>());
+    case 128: return f(Shape<128, 16, 8, 1>());
+    case 192: return f(Shape<192, 12, 16, 1>());
+    case 256: return f(Shape<256, 16, 16, 1>());
+    case 384: return f(Shape<384, 12, 8, 4>());
+    case 512: return f(Shape<512, 16, 8, 4>());
+    case 768: return f(Shape<768, 12, 8, 8>());
+    case 1024: return f(Shape<1024, 16, 8, 8>());
+    default: return DCCM_ERR_UNSUPPORTED;
+  }
 }
 
 }  // namespace f64
 
+// Twiddles of both directions: forward entries e^{-i theta} 2^(64 - s), such that twmul<32> scales by 2^-s, s = ceil(log2 R) (and by 2/3 in the
+// first pass of lengths with a factor 3, the odd part of 1/I); inverse
+// entries e^{+i theta} 2^62 for twmul<30>.
+int build_fft_f64(Plan &P, std::vector<int4> &h) {
+  using namespace f64;
+  return with_shape(P.I, [&](auto sh) {
+    using Sh = decltype(sh);
+    h.assign(2 * Sh::TW + 1, int4());
+    const bool three = Sh::I % 3 == 0;
+    for (int dir = 0; dir < 2; ++dir) {
+      int4 *w = h.data() + dir * Sh::TW;
+      auto fill = [&](int R, int NS, int scale, bool th) {
+        for (int p = 1; p < R; ++p)
+          for (int k = 0; k < NS; ++k) {
+            long long c, s;
+            unit_root(p * k, R * NS, c, s);  // p k < R NS
+            if (dir == 0) *w++ = words(scaled(c, scale - 2, th), scaled(-s, scale - 2, th));
+            else *w++ = words(c, s);
+          }
+      };
+      fill(Sh::R1, Sh::N1, Sh::S1, three);
+      if (Sh::R3 > 1) fill(Sh::R2, Sh::N2, Sh::S2, false);
+    }
+    // the first pass's twiddle 1, scaled
+    h[2 * Sh::TW] = words(scaled(1ll << 62, Sh::S1 - 2, three), 0);
+    return DCCM_OK;
+  });
+}
+
 int fft_inverse_f64(const Plan &P, int batch, const double *F, double *grid, cudaStream_t s) {
   if (batch <= 0) return DCCM_OK;
-  f64::Radix a;
-  if (!f64::radix_plan(P.I, a)) return DCCM_ERR_UNSUPPORTED;
-  size_t smem;
-  const int BB = f64::pick_bb(P, batch, &smem);
-  DCCM_CUDA(cudaFuncSetAttribute(f64::fft64_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-  f64::fft64_inverse_kernel<<<dim3(P.Jh, (batch + BB - 1) / BB), 32 * BB, smem, s>>>(a, P.N, P.J, batch, BB, F,
-                                                                                     grid, P.d_tw64);
-  DCCM_LAUNCH_CHECK();
-  return DCCM_OK;
+  return f64::with_shape(P.I, [&](auto sh) {
+    using Sh = decltype(sh);
+    const size_t smem = (size_t)Sh::BB * Sh::LD * sizeof(f64::C64);
+    DCCM_CUDA(cudaFuncSetAttribute(f64::fft_inverse_kernel<Sh>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DCCM_CUDA(launch_pdl(f64::fft_inverse_kernel<Sh>, dim3((unsigned)P.Jh * ((batch + Sh::BB - 1) / Sh::BB)), dim3(Sh::THREADS), smem,
+                         s, P.N, P.J, batch, F, grid, P.d_twfx + Sh::TW));
+    return DCCM_OK;
+  });
 }
 
 int fft_forward_f64(const Plan &P, int batch, const double *grid, double *G, cudaStream_t s) {
   if (batch <= 0) return DCCM_OK;
-  f64::Radix a;
-  if (!f64::radix_plan(P.I, a)) return DCCM_ERR_UNSUPPORTED;
-  size_t smem;
-  const int BB = f64::pick_bb(P, batch, &smem);
-  DCCM_CUDA(cudaFuncSetAttribute(f64::fft64_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-  f64::fft64_forward_kernel<<<dim3(P.Jh, (batch + BB - 1) / BB), 32 * BB, smem, s>>>(a, P.N, P.J, batch, BB, grid,
-                                                                                     G, P.d_tw64);
-  DCCM_LAUNCH_CHECK();
-  return DCCM_OK;
+  return f64::with_shape(P.I, [&](auto sh) {
+    using Sh = decltype(sh);
+    const size_t smem = (size_t)Sh::BB * Sh::LD * sizeof(f64::C64);
+    DCCM_CUDA(cudaFuncSetAttribute(f64::fft_forward_kernel<Sh>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DCCM_CUDA(launch_pdl(f64::fft_forward_kernel<Sh>, dim3((unsigned)P.Jh * ((batch + Sh::BB - 1) / Sh::BB)), dim3(Sh::THREADS), smem,
+                         s, P.N, P.J, batch, grid, G, P.d_twfx, P.twfx0));
+    return DCCM_OK;
+  });
 }
 
 }  // namespace sht

@@ -93,7 +93,7 @@ __global__ void pnm_kernel(int N, int Jh, const double *__restrict__ mu, double 
 }
 
 static void destroy(Plan &P) {
-  void *ptrs[] = {P.d_mu,      P.d_w,        P.d_pnm,       P.d_tw64,  P.d_tw32,  P.d_twl32,
+  void *ptrs[] = {P.d_mu,      P.d_w,        P.d_pnm,       P.d_twfx,  P.d_tw32,  P.d_twl32,
                   P.tinv.d,    P.tfwd.d,     P.tinv.d_mi,   P.tfwd.d_mi, P.tinv.d_items,
                   P.tfwd.d_items, P.d_work,  P.d_err,       P.d_apack, P.d_punits, P.d_cexp,
                   P.d_wa_pos, P.d_wa_src, P.d_dig,     P.dinv.d_mem, P.dfwd.d_mem};
@@ -128,26 +128,29 @@ static int create(Plan &P, int N, int I, int J, int precision, int max_batch) {
   P.w.resize(J);
   DCCM_CUDA(cudaMemcpy(P.mu.data(), P.d_mu, J * sizeof(double), cudaMemcpyDeviceToHost));
   DCCM_CUDA(cudaMemcpy(P.w.data(), P.d_w, J * sizeof(double), cudaMemcpyDeviceToHost));
-  // FFT twiddles e^{-2 pi i t / I} in FP64 on the host.
-  // and, for the FP32 warp transform, the per-lane table e^{-2 pi i l k / I}
-  // at [k][l] (l < 32, k < I/32).
-  std::vector<double2> tw64(I);
-  std::vector<float2> tw32(I), twl32(I);
-  const double PI = acos(-1.0);
-  for (int t = 0; t < I; ++t) {
-    const double ang = 2.0 * PI * (double)t / (double)I;
-    tw64[t] = make_double2(cos(ang), -sin(ang));
-    tw32[t] = make_float2((float)tw64[t].x, (float)tw64[t].y);
-    const int k = t / 32, l = t % 32;
-    const double al = 2.0 * PI * (double)(l * k) / (double)I;
-    twl32[t] = make_float2((float)cos(al), (float)-sin(al));
+  if (precision == DCCM_SHT_FP64) {
+    std::vector<int4> tw;
+    DCCM_TRY(build_fft_f64(P, tw));
+    P.twfx0 = tw.back();
+    DCCM_CUDA(cudaMalloc(&P.d_twfx, tw.size() * sizeof(int4)));
+    DCCM_CUDA(cudaMemcpy(P.d_twfx, tw.data(), tw.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  } else {
+    // FFT twiddles e^{-2 pi i t / I} and the per-lane table e^{-2 pi i l k / I}
+    // at [k][l] (l < 32, k < I/32), rounded from FP64.
+    std::vector<float2> tw32(I), twl32(I);
+    const double PI = acos(-1.0);
+    for (int t = 0; t < I; ++t) {
+      const double ang = 2.0 * PI * (double)t / (double)I;
+      tw32[t] = make_float2((float)cos(ang), (float)-sin(ang));
+      const int k = t / 32, l = t % 32;
+      const double al = 2.0 * PI * (double)(l * k) / (double)I;
+      twl32[t] = make_float2((float)cos(al), (float)-sin(al));
+    }
+    DCCM_CUDA(cudaMalloc(&P.d_tw32, I * sizeof(float2)));
+    DCCM_CUDA(cudaMalloc(&P.d_twl32, I * sizeof(float2)));
+    DCCM_CUDA(cudaMemcpy(P.d_tw32, tw32.data(), I * sizeof(float2), cudaMemcpyHostToDevice));
+    DCCM_CUDA(cudaMemcpy(P.d_twl32, twl32.data(), I * sizeof(float2), cudaMemcpyHostToDevice));
   }
-  DCCM_CUDA(cudaMalloc(&P.d_tw64, I * sizeof(double2)));
-  DCCM_CUDA(cudaMalloc(&P.d_tw32, I * sizeof(float2)));
-  DCCM_CUDA(cudaMalloc(&P.d_twl32, I * sizeof(float2)));
-  DCCM_CUDA(cudaMemcpy(P.d_tw64, tw64.data(), I * sizeof(double2), cudaMemcpyHostToDevice));
-  DCCM_CUDA(cudaMemcpy(P.d_tw32, tw32.data(), I * sizeof(float2), cudaMemcpyHostToDevice));
-  DCCM_CUDA(cudaMemcpy(P.d_twl32, twl32.data(), I * sizeof(float2), cudaMemcpyHostToDevice));
   if (precision != DCCM_SHT_FP64) {
     // F (FP32, [m][j][2 max_batch]) and G3 (three BF16 or two FP16 planes,
     // rows of C2Bp) share the Fourier buffer.

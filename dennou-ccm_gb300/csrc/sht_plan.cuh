@@ -72,8 +72,9 @@ struct Plan {
   // device
   double *d_mu = nullptr, *d_w = nullptr;
   double *d_pnm = nullptr;     // FP64 Pbar(m, n, jj): [idx(m,n)][Jh]
-  double2 *d_tw64 = nullptr;   // FFT twiddles e^{-2 pi i t / I}
-  float2 *d_tw32 = nullptr;
+  int4 *d_twfx = nullptr;      // FP64 path: fixed-point FFT twiddles, forward then inverse (fft_f64.cu)
+  int4 twfx0 = {0, 0, 0, 0};   // the forward first pass's twiddle 1 with its scaling
+  float2 *d_tw32 = nullptr;    // mixed path: FFT twiddles e^{-2 pi i t / I}
   float2 *d_twl32 = nullptr;   // per-lane twiddles e^{-2 pi i l k / I} at [k][l], l < 32, k < I/32
   TileTable tinv, tfwd;        // bf16x3 tiles for the tensor path
   void *d_work = nullptr;      // Fourier buffer (F, G or G3), sized for max_batch
@@ -129,6 +130,7 @@ int inverse(Plan &P, const double *spec, double *grid, int batch, cudaStream_t s
 int forward(Plan &P, const double *grid, double *spec, int batch, cudaStream_t s);
 int build_tiles(Plan &P);
 int build_digits(Plan &P);
+int build_fft_f64(Plan &P, std::vector<int4> &h);
 
 }  // namespace sht
 }  // namespace dccm

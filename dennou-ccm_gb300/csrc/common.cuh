@@ -32,8 +32,8 @@ void set_cuda_error(cudaError_t e);
 struct Tunables {
   int tc_ctas = 0;        // persistent CTAs of the tensor-core Legendre kernel (at most one wave)
   int tc_shape = 0;       // tensor-core Legendre kernel: 0 wide, 1 narrow where the table allows (2 CTAs an SM)
-  int fft_bb = 0;         // warps per FFT CTA (4, 8, 16)
-  int fft_rpw = 0;        // row pairs per FFT warp where a row pair takes one warp (1, 2; 0: 1)
+  int fft_bb = 0;         // warps per FFT CTA (4, 8, 16; 0: by the rule of fft_multi)
+  int fft_rpw = 0;        // row pairs per FFT warp where a row pair takes one warp (1, 2; 0: by the rule of fft_multi)
   int flux_threads = 0;   // threads per CTA of the bulk-flux kernel
   int flux_ctas = 0;      // CTA cap of the bulk-flux kernel's grid-stride loop (0: 16 per SM)
   int remap_threads = 0;  // threads per CTA of the remap kernel

@@ -880,12 +880,29 @@ int fft_multi(Plan *const *plans, const int *batch, const void *const *in, void 
   // turn: half the warps for the same row pairs, twice the field-levels a
   // CTA (W = 3 rows keep one row pair a group).
   const size_t budget = 110 * 1024;  // two CTAs an SM
-  const int tb = tunables().fft_bb;
-  const int WPC = (tb == 4 || tb == 8 || tb == 16) ? tb : 8;
-  const int rpw = tunables().fft_rpw == 2 ? 2 : 1;
-  int rmax = 2, warps = 1;
-  for (int g = 0; g < ngroups; ++g)
+  const int tb = tunables().fft_bb, tr = tunables().fft_rpw;
+  int rmax = 2, warps = 1, wmin = 4;
+  long long wt = 0;  // warps that one row pair a warp (group) would take
+  for (int g = 0; g < ngroups; ++g) {
     if (!fft_length_supported(plans[g]->I)) return DCCM_ERR_UNSUPPORTED;
+    if (batch[g] <= 0) continue;
+    const int W = fft_warps_per_row(plans[g]->I / 32);
+    wmin = W < wmin ? W : wmin;
+    wt += (long long)plans[g]->Jh * batch[g] * W;
+  }
+  // Defaults where the knobs are 0.  Rows over three or four warps: 16 warps
+  // a CTA, so that a G3 run is wider (inverse / forward with their Legendre
+  // steps, 16 against 8 warps: T255 x 16 58 / 58 and 60 / 61 us, x 300 529 /
+  // 588 and 541 / 664 us; T341 x 4 66 / 70 and 66 / 73 us).  Two row pairs a
+  // warp halve the warps and widen the runs once the launch has warps for
+  // two waves: 60 an SM (T21 x 700 18.7 / 15.5 with two, 17.9 / 16.4 us with
+  // one; T63 x 200 24.2 / 23.9 and 24.9 / 23.7; T85 x 512 79.6 / 78.6 and
+  // 84.6 / 82.2; T170 x 40 41.6 / 41.5 and 43.4 / 44.3; below, T42 x 104
+  // 15.8 / 15.6 and 14.3 / 13.0, T127 x 60 33.9 / 35.0 and 30.1 / 31.3), 40
+  // for rows over four warps, whose CTAs are larger (T341 x 8 74 / 77 and
+  // 79 / 82 us, x 192 530 / 580 and 602 / 685; x 4 70 / 74 and 66 / 70).
+  const int WPC = (tb == 4 || tb == 8 || tb == 16) ? tb : (wmin >= 3 ? 16 : 8);
+  const int rpw = tr == 1 || tr == 2 ? tr : (wt >= (wmin == 4 ? 40LL : 60LL) * sm_count() ? 2 : 1);
   FftLaunch L;
   memset(&L, 0, sizeof L);
   int nblk = 0, ng = 0;

@@ -35,7 +35,7 @@ struct Tunables {
   int fft_bb = 0;         // warps per FFT CTA (4, 8, 16; 0: by the rule of fft_multi)
   int fft_rpw = 0;        // row pairs per FFT warp where a row pair takes one warp (1, 2; 0: by the rule of fft_multi)
   int flux_threads = 0;   // threads per CTA of the bulk-flux kernel
-  int flux_ctas = 0;      // CTA cap of the bulk-flux kernel's grid-stride loop (0: 16 per SM)
+  int flux_ctas = 0;      // CTA cap of the bulk-flux kernel's grid-stride loop (0: a thread a column)
   int remap_threads = 0;  // threads per CTA of the remap kernel
   int remap_fc = 0;       // fields per thread of the remap kernel (1, 2, 3, 4, 6; 0: 3, or all below 6)
   int serial = 0;         // 1: launch_pdl makes ordinary launches

@@ -553,7 +553,7 @@ int dccm_step_autotune_host(dccm_step *step, void *stream, const dccm_host_copy 
  * and the flux's kernels at the device's greatest priority, so that SMs
  * freed while both branches have CTAs waiting go to that branch first),
  * and, with a flux, "prio", "flux_threads" and "flux_ctas" (CTA cap of the
- * flux kernel's grid, 0: 16 per SM) together (3 x 3 x 4 candidates), on
+ * flux kernel's grid, 0: a thread a column) together (3 x 3 x 4 candidates), on
  * replays of the whole step graph,
  * where the two branches run concurrently; applies the winners and
  * records the step's graph again.  Every timed run follows a 256 MB

@@ -119,6 +119,21 @@ __device__ __forceinline__ UF one_plus(UF a) {
   return {(a.m >> 1) + (one >> 1), a.e + 1};
 }
 
+// a + b + c, rounded down at 2^-61 of the largest term; normalised.
+__device__ __forceinline__ UF sum3(UF a, UF b, UF c) {
+  const int e = max(max(a.e, b.e), c.e) + 2;
+  return norm({(a.m >> min(e - a.e, 63)) + (b.m >> min(e - b.e, 63)) + (c.m >> min(e - c.e, 63)), e});
+}
+// a - b into r (normalised, rounded at 2^-62 of the larger one); false unless
+// positive.
+__device__ __forceinline__ bool sub(UF a, UF b, UF &r) {
+  const int e = max(a.e, b.e) + 1;
+  const long long s = (long long)(a.m >> min(e - a.e, 63)) - (long long)(b.m >> min(e - b.e, 63));
+  const int z = __clzll(s);
+  r = {(u64)s << (z & 63), e - z};
+  return s > 0;
+}
+
 // e^x for x in 2^-58 units, |x| < 32.
 __device__ __forceinline__ UF exp_fix(long long x) {
   // n = floor(256 x / ln 2), at most a little below it, so that the rest r >= 0
@@ -159,6 +174,15 @@ __device__ __forceinline__ double rcp_d(double x) {
   const unsigned ef = hi >> 20 & 0x7FFu;
   if (ef - 16u >= 2016u) return 1.0 / x;
   const double y = to_double(rcp(from_double(x)));
+  return __hiloint2double(__double2hiint(y) | (int)(hi & 0x80000000u), __double2loint(y));
+}
+
+// x c for a double x and a constant c > 0, given as a UF within 2^+-100 and
+// as a double; c's UF {0, 0} or an x far from 1 takes the FP64 product.
+__device__ __forceinline__ double scale_d(double x, UF c, double cd) {
+  const unsigned hi = (unsigned)__double2hiint(x);
+  if ((hi >> 20 & 0x7FFu) - 128u >= 1790u || c.m == 0) return x * cd;
+  const double y = to_double(mul(from_double(x), c));
   return __hiloint2double(__double2hiint(y) | (int)(hi & 0x80000000u), __double2loint(y));
 }
 

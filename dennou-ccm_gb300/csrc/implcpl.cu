@@ -13,15 +13,13 @@
 // reference keeps as module state for the backward sweep are written once
 // and never re-read.
 //
-// FP64 throughout.  Divisions are the scarce operation on this GPU (the
-// FP64 pipe is 1/64 of FP32), so the elimination computes one reciprocal
-// of (M(k,-1) M(k+1,0)) per level and matrix and multiplies every
-// right-hand side by it (the momentum matrix serves U and V, the tracer
-// matrix every tracer), the mass term uses 1 / (g 2 dt), and each level's
-// full Exner function is inverted once.  The reciprocals are fp64::rcp
-// (an FP32 seed and one cubic Newton step: 3 DFMA, within half an ulp
-// and a little; zeros, infinities and out-of-range values take the exact
-// division).  Results agree with the reference's operation order to
+// FP64 accuracy throughout.  The FP64 pipe is the scarce one on this GPU
+// (1/64 of FP32), so reciprocals and products of positive numbers run with
+// 64-bit mantissas on the integer pipes (fx64.cuh; zeros, infinities and
+// out-of-range values take FP64 divisions), one reciprocal per level and
+// matrix serves every right-hand side (the momentum matrix serves U and V,
+// the tracer matrix every tracer), the mass term uses 1 / (g 2 dt), and each
+// level's full Exner function is inverted once.  Results agree with the reference's operation order to
 // rounding (the tests hold 1e-13).  Level 1
 // of the eliminated systems divides by the zero sub-diagonal the reference
 // sets at k = 1 (:199, :237, :272), as the reference does: the coupler
@@ -30,7 +28,7 @@
 #include <new>
 
 #include "common.cuh"
-#include "fp64_fast.cuh"
+#include "fx64.cuh"
 #include "nvtx.cuh"
 
 struct dccm_implcpl {
@@ -48,10 +46,12 @@ struct Fwd {
   const double *MomX, *MomY, *Heat, *QFlx, *P, *Ef, *Eh, *Tv, *Z, *Kv, *Kt, *Kq;
   double *DU, *DV, *DT, *DQ, *C1, *C2;
   double *uv, *tm, *qm;
-  double *G, *IEF;  // per (level, column) factors shared by the systems (geo_kernel)
+  double *G, *IEF, *Mass;  // per (level, column) factors shared by the systems (geo_kernel)
   long long ncol;
   int kmax, ncmax, ih2o;
   double Grav, CpDry, GasR, inv_g2dt;
+  fx::UF uCp, uGasR;  // CpDry and GasR for the integer arithmetic
+  bool fast;          // both positive and within 2^+-100
 };
 
 // One thread per (column, system): blockIdx.y 0 = momentum (U and V share
@@ -62,29 +62,86 @@ struct Fwd {
 // of the level above; the eliminated matrix and tendencies are written
 // once.  The level inputs are fetched LV levels ahead into registers, so
 // the loads of a chunk overlap while the serial elimination runs.
-constexpr int LV = 4;   // forward sweep: levels fetched ahead
+//
+// With the couplings' magnitudes l = -M(k,-1), u = -M(k,1) and a = -M(k+1,0),
+// all positive in an ordinary column, the elimination
+//   M(k,0) <- (M(k,0) M(k+1,0) - M(k,1)) / (M(k,-1) M(k+1,0)), and the same
+//   of the right-hand side,
+// is, with c = u / a,
+//   a <- (M(k,0) - c) / l,   r <- (c r - b) / l
+// (with q = 1 / a carried: c = u q, q <- l / (M(k,0) - c)): products and reciprocals of positive numbers, which run with 64-bit
+// mantissas on the integer pipes (fx64.cuh), and a few signed sums in FP64.
+// The top and bottom rows, and rows where a coupling is zero, negative, not
+// finite or beyond 2^+-100, take the reference's form in FP64 (a warp
+// decides as one).  FP64 was the sweeps' limit (67 operations a column and
+// level forward, 21 backward; now 12 and 8): 32,768 columns x 32 levels forward
+// 174 -> 95 us, backward 71 -> 35 us; 131,072 x 48 849 -> 397 and 253 -> 172 us.
+// What is left is the sum of three pipes' work (the ALU's about as long as
+// FP64's) with five warps a scheduler; two levels fetched ahead at 102
+// registers and five CTAs an SM beat four at 128 (95 against 99, 397 against
+// 401 us).
+constexpr int LV = 2;   // forward sweep: levels fetched ahead
 constexpr int LVB = 8;  // backward sweep
+
+// positive, exponent field in [lo, hi]
+__device__ __forceinline__ bool pos_in(double x, unsigned lo, unsigned hi) {
+  return ((unsigned)__double2hiint(x) >> 20) - lo <= hi - lo;
+}
+// -x by the sign bit (a negation that stays a value of its own costs a DADD)
+__device__ __forceinline__ double negd(double x) {
+  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
+}
+__device__ __forceinline__ bool usual(double x) { return pos_in(x, 923, 1123); }
 
 // The factors every system's row uses, once per (level, column) instead of
 // once per system: G(j) = P_h(j) / (R Tv_h(j) (z(j+1) - z(j))) at half level
-// j = 1..kmax-1 (the transfer coefficient of :182-195 is K(j) G(j)), and the
+// j = 1..kmax-1 (the transfer coefficient of :182-195 is K(j) G(j)), the
 // reciprocal Exner function 1 / Exner_f(j) at full level j (0-based index,
-// the temperature rows of :222-260).  Same expressions; G as a product
-// with the reciprocal.
+// the temperature rows of :222-260), and the mass term of that level's row.
 __global__ void __launch_bounds__(256) geo_kernel(const Fwd a) {
   const long long n = a.ncol;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= n * a.kmax) return;
   const int j = (int)(t / n);
   const long long c = t - j * n;
-  a.IEF[t] = fp64::rcp(a.Ef[c + n * j]);
-  if (j >= 1)
-    a.G[t] = a.P[c + n * j] * fp64::rcp(a.GasR * a.Tv[c + n * j] * (a.Z[c + n * j] - a.Z[c + n * (j - 1)]));
+  const double P0 = a.P[c + n * j];
+  a.Mass[t] = (P0 - a.P[c + n * (j + 1)]) * a.inv_g2dt;
+  a.IEF[t] = fx::rcp_d(a.Ef[c + n * j]);
+  if (j >= 1) {
+    const double Tv = a.Tv[c + n * j], dz = a.Z[c + n * j] - a.Z[c + n * (j - 1)];
+    double g;
+    if (a.fast && usual(P0) && usual(Tv) && usual(dz)) {
+      using namespace fx;
+      const UF d = mul(mul(from_double(Tv), a.uGasR), from_double(dz));
+      g = to_double(mul(from_double(P0), rcp(norm(d))));
+    } else {
+      g = P0 * fx::rcp_d(a.GasR * Tv * dz);
+    }
+    a.G[t] = g;
+  }
+}
+
+// Row k eliminated as the reference does, in FP64 (top: the row at the model
+// top).  A call of its own, so that its FP64 operations are not issued,
+// predicated off, on the rows that do not take it.
+struct Row {
+  double m0, r[2];
+};
+static __device__ __noinline__ Row eliminate_fp64(bool top, double mm, double m0, double mp, double m0p, double b0,
+                                                  double b1, double rp0, double rp1) {
+  Row w;
+  const double inv = fx::rcp_d(top ? mm : mm * m0p);
+  w.m0 = top ? m0 * inv : (m0 * m0p - mp) * inv;
+  w.r[0] = top ? b0 * inv : (b0 * m0p - mp * rp0) * inv;
+  w.r[1] = top ? b1 * inv : (b1 * m0p - mp * rp1) * inv;
+  return w;
 }
 
 template <int SYS>
 __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tracer) {
+  using fx::UF;
   constexpr int NR = SYS == 0 ? 2 : 1;
+  const unsigned warp = __activemask();
   const long long n = a.ncol;
   const int K = a.kmax;
   const long long mstr = n * K;
@@ -106,20 +163,24 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
   double *mat = SYS == 0 ? a.uv : (SYS == 1 ? a.tm : a.qm);
   const bool store_mat = SYS != 2 || tracer == 0;
   // values at level k carried from the previous (upper) iteration
-  double Pk = a.P[c + n * K], Ehk = a.Eh[c + n * K];
   double flk[NR];
 #pragma unroll
   for (int r = 0; r < NR; ++r) flk[r] = fl[r][c + n * K];
-  double tck = 0.0, ief_k1 = 0.0, ief_k = a.IEF[c + n * (K - 1)];
-  double m0p = 0.0, rp[NR], m0_2 = 0.0, r_2[NR], c2[NR], tc1 = 0.0, dfadt1 = 0.0, dfadt2 = 0.0;
+  double Kdk = 0.0, Gk = 0.0, Ehk = 0.0;  // of half level k (0 at the top)
+  double ief_k1 = 0.0, ief_k = SYS == 1 ? a.IEF[c + n * (K - 1)] : 0.0;
+  double m0p = 0.0, rp[NR] = {}, m0_2 = 0.0, r_2[NR], c2[NR], tc1 = 0.0, dfadt1 = 0.0, dfadt2 = 0.0;
+  // the integer forms: the transfer coefficient of half level k (SYS 1: times
+  // Cp Exner_h), 1 / a
+  UF upU{1ull << 63, 0}, qU{1ull << 63, 0};
+  bool upv = false, qv = false;
   for (int k0 = K; k0 >= 1; k0 -= LV) {
     // fetch half level k-1 and full level k-1 of the next LV levels
-    double Pm[LV], Gm[LV], Kdm[LV], Ehm[LV], Iefm[LV], flm[LV][NR];
+    double Mm[LV], Gm[LV], Kdm[LV], Ehm[LV], Iefm[LV], flm[LV][NR];
 #pragma unroll
     for (int i = 0; i < LV; ++i) {
       const int k = k0 - i;
       if (k >= 1) {
-        Pm[i] = a.P[c + n * (k - 1)];
+        Mm[i] = a.Mass[c + n * (k - 1)];
         if (k > 1) {
           Gm[i] = a.G[c + n * (k - 1)];
           Kdm[i] = Kd[c + n * (k - 1)];
@@ -136,46 +197,80 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
     for (int i = 0; i < LV; ++i) {
       const int k = k0 - i;
       if (k < 1) break;
-      // transfer coefficient at half level k-1 (0 at the surface, :182-195)
-      double tkm = 0.0, ief_km = 0.0;
+      const double ief_km = SYS == 1 && k > 1 ? Iefm[i] : 0.0;
+      // transfer coefficient of half level k-1 (SYS 1: times Cp Exner_h)
+      UF lowU{1ull << 63, 0};
+      bool lv = false;
       if (k > 1) {
-        tkm = Kdm[i] * Gm[i];
-        if (SYS == 1) ief_km = Iefm[i];
+        lv = a.fast && usual(Kdm[i]) && usual(Gm[i]);
+        if (SYS == 1) lv = lv && usual(Ehm[i]) && usual(ief_km);
+        lowU = fx::mul(fx::from_double(Kdm[i]), fx::from_double(Gm[i]));
+        if (SYS == 1) lowU = fx::mul(fx::mul(lowU, a.uCp), fx::from_double(Ehm[i]));
+        lowU = fx::norm(lowU);
       }
-      const double mass = -(Pk - Pm[i]) * a.inv_g2dt;
-      double mm, m0, mp;  // row k; +0 where the reference assigns 0
-      if constexpr (SYS != 1) {
-        mm = k > 1 ? -tkm : 0.0;
-        m0 = mass + tkm + tck;
-        mp = k < K ? -tck : 0.0;
-      } else {
-        const double ehm = k > 1 ? a.CpDry * Ehm[i] * tkm : 0.0;
-        const double ehk = a.CpDry * Ehk * tck;
-        mm = k > 1 ? -(ehm * ief_km) : 0.0;
-        m0 = a.CpDry * mass + ehm * ief_k + ehk * ief_k;
-        mp = k < K ? -(ehk * ief_k1) : 0.0;
-        if (k == 1) {
-          dfadt1 = ehk * ief_k;  // DFADT1 = Cp Exner_h(1) TTC(1) / Exner_f(1)
-          dfadt2 = mp;           // DFADT2 = -Cp Exner_h(1) TTC(1) / Exner_f(2)
+      double b[NR], re[NR], m0e;
+#pragma unroll
+      for (int r = 0; r < NR; ++r) b[r] = flm[i][r] - flk[r];
+      bool done = false;
+      if (__all_sync(warp, lv && upv && qv && usual(Mm[i]))) {
+        // row k: its diagonal mass + l' + u', the couplings l and u (SYS 1: the
+        // couplings with their own level's Exner function, l' and u' with k's)
+        UF mU = fx::from_double(Mm[i]), l = lowU, u = upU, l0 = lowU, u0 = upU;
+        if (SYS == 1) {
+          const UF ik = fx::from_double(ief_k);
+          mU = fx::mul(mU, a.uCp);
+          l0 = fx::mul(lowU, ik);
+          u0 = fx::mul(upU, ik);
+          l = fx::norm(fx::mul(lowU, fx::from_double(ief_km)));
+          u = fx::mul(upU, fx::from_double(ief_k1));
+        }
+        const UF cU = fx::mul(u, qU);
+        UF dU;
+        if (__all_sync(warp, fx::sub(fx::sum3(mU, l0, u0), cU, dU))) {
+          const UF iU = fx::rcp(l);
+          qU = fx::mul(l, fx::rcp(dU));
+          const double il = fx::to_double(iU), cc = fx::to_double(cU);
+          m0e = negd(fx::to_double(fx::mul(dU, iU)));
+#pragma unroll
+          for (int r = 0; r < NR; ++r) re[r] = fma(cc, rp[r], -b[r]) * il;
+          done = true;
         }
       }
-      if (k == 1) tc1 = tck;
-      double inv, m0e;
-      if (k == K) {
-        inv = fp64::rcp(mm);
-        m0e = m0 * inv;
-      } else {
-        inv = fp64::rcp(mm * m0p);
-        m0e = (m0 * m0p - mp) * inv;
+      if (!done) {
+        // row k as the reference builds (:182-256) and eliminates it; +0
+        // where it assigns 0
+        const double tkm = k > 1 ? Kdm[i] * Gm[i] : 0.0, tck = Kdk * Gk;
+        double mm, m0, mp;
+        if constexpr (SYS != 1) {
+          m0 = Mm[i] + tkm + tck;
+          mm = k > 1 ? -tkm : 0.0;
+          mp = k < K ? -tck : 0.0;
+          if (k == 1) tc1 = tck;
+        } else {
+          const double ehm = k > 1 ? a.CpDry * Ehm[i] * tkm : 0.0, ehk = a.CpDry * Ehk * tck;
+          m0 = a.CpDry * Mm[i] + ehm * ief_k + ehk * ief_k;
+          mm = k > 1 ? -(ehm * ief_km) : 0.0;
+          mp = k < K ? -(ehk * ief_k1) : 0.0;
+          if (k == 1) {
+            dfadt1 = ehk * ief_k;  // DFADT1 = Cp Exner_h(1) TTC(1) / Exner_f(1)
+            dfadt2 = mp;           // DFADT2 = -Cp Exner_h(1) TTC(1) / Exner_f(2)
+          }
+        }
+        const Row w = eliminate_fp64(k == K, mm, m0, mp, m0p, b[0], b[NR - 1], rp[0], rp[NR - 1]);
+        m0e = w.m0;
+        re[0] = w.r[0];
+        if (NR == 2) re[NR - 1] = w.r[1];
+        qU = fx::rcp(fx::from_double(negd(m0e)));
       }
+      qv = pos_in(negd(m0e), 723, 1323);
+      upU = lowU;
+      upv = lv;
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
-        const double b = -(flk[r] - flm[i][r]);
-        if (k == 1) c2[r] = b;  // ImplCplCoef2 starts from the level-1 divergence (:310-313)
-        const double re = k == K ? b * inv : (b * m0p - mp * rp[r]) * inv;
-        out[r][c + n * (k - 1)] = re;
-        rp[r] = re;
-        if (k == 2) r_2[r] = re;
+        if (k == 1) c2[r] = b[r];  // ImplCplCoef2 starts from the level-1 divergence (:310-313)
+        out[r][c + n * (k - 1)] = re[r];
+        rp[r] = re[r];
+        if (k == 2) r_2[r] = re[r];
         flk[r] = flm[i][r];
       }
       if (store_mat) {
@@ -185,16 +280,18 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
       }
       if (k == 2) m0_2 = m0e;
       m0p = m0e;
-      tck = tkm;
       ief_k1 = ief_k;
       ief_k = ief_km;
-      Pk = Pm[i];
-      if (SYS == 1 && k > 1) Ehk = Ehm[i];
+      if (k > 1) {
+        Kdk = Kdm[i];
+        Gk = Gm[i];
+        if (SYS == 1) Ehk = Ehm[i];
+      }
     }
   }
   // coupling coefficients (:342-375); DFADUV1 = -DFADUV2 = TC(1)
-  const double Tmp = -(a.P[c + n] - a.P[c]) * a.inv_g2dt;
-  const double i2 = fp64::rcp(m0_2);
+  const double Tmp = a.Mass[c];
+  const double i2 = fx::rcp_d(m0_2);
   if constexpr (SYS == 0) {
     const double cu = Tmp + tc1 + tc1 * i2;
     a.C1[c + n * 0] = cu;
@@ -212,7 +309,7 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
   }
 }
 
-__global__ void __launch_bounds__(128) forward_kernel(const Fwd a) {
+__global__ void __launch_bounds__(128, 5) forward_kernel(const Fwd a) {
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= a.ncol) return;
   if (blockIdx.y == 0) forward_column<0>(a, c, 0);
@@ -224,27 +321,30 @@ __global__ void __launch_bounds__(128) forward_kernel(const Fwd a) {
 // thread per (column, matrix): blockIdx.y 0 = momentum (U and V), 1 =
 // temperature, 2 = the tracers; one reciprocal of M(k,0) per level serves
 // every right-hand side of the matrix, and levels are fetched LVB at a time
-// ahead of the serial chains.
+// ahead of the serial chains.  M(k,-1) is 1 after the forward sweep and is
+// not read; the reciprocals and the products with 1 / (2 dt) run on the
+// integer pipes.
 struct Bwd {
   const double *uv, *tm, *qm;
   double *DU, *DV, *DT, *DQ;
   long long ncol;
   int kmax, ncmax;
   double inv_2dt;
+  fx::UF u2dt;  // inv_2dt
 };
 
 template <int NR>
 __device__ __forceinline__ void backward_chains(const double *__restrict__ mat, double *const *x, long long c,
-                                                long long n, int K, double inv_2dt) {
+                                                long long n, int K, double inv_2dt, fx::UF u2dt) {
   const long long mstr = n * K;
   double v[NR];
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
     v[r] = x[r][c];
-    x[r][c] = v[r] * inv_2dt;
+    x[r][c] = fx::scale_d(v[r], u2dt, inv_2dt);
   }
   for (int k0 = 2; k0 <= K; k0 += LVB) {
-    double xs[LVB][NR], mm[LVB], m0[LVB];
+    double xs[LVB][NR], m0[LVB];
 #pragma unroll
     for (int i = 0; i < LVB; ++i) {
       const int k = k0 + i;
@@ -252,7 +352,6 @@ __device__ __forceinline__ void backward_chains(const double *__restrict__ mat, 
         const long long o = c + n * (k - 1);
 #pragma unroll
         for (int r = 0; r < NR; ++r) xs[i][r] = x[r][o];
-        mm[i] = mat[o];
         m0[i] = mat[o + mstr];
       }
     }
@@ -260,11 +359,11 @@ __device__ __forceinline__ void backward_chains(const double *__restrict__ mat, 
     for (int i = 0; i < LVB; ++i) {
       const int k = k0 + i;
       if (k > K) break;
-      const double im = fp64::rcp(m0[i]);
+      const double im = fx::rcp_d(m0[i]);
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
-        v[r] = (xs[i][r] - mm[i] * v[r]) * im;
-        x[r][c + n * (k - 1)] = v[r] * inv_2dt;
+        v[r] = (xs[i][r] - v[r]) * im;
+        x[r][c + n * (k - 1)] = fx::scale_d(v[r], u2dt, inv_2dt);
       }
     }
   }
@@ -277,19 +376,19 @@ __global__ void __launch_bounds__(128) backward_kernel(const Bwd a) {
   const int K = a.kmax;
   if (blockIdx.y == 0) {
     double *x[2] = {a.DU, a.DV};
-    backward_chains<2>(a.uv, x, c, n, K, a.inv_2dt);
+    backward_chains<2>(a.uv, x, c, n, K, a.inv_2dt, a.u2dt);
   } else if (blockIdx.y == 1) {
     double *x[1] = {a.DT};
-    backward_chains<1>(a.tm, x, c, n, K, a.inv_2dt);
+    backward_chains<1>(a.tm, x, c, n, K, a.inv_2dt, a.u2dt);
   } else {
     // tracers in pairs (one reciprocal per level for both)
     for (int t = 0; t < a.ncmax; t += 2) {
       if (t + 1 < a.ncmax) {
         double *x[2] = {a.DQ + n * (long long)K * t, a.DQ + n * (long long)K * (t + 1)};
-        backward_chains<2>(a.qm, x, c, n, K, a.inv_2dt);
+        backward_chains<2>(a.qm, x, c, n, K, a.inv_2dt, a.u2dt);
       } else {
         double *x[1] = {a.DQ + n * (long long)K * t};
-        backward_chains<1>(a.qm, x, c, n, K, a.inv_2dt);
+        backward_chains<1>(a.qm, x, c, n, K, a.inv_2dt, a.u2dt);
       }
     }
   }
@@ -315,8 +414,8 @@ extern "C" int dccm_implcpl_create(int ncol, int kmax, int ncmax, int index_h2ov
   p->ih2o = index_h2ovap;
   p->k = *consts;
   // the three matrices (3 diagonals each), then the forward sweep's shared
-  // factors G and 1/Exner_f (kmax x ncol each)
-  const cudaError_t e = cudaMalloc(&p->d_mtx, (size_t)(3 * 3 + 2) * kmax * ncol * sizeof(double));
+  // factors G, 1/Exner_f and the mass term (kmax x ncol each)
+  const cudaError_t e = cudaMalloc(&p->d_mtx, (size_t)(3 * 3 + 3) * kmax * ncol * sizeof(double));
   if (e != cudaSuccess) {
     set_cuda_error(e);
     delete p;
@@ -337,6 +436,9 @@ extern "C" int dccm_implcpl_destroy(dccm_implcpl *p) {
 }
 
 static size_t mstride(const dccm_implcpl *p) { return (size_t)3 * p->kmax * p->ncol; }
+
+// A constant the integer arithmetic takes: positive, within 2^+-100.
+static bool ordinary(double x) { return x > 0x1p-100 && x < 0x1p100; }
 
 extern "C" int dccm_implcpl_forward_dev(dccm_implcpl *p, const dccm_implcpl_forward_args *a, void *stream) {
   DCCM_NVTX_FUNC();
@@ -379,6 +481,10 @@ extern "C" int dccm_implcpl_forward_dev(dccm_implcpl *p, const dccm_implcpl_forw
   f.inv_g2dt = 1.0 / (p->k.Grav * (2.0 * p->k.DelTime));
   f.G = p->d_mtx + 3 * mstride(p);
   f.IEF = f.G + (size_t)p->kmax * p->ncol;
+  f.Mass = f.IEF + (size_t)p->kmax * p->ncol;
+  f.fast = ordinary(f.CpDry) && ordinary(f.GasR);
+  f.uCp = fx::uf(f.fast ? f.CpDry : 1.0);
+  f.uGasR = fx::uf(f.fast ? f.GasR : 1.0);
   const long long nk = (long long)p->ncol * p->kmax;
   implcpl::geo_kernel<<<(unsigned)((nk + 255) / 256), 256, 0, as_stream(stream)>>>(f);
   DCCM_LAUNCH_CHECK();
@@ -405,6 +511,8 @@ extern "C" int dccm_implcpl_backward_dev(dccm_implcpl *p, double *xyz_DUDt, doub
   b.kmax = p->kmax;
   b.ncmax = p->ncmax;
   b.inv_2dt = 1.0 / (2.0 * p->k.DelTime);
+  // an exponent that sends every product to the FP64 form where 1 / (2 dt) is not ordinary
+  b.u2dt = ordinary(b.inv_2dt) ? fx::uf(b.inv_2dt) : fx::UF{0, 0};
   const int threads = 128;
   implcpl::backward_kernel<<<dim3((unsigned)((p->ncol + threads - 1) / threads), 3), threads, 0,
                              as_stream(stream)>>>(b);

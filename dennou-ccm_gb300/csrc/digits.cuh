@@ -6,7 +6,7 @@
 // mantissas exact down to 2^-9 of the vector's largest binade and rounded
 // at 2^-62 of it below), and Q in seven balanced digits of 9 bits,
 //   a = 2^(E-1030) sum_{i=1..7} d_i 2^(-9 (i-1)),  |d_i| <= 256,
-// every one a BF16 number exactly.  Products of digits are integers of at
+// every one an FP16 number exactly.  Products of digits are integers of at
 // most 2^16, so FP32 accumulation of up to 2^24 / 2^16 of them is exact.
 #pragma once
 #include <cuda_runtime.h>
@@ -24,105 +24,107 @@ __device__ __forceinline__ int dg_exp(unsigned maxmag) {
   return e < 1 ? 1 : e;
 }
 
-// Q of x for scale exponent E, with half of each lower digit's range added
-// so that the digits come off as plain bit fields.
+// Q of x for scale exponent E (at least that of the vector), with 256 added
+// to every digit so that they come off as plain bit fields.
 __device__ __forceinline__ unsigned long long dg_fixed(double x, int E) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const int ef = (int)(b >> 52) & 0x7FF;
-  const unsigned long long mant = (b & 0xFFFFFFFFFFFFFull) | (ef ? 0x10000000000000ull : 0ull);
-  const int sh = 9 + (ef ? ef : 1) - E;  // <= 9
-  unsigned long long q;
-  if (sh >= 0) q = mant << sh;
-  else q = sh < -60 ? 0ull : ((mant >> (-sh - 1)) + 1ull) >> 1;
-  if ((long long)b < 0) q = 0ull - q;
+  // the 53-bit mantissa at bits 10 .. 62, moved down by E - ef + 1, rounded
+  const unsigned long long m = ((b << 10) & 0x3FFFFFFFFFFFFC00ull) | (ef ? 1ull << 62 : 0ull);
+  const int r = min(E - max(ef, 1), 62);
+  const unsigned long long q = ((m >> r) + 1ull) >> 1;
   constexpr unsigned long long BIAS =
-      256ull * (1ull + (1ull << 9) + (1ull << 18) + (1ull << 27) + (1ull << 36) + (1ull << 45));
-  return q + BIAS;
+      256ull * (1ull + (1ull << 9) + (1ull << 18) + (1ull << 27) + (1ull << 36) + (1ull << 45) + (1ull << 54));
+  const unsigned long long s = (unsigned long long)((long long)b >> 63);
+  return (q ^ s) + (BIAS - s);
 }
 
-// Digit i = 1..7 of a biased Q as an FP32 number (low 16 bits zero: BF16 exact).
-template <int i> __device__ __forceinline__ float dg_digit(unsigned long long q) {
-  if constexpr (i == 1) {
-    const unsigned u = (unsigned)((int)(q >> 32) >> 22) & 1023u;  // signed, -256 .. 256 (mod 1024)
-    return __uint_as_float(0x4B000000u | ((u + 512u) & 1023u)) - 8389120.f;
-  } else {
-    const unsigned u = (unsigned)(q >> (9 * (7 - i))) & 511u;
-    return __uint_as_float(0x4B000000u | u) - 8388864.f;
-  }
+__device__ __forceinline__ unsigned sub_f16x2(unsigned a, unsigned b) {
+  unsigned r;
+  asm("sub.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
 }
-
-// Digit i of two values as one BF16 pair (a in the low half).
-template <int i> __device__ __forceinline__ unsigned dg_pair(unsigned long long a, unsigned long long b) {
-  return __byte_perm(__float_as_uint(dg_digit<i>(a)), __float_as_uint(dg_digit<i>(b)), 0x7632);
+// The digits in bits 0 .. 8 (FIELD 0), 9 .. 17 (1) or 0 .. 9 (2, the leading
+// digit) of two words as a pair of FP16 integers (a in the low half): the
+// fields become the low mantissa bits of 1024 + u, or one bit higher of 512 +
+// u, and the subtraction is exact.
+template <int FIELD> __device__ __forceinline__ unsigned dg_pair(unsigned a, unsigned b) {
+  if constexpr (FIELD == 1) return sub_f16x2((__byte_perm(a, b, 0x6521) & 0x03FE03FEu) | 0x60006000u, 0x62006200u);
+  const unsigned mask = FIELD == 0 ? 0x01FF01FFu : 0x03FF03FFu;
+  return sub_f16x2((__byte_perm(a, b, 0x5410) & mask) | 0x64006400u, 0x65006500u);
 }
 
 // The seven slices of eight values of one row (consecutive along K): one
 // 16-byte store per slice, slices `stride` bytes apart.
-template <int i = 1>
 __device__ __forceinline__ void dg_store8(unsigned char *dst, size_t stride, const unsigned long long (&q)[8]) {
-  *reinterpret_cast<uint4 *>(dst) =
-      make_uint4(dg_pair<i>(q[0], q[1]), dg_pair<i>(q[2], q[3]), dg_pair<i>(q[4], q[5]), dg_pair<i>(q[6], q[7]));
-  if constexpr (i < DG_SLICES) dg_store8<i + 1>(dst + stride, stride, q);
-}
-
-// 96-bit two's complement sum of drained accumulators.
-struct Dg96 {
-  unsigned w0, w1, w2;
-};
-
-// x += vh 2^36 + vl
-__device__ __forceinline__ void dg_add(Dg96 &x, long long vh, long long vl) {
-  const unsigned h0 = (unsigned)vh << 4, h1 = (unsigned)(vh >> 28);
-  const unsigned l0 = (unsigned)vl, l1 = (unsigned)(vl >> 32), l2 = (unsigned)((int)l1 >> 31);
-  asm("{\n\t.reg .u32 a, b;\n\t"
-      "add.cc.u32 a, %4, %6;\n\t"
-      "addc.u32 b, %5, %7;\n\t"
-      "add.cc.u32 %0, %0, %3;\n\t"
-      "addc.cc.u32 %1, %1, a;\n\t"
-      "addc.u32 %2, %2, b;\n\t}"
-      : "+r"(x.w0), "+r"(x.w1), "+r"(x.w2)
-      : "r"(l0), "r"(l1), "r"(l2), "r"(h0), "r"(h1));
-}
-__device__ __forceinline__ Dg96 dg_sum(const Dg96 &x, const Dg96 &y) {
-  Dg96 r;
-  asm("add.cc.u32 %0, %3, %6;\n\taddc.cc.u32 %1, %4, %7;\n\taddc.u32 %2, %5, %8;"
-      : "=&r"(r.w0), "=&r"(r.w1), "=r"(r.w2)
-      : "r"(x.w0), "r"(x.w1), "r"(x.w2), "r"(y.w0), "r"(y.w1), "r"(y.w2));
-  return r;
-}
-__device__ __forceinline__ Dg96 dg_diff(const Dg96 &x, const Dg96 &y) {
-  Dg96 r;
-  asm("sub.cc.u32 %0, %3, %6;\n\tsubc.cc.u32 %1, %4, %7;\n\tsubc.u32 %2, %5, %8;"
-      : "=&r"(r.w0), "=&r"(r.w1), "=r"(r.w2)
-      : "r"(x.w0), "r"(x.w1), "r"(x.w2), "r"(y.w0), "r"(y.w1), "r"(y.w2));
-  return r;
-}
-
-// x 2^ex as the nearest double (ties away from zero; bits below the top 64
-// of x are dropped, 2^-11 of the result's last place).
-__device__ __forceinline__ double dg_to_double(Dg96 x, int ex) {
-  const unsigned sgn = x.w2 & 0x80000000u;
-  if (sgn) x = dg_diff(Dg96{0, 0, 0}, x);
-  int be = ex + 95 + 1023;  // biased exponent of bit 95
+  unsigned w[8];
+  auto put = [&](int i, auto pair) {
+    *reinterpret_cast<uint4 *>(dst + i * stride) =
+        make_uint4(pair(w[0], w[1]), pair(w[2], w[3]), pair(w[4], w[5]), pair(w[6], w[7]));
+  };
+  auto low = [](unsigned a, unsigned b) { return dg_pair<0>(a, b); };
+  auto high = [](unsigned a, unsigned b) { return dg_pair<1>(a, b); };
+  auto top = [](unsigned a, unsigned b) { return dg_pair<2>(a, b); };
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
-    if (x.w2 == 0) {
-      x.w2 = x.w1;
-      x.w1 = x.w0;
-      x.w0 = 0;
-      be -= 32;
-    }
-  if (x.w2 == 0) return 0.0;
-  const int z = __clz((int)x.w2);
-  be -= z;
-  const unsigned mh = __funnelshift_l(x.w1, x.w2, z), ml = __funnelshift_l(x.w0, x.w1, z);
-  const unsigned long long mant = ((((unsigned long long)mh << 32) | ml) >> 11) + ((ml >> 10) & 1u);  // 53 bits, or 2^53
+  for (int e = 0; e < 8; ++e) w[e] = (unsigned)(q[e] >> 54);
+  put(0, top);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) w[e] = (unsigned)(q[e] >> 36);
+  put(1, high);
+  put(2, low);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) w[e] = (unsigned)(q[e] >> 18);
+  put(3, high);
+  put(4, low);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) w[e] = (unsigned)q[e];
+  put(5, high);
+  put(6, low);
+}
+
+// Sum of drained accumulators (levels s = 2 .. 8 of digit products, integers
+// below 2^24): t in units of level 6 (2^18 level-8 units), the two lowest
+// levels beside it in FP32 (its 24 bits reach 2^-61 of the largest product).
+// 1.01 K 2^52 < 2^63 for K products: K < 2,000.
+struct DgSum {
+  long long t;
+  float l;
+};
+__device__ __forceinline__ void dg_accumulate(DgSum &x, const unsigned (&r)[DG_SLICES]) {
+  int v[5];
+#pragma unroll
+  for (int s = 0; s < 5; ++s) v[s] = __float2int_rn(__uint_as_float(r[s]));
+  x.t += v[4];
+  x.t += (long long)v[3] * (1 << 9);
+  x.t += (long long)v[2] * (1 << 18);
+  x.t += (long long)v[1] * (1 << 27);
+  x.t += (long long)v[0] << 36;
+  x.l = fmaf(__uint_as_float(r[5]), 512.f, x.l) + __uint_as_float(r[6]);
+}
+
+// q 2^ex as the nearest double (ties away from zero).
+__device__ __forceinline__ double fixed_to_double(long long q, int ex) {
+  const long long s = q >> 63;
+  unsigned long long m = (unsigned long long)((q ^ s) - s);
+  const int z = __clzll((long long)m);
+  if (m == 0) return 0.0;
+  m <<= z;
+  const unsigned long long mant = (m >> 11) + ((unsigned)m >> 10 & 1u);  // 53 bits, or 2^53
+  const int be = ex + 63 - z + 1023;
   if ((unsigned)(be - 1) >= 2045u) {  // subnormal result or overflow
     const double r = ldexp((double)mant, be - 1075);
-    return sgn ? -r : r;
+    return s ? -r : r;
   }
-  const unsigned long long bits = ((unsigned long long)(be - 1) << 52) + mant;
-  return __longlong_as_double((long long)(bits | ((unsigned long long)sgn << 32)));
+  return __longlong_as_double((long long)((((unsigned long long)(unsigned)(be - 1) << 52) + mant) |
+                                          ((unsigned long long)s << 63)));
+}
+
+// x in units of 2^ex level-6 units, as the nearest double.
+__device__ __forceinline__ double dg_to_double(const DgSum &x, int ex) {
+  const int hi = (int)(x.t >> 32);
+  const int k = min(__clz(hi ^ (hi >> 31)) - 1, 10);  // room above t
+  const long long q = (x.t << k) + __float2int_rn(x.l * __int_as_float((k + 109) << 23));  // l 2^(k - 18)
+  return fixed_to_double(q, ex - k);
 }
 
 }  // namespace dccm

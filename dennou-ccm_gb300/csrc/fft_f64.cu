@@ -16,8 +16,8 @@
 //            so nothing overflows (|Z| <= sum |z|) and a pass rounds once,
 //            below 2^-53 of the row's r.m.s. for noise-like rows;
 //   inverse  every partial sum of the transform is bounded by the sum S of
-//            the input magnitudes, so the inputs are scaled with S at 2^61
-//            and no pass scales: roundings are a few 2^-61 S.
+//            the input magnitudes, so the inputs are scaled with S at 2^62
+//            and no pass scales: roundings are a few 2^-62 S.
 // Both are below the rounding errors of an FP64 transform (about 2.5e-16 of
 // the r.m.s.; measured errors of the whole transforms fell, see the tests).
 // A row pair that holds an infinity or NaN comes out NaN.
@@ -33,6 +33,7 @@
 #include <math.h>
 #include <string.h>
 
+#include "digits.cuh"
 #include "sht_plan.cuh"
 
 namespace dccm {
@@ -223,23 +224,6 @@ __device__ __forceinline__ long long to_fixed(double x, int rbase) {
   return (long long)b < 0 ? -q : q;
 }
 
-// q 2^ex as the nearest double (ties away from zero).
-__device__ __forceinline__ double to_double(long long q, int ex) {
-  const long long s = q >> 63;
-  unsigned long long m = (unsigned long long)((q ^ s) - s);
-  const int z = __clzll((long long)m);
-  if (m == 0) return 0.0;
-  m <<= z;
-  const unsigned long long mant = (m >> 11) + ((unsigned)m >> 10 & 1u);
-  const int be = ex + 63 - z + 1023;
-  if ((unsigned)(be - 1) >= 2045u) {  // subnormal result or overflow
-    const double r = ldexp((double)mant, be - 1075);
-    return s ? -r : r;
-  }
-  return __longlong_as_double((long long)((((unsigned long long)(unsigned)(be - 1) << 52) + mant) |
-                                          ((unsigned long long)s << 63)));
-}
-
 // One in-place pass over the buffer of a row pair: DFTs of radix R over
 // stride NS within blocks of R NS.  SG < 0: DFT, then twiddles (scaled);
 // SG > 0: twiddles, then DFT.
@@ -342,8 +326,8 @@ fft_forward_kernel(int N, int J, int batch, const double *__restrict__ grid, dou
     const C64 a = zb[Sh::pos(m)], c = zb[Sh::pos(m ? Sh::I - m : 0)];
     // 2A = (a.x + c.x, a.y - c.y), 2B = (a.y + c.y, c.x - a.x)
     const long long ar = a.x + c.x, ai = a.y - c.y, br = a.y + c.y, bi = c.x - a.x;
-    double2 e = make_double2(to_double(ar + br, ex), to_double(ai + bi, ex));
-    double2 o = make_double2(to_double(ar - br, ex), to_double(ai - bi, ex));
+    double2 e = make_double2(fixed_to_double(ar + br, ex), fixed_to_double(ai + bi, ex));
+    double2 o = make_double2(fixed_to_double(ar - br, ex), fixed_to_double(ai - bi, ex));
     if (m == 0) e.y = o.y = 0.0;
     if (E >= 2047) e = o = make_double2(nan, m ? nan : 0.0);
     out[(int64_t)(2 * m) * pst] = e;
@@ -398,10 +382,10 @@ fft_inverse_kernel(int N, int J, int batch, const double *__restrict__ F, double
   for (int i = 0; i < KI; ++i) sum += units(a[i].x) + units(a[i].y) + units(b[i].x) + units(b[i].y);
   atomicAdd(&ssum[bl], sum);
   __syncthreads();
-  // sum of |Re Z| + |Im Z| over all frequencies < 2^(nbit + 1) units -> 2^61:
-  // the mantissa moves by ef - E + 27 - nbit
+  // sum of |Re Z| + |Im Z| over all frequencies < 2^(nbit + 1) units -> 2^62:
+  // the mantissa moves by ef - E + 28 - nbit
   const int nbit = 32 - __clz((int)ssum[bl]);
-  const int rb = 10 - (27 - nbit) + E;
+  const int rb = 10 - (28 - nbit) + E;
   C64 *zb = buf + (size_t)bl * Sh::LD;
 #pragma unroll
   for (int i = 0; i < KI; ++i) {
@@ -429,14 +413,14 @@ fft_inverse_kernel(int N, int J, int batch, const double *__restrict__ F, double
   for (int q = 1; q < Sh::R1; ++q) v[q] = twmul<30>(v[q], __ldg(tw + (q - 1) * Sh::N1 + t));
   dft<1, Sh::R1>(v);
   const int Eg = max((int)(smx[g] >> 20), 1);
-  const int ex = Eg - 1075 - (27 - (32 - __clz((int)ssum[g])));
+  const int ex = Eg - 1075 - (28 - (32 - __clz((int)ssum[g])));
   const double nan = __longlong_as_double(0x7FF8000000000000ll);
   double *gn = grid + ((int64_t)(b0 + g) * J + jn) * Sh::I + t;
   double *gs = grid + ((int64_t)(b0 + g) * J + js) * Sh::I + t;
 #pragma unroll
   for (int p = 0; p < Sh::R1; ++p) {
-    gn[p * Sh::N1] = Eg >= 2047 ? nan : to_double(v[p].x, ex);
-    gs[p * Sh::N1] = Eg >= 2047 ? nan : to_double(v[p].y, ex);
+    gn[p * Sh::N1] = Eg >= 2047 ? nan : fixed_to_double(v[p].x, ex);
+    gs[p * Sh::N1] = Eg >= 2047 ? nan : fixed_to_double(v[p].y, ex);
   }
 }
 

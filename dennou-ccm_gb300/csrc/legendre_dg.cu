@@ -5,7 +5,7 @@
 // (1.05 TFLOP/s measured), and the contraction took 80 % of the plain FP64
 // transforms as an FP64 FMA loop (T341 x 192 field-levels: synthesis 10.4
 // ms, analysis 13.5 ms; T85 x 128: 209 and 340 us; with the kernels below
-// 0.78, 0.76 ms, 50 and 43 us, packs included).  Here every operand is
+// 0.56, 0.63 ms, 36 and 35 us, packs included).  Here every operand is
 // split into seven 9-bit digits (digits.cuh: the scheme of K. Ozaki, T.
 // Ogita, S. Oishi, S. Rump, "Error-free transformations of matrix
 // multiplication", Numer. Algorithms 59 (2012), with integer digits), and
@@ -39,8 +39,16 @@
 // accumulators s = i + j: a slice of A is read from shared memory once for
 // all of them.
 //
+// What bounds it (T341 x 192, parts taken out one by one): the packs 140 and
+// 250 us (the analysis pack moves 1.5 GB), the MMAs alone 277 us against 140
+// at the peak rate (short N: 7 MMAs of 32 to 224 columns a K step), draining
+// about 60 and storing 50-100 us, mostly behind the MMAs.  TN = 64 (half the
+// reads of A, 193-227 us of MMAs, but one accumulator set, whose drains the
+// MMAs then wait for) came out at 591 and 644 us against 571 and 626, and
+// 16 % slower at T85.  Sixteen epilogue warps instead of eight: 776 -> 710 us.
+//
 // A work item is (m, 128 columns c, TN rows of N).  Warp 0 copies, warp 1
-// allocates TMEM and issues the MMAs, warps 2-9 drain the accumulators
+// allocates TMEM and issues the MMAs, warps 2-17 drain the accumulators
 // (7 TMEM columns an output, integer arithmetic, one store).  Every wait is
 // bounded, as in legendre_tc.cu.
 #include <math.h>
@@ -58,17 +66,15 @@ constexpr int DG_KB = 4;                                       // chunks an accu
 constexpr int DG_ROW = 2 * DG_CHUNK;                           // bytes of a K-major row of a chunk
 constexpr int DG_A_SLICE = 128 * DG_ROW;                       // 8 KB
 constexpr int DG_A_BYTES = DG_SLICES * DG_A_SLICE;             // 56 KB
-constexpr int DG_EPI_WARPS = 8;
+constexpr int DG_EPI_WARPS = 16;
 constexpr int DG_THREADS = 64 + 32 * DG_EPI_WARPS;
 constexpr size_t DG_WORK_CAP = (size_t)4 << 30;                // A images of one launch
-template <int TN> struct DgShape {
-  static constexpr int B_BYTES = DG_SLICES * TN * DG_ROW;
-  static constexpr int STAGE = DG_A_BYTES + B_BYTES;
-  static constexpr int NSTAGE = TN == 32 ? 3 : 2;
-  static constexpr int NACC = TN == 32 ? 2 : 1;                // accumulator sets (7 TN columns each)
-  static constexpr int ACC_COLS = TN == 32 ? 256 : 512;
-  static constexpr int SMEM = 1024 + NSTAGE * STAGE + 256;
-};
+constexpr int TN = 32;                                         // rows of N an item
+constexpr int DG_B_BYTES = DG_SLICES * TN * DG_ROW;
+constexpr int DG_STAGE = DG_A_BYTES + DG_B_BYTES;              // 70 KB
+constexpr int DG_NSTAGE = 3;
+constexpr int DG_NACC = 2;                                     // accumulator sets (7 TN TMEM columns each)
+constexpr int DG_SMEM = 1024 + DG_NSTAGE * DG_STAGE + 256;
 
 struct DgMInfo {
   long long tab[2];  // first table tile of (m, p), bytes
@@ -87,6 +93,7 @@ struct DgArgs {
   int nitems;        // items per column tile
   int nchunk;        // A chunks per column tile
   int ldea;          // row length of ea
+  int enan;          // scale exponent from which an operand was not finite
   long long ncoef;
   const DgMInfo *mi;
   const int2 *items;           // (m, nt)
@@ -108,19 +115,41 @@ __device__ __forceinline__ uint64_t dg_desc(uint32_t addr) {
 // byte offset of 16-byte unit u (8 values of K) of row r in a swizzled slice
 __host__ __device__ __forceinline__ int dg_unit(int r, int u) { return r * DG_ROW + ((u ^ ((r >> 1) & 3)) << 4); }
 
+// The MMAs of one stage, ks K steps of 16, for a tile of NTW rows of N: slice
+// i of A with as many consecutive slices j of B as 256 columns hold, into
+// accumulators i + j.  Descriptors by constant offsets from the stage's two:
+// with them built anew for each MMA the issuing thread was the limit (T341 x
+// 192 with loads and epilogue taken out: synthesis 250, analysis 298 us).
+template <int NTW>
+__device__ __forceinline__ void dg_mma(uint32_t acc, uint64_t da, uint64_t db, int ks, int first) {
+  constexpr int PER = 256 / NTW;
+  for (int kk = 0; kk < ks; ++kk) {
+#pragma unroll
+    for (int i = 0; i < DG_SLICES; ++i)
+#pragma unroll
+      for (int j = 0; j < DG_SLICES - i; j += PER) {
+        const int n = DG_SLICES - i - j < PER ? DG_SLICES - i - j : PER;
+        mma_bf16(acc + (i + j) * NTW, da + (i * DG_A_SLICE >> 4), db + (j * NTW * DG_ROW >> 4),
+                 idesc_f16kind(n * NTW, 0, 0), i ? 1 : first);
+      }
+    first = 1;
+    da += 2;  // 32 bytes
+    db += 2;
+  }
+}
+
 __device__ __forceinline__ int dg_item(int k) {  // as cta_item: rounds in alternating directions
   const int G = (int)gridDim.x, b = (int)blockIdx.x;
   return (k & 1) ? (k + 1) * G - 1 - b : k * G + b;
 }
 
-template <int TN, int DIR>
+template <int DIR>
 __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid_constant__ DgArgs a) {
-  using Sh = DgShape<TN>;
-  constexpr int NSTAGE = Sh::NSTAGE, NACC = Sh::NACC;
+  constexpr int NSTAGE = DG_NSTAGE, NACC = DG_NACC;
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
   unsigned char *stage = reinterpret_cast<unsigned char *>(
       (reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-  uint64_t *bars = reinterpret_cast<uint64_t *>(stage + NSTAGE * Sh::STAGE);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(stage + NSTAGE * DG_STAGE);
   uint64_t *full = bars, *empty = bars + NSTAGE, *accf = bars + 2 * NSTAGE, *acce = accf + NACC;
   uint64_t *drain = bars + 15;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 16);
@@ -173,7 +202,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
           for (int q = 0; q < mi.nq[p]; ++q, ++g) {
             const int s = g % NSTAGE;
             if (!mbar_wait(&empty[s], ((g / NSTAGE) & 1) ^ 1, a.err, abort_flag, 1, a.wait_ns)) { ok = false; break; }
-            unsigned char *As = stage + s * Sh::STAGE;
+            unsigned char *As = stage + s * DG_STAGE;
             const unsigned char *Ag = a.A + ((long long)ct * a.nchunk + mi.ch[p] + q) * DG_A_BYTES;
             const uint32_t bb = (uint32_t)(DG_SLICES * DG_ROW * ntw);
             mbar_arrive_tx(&full[s], (uint32_t)(DG_SLICES * DG_ROW * rows) + bb);
@@ -205,32 +234,22 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
         for (int p = 0; p < 2 && ok; ++p) {
           if (nt * TN >= mi.nr[p]) continue;
           const int ntw = min(TN, mi.nr[p] - nt * TN);
-          const int per = 256 / ntw;  // slices of B an MMA can take
           for (int q0 = 0; q0 < mi.nq[p] && ok; q0 += DG_KB, ++seg) {
             const int set = seg % NACC;
             if (!mbar_wait(&acce[set], ((seg / NACC) & 1) ^ 1, a.err, abort_flag, 2, a.wait_ns)) { ok = false; break; }
             tc_fence_after();
-            const uint32_t acc = tmem + set * Sh::ACC_COLS;
+            const uint32_t acc = tmem + set * 256;
             int first = 0;  // 0 until the accumulators have been written
             for (int q = q0; q < min(mi.nq[p], q0 + DG_KB); ++q, ++g) {
               const int s = g % NSTAGE;
               if (!mbar_wait(&full[s], (g / NSTAGE) & 1, a.err, abort_flag, 3, a.wait_ns)) { ok = false; break; }
               tc_fence_after();
-              const uint32_t As = smem_u32(stage + s * Sh::STAGE), Bs = As + DG_A_BYTES;
+              const uint32_t As = smem_u32(stage + s * DG_STAGE);
+              const uint64_t da = dg_desc(As), db = dg_desc(As + DG_A_BYTES);
               const int ks = min(2, (mi.kv[p] - q * DG_CHUNK + 15) / 16);
-              for (int kk = 0; kk < ks; ++kk) {
-#pragma unroll
-                for (int i = 0; i < DG_SLICES; ++i) {
-                  const uint64_t da = dg_desc(As + i * DG_A_SLICE + kk * 32);
-                  // slices j = 0 .. 6 - i of B into accumulators i + j
-                  for (int j = 0; j < DG_SLICES - i; j += per) {
-                    const int n = min(per, DG_SLICES - i - j);
-                    mma_bf16(acc + (i + j) * ntw, da, dg_desc(Bs + j * ntw * DG_ROW + kk * 32),
-                             idesc_f16kind(n * ntw, 0, 1), first | i);
-                  }
-                }
-                first = 1;
-              }
+              if (ntw == TN) dg_mma<TN>(acc, da, db, ks, first);
+              else dg_mma<16>(acc, da, db, ks, first);
+              first = 1;
               mma_commit(&empty[s]);
             }
             if (ok) mma_commit(&accf[set]);
@@ -245,8 +264,9 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
     __syncwarp();
   } else {
     // ----------------------------------------------------- epilogue
-    constexpr int HC = TN / 16;               // groups of 8 columns a thread drains
-    const int quad = warp & 3, half = (warp - 2) >> 2;
+    // four warps a TMEM lane quarter, each with TN / 4 columns
+    constexpr int EC = TN / 4;
+    const int quad = warp & 3, j0 = ((warp - 2) >> 2) * EC;
     const int row = quad * 32 + lane;
     const int C2B = 2 * a.batch;
     int seg = 0;
@@ -258,14 +278,12 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
       const int c = a.c0 + ct * 128 + row;
       const bool live = c < C2B;
       // inverse: both parities' sums; forward: the current parity's
-      Dg96 sum[DIR == 0 ? 2 : 1][HC][8];
+      DgSum sum[DIR == 0 ? 2 : 1][EC];
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
-        Dg96(&S)[HC][8] = sum[DIR == 0 ? p : 0];
+        DgSum(&S)[EC] = sum[DIR == 0 ? p : 0];
 #pragma unroll
-        for (int h = 0; h < HC; ++h)
-#pragma unroll
-          for (int x = 0; x < 8; ++x) S[h][x] = Dg96{0, 0, 0};
+        for (int x = 0; x < EC; ++x) S[x] = DgSum{0, 0.f};
         if (nt * TN >= mi.nr[p]) continue;
         const int ntw = min(TN, mi.nr[p] - nt * TN);
         for (int q0 = 0; q0 < mi.nq[p]; q0 += DG_KB, ++seg) {
@@ -275,22 +293,18 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
             break;
           }
           tc_fence_after();
-          const uint32_t tb = tmem + ((uint32_t)(quad * 32) << 16) + set * Sh::ACC_COLS;
+          const uint32_t tb = tmem + ((uint32_t)(quad * 32) << 16) + set * 256 + j0;
+          if (j0 < ntw) {
 #pragma unroll
-          for (int h = 0; h < HC; ++h) {
-            const int j0 = 16 * h + 8 * half;
-            if (j0 < ntw) {
-              uint32_t r[DG_SLICES][8];
+            for (int h = 0; h < EC; h += 4) {
+              uint32_t v[DG_SLICES][4];
 #pragma unroll
-              for (int s = 0; s < DG_SLICES; ++s) tmem_ld8_nw(tb + s * ntw + j0, r[s]);
+              for (int s = 0; s < DG_SLICES; ++s) tmem_ld4_nw(tb + s * ntw + h, v[s]);
               tmem_wait_ld();
 #pragma unroll
-              for (int x = 0; x < 8; ++x) {
-                int v[DG_SLICES];
-#pragma unroll
-                for (int s = 0; s < DG_SLICES; ++s) v[s] = __float2int_rn(__uint_as_float(r[s][x]));
-                dg_add(S[h][x], (long long)v[0] * 262144 + ((long long)v[1] * 512 + v[2]),
-                       ((long long)v[3] * 512 + v[4]) * 262144 + ((long long)v[5] * 512 + v[6]));
+              for (int x = 0; x < 4; ++x) {
+                const uint32_t w7[DG_SLICES] = {v[0][x], v[1][x], v[2][x], v[3][x], v[4][x], v[5][x], v[6][x]};
+                dg_accumulate(S[h + x], w7);
               }
             }
           }
@@ -298,40 +312,36 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
           mbar_arrive(&acce[set]);
         }
         if (dead) break;
-        if (DIR == 1 && live) {
+        if (DIR == 1 && live && j0 < ntw) {
           // column k of the tile is n = m + p + 2 (nt TN + k)
           const int E = a.ea[(long long)(2 * m + p) * a.ldea + c];
+          const long long id0 = mi.eb[p] + p + 2 * (nt * TN + j0);
+          double *dst = a.out + ((long long)(c >> 1) * a.ncoef + id0) * 2 + (c & 1);
 #pragma unroll
-          for (int h = 0; h < HC; ++h)
-#pragma unroll
-            for (int x = 0; x < 8; ++x) {
-              const int kk = nt * TN + 16 * h + 8 * half + x;
-              if (kk < mi.nv[p] && 16 * h + 8 * half < ntw) {
-                const long long id = mi.eb[p] + p + 2 * kk;
-                double v = dg_to_double(S[h][x], E - 1022 + a.eb[id] - 70);
-                if (E >= 2047) v = __longlong_as_double(0x7FF8000000000000ll);
-                a.out[((long long)(c >> 1) * a.ncoef + id) * 2 + (c & 1)] = (m == 0 && (c & 1)) ? 0.0 : v;
-              }
+          for (int x = 0; x < EC; ++x)
+            if (nt * TN + j0 + x < mi.nv[p]) {
+              double v = dg_to_double(S[x], E - 1022 + a.eb[id0 + 2 * x] - 52);
+              if (E >= a.enan) v = __longlong_as_double(0x7FF8000000000000ll);
+              dst[4 * x] = (m == 0 && (c & 1)) ? 0.0 : v;
             }
         }
       }
       if (DIR == 0 && !dead && live) {
-        const int ntw = min(TN, mi.nr[0] - nt * TN);
         const int E = a.ea[(long long)m * a.ldea + c];
-        double *Fm = a.out + (long long)m * 2 * a.Jh * C2B + c;
+        const int jb = nt * TN + j0;
+        const short *eb = a.eb + mi.eb[0] + jb;
+        double *Fn = a.out + ((long long)m * 2 * a.Jh + a.Jh + jb) * C2B + c;      // latitude Jh + jj
+        double *Fs = a.out + ((long long)m * 2 * a.Jh + a.Jh - 1 - jb) * C2B + c;  // its mirror
 #pragma unroll
-        for (int h = 0; h < HC; ++h)
-#pragma unroll
-          for (int x = 0; x < 8; ++x) {
-            const int jj = nt * TN + 16 * h + 8 * half + x;
-            if (jj < a.Jh && 16 * h + 8 * half < ntw) {
-              const int ex = E - 1022 + a.eb[mi.eb[0] + jj] - 70;
-              double fn = dg_to_double(dg_sum(sum[0][h][x], sum[DIR == 0][h][x]), ex);
-              double fs = dg_to_double(dg_diff(sum[0][h][x], sum[DIR == 0][h][x]), ex);
-              if (E >= 2047) fn = fs = __longlong_as_double(0x7FF8000000000000ll);
-              Fm[(long long)(a.Jh + jj) * C2B] = fn;
-              Fm[(long long)(a.Jh - 1 - jj) * C2B] = fs;
-            }
+        for (int x = 0; x < EC; ++x)
+          if (jb + x < a.Jh) {
+            const int ex = E - 1022 + eb[x] - 52;
+            const DgSum &e = sum[0][x], &o = sum[DIR == 0][x];
+            double fn = dg_to_double(DgSum{e.t + o.t, e.l + o.l}, ex);
+            double fs = dg_to_double(DgSum{e.t - o.t, e.l - o.l}, ex);
+            if (E >= a.enan) fn = fs = __longlong_as_double(0x7FF8000000000000ll);
+            Fn[(long long)x * C2B] = fn;
+            Fs[-(long long)x * C2B] = fs;
           }
       }
     }
@@ -408,7 +418,7 @@ dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const doub
 template <int WQ>
 __global__ void __launch_bounds__(256)
 dg_pack_four(const DgMInfo *__restrict__ mi_, int Jh, int C2B, int c0, int nc, const double *__restrict__ Gf, int nchunk,
-             unsigned char *__restrict__ A, int *__restrict__ ea, int ldea) {
+             unsigned char *__restrict__ A, int *__restrict__ ea, int ldea, int guard) {
   __shared__ unsigned smx[8][8];
   pdl_wait();
   pdl_trigger();
@@ -439,7 +449,7 @@ dg_pack_four(const DgMInfo *__restrict__ mi_, int Jh, int C2B, int c0, int nc, c
     for (int k = 0; k < WQ; ++k) mx = max(mx, smx[warp / WQ * WQ + k][c8]);
   }
   if (!live) return;
-  const int E = dg_exp(mx);
+  const int E = dg_exp(mx) + guard;
   if (u == 0 && warp % WQ == 0) ea[(long long)mp * ldea + c0 + cl] = E;
   const int ct = cl / 128, row = cl % 128;
   const bool keep = nq <= WQ;
@@ -479,7 +489,7 @@ __global__ void dg_row_scale(int dir, int N, int Jh, const double *__restrict__ 
 
 // Table tiles: thread = (m, p, row of N, unit of 8 along K).
 __global__ void __launch_bounds__(256)
-dg_build(int dir, int N, int Jh, int TN, const DgMInfo *__restrict__ mi_, const double *__restrict__ pnm,
+dg_build(int dir, int N, int Jh, const DgMInfo *__restrict__ mi_, const double *__restrict__ pnm,
          const double *__restrict__ w, const short *__restrict__ eb, unsigned char *__restrict__ B) {
   const int m = blockIdx.y, p = blockIdx.z;
   const DgMInfo &mi = mi_[m];
@@ -508,7 +518,6 @@ dg_build(int dir, int N, int Jh, int TN, const DgMInfo *__restrict__ mi_, const 
 }
 
 // ------------------------------------------------------------------ host
-constexpr int DG_TN = 32;
 
 static int build_dir(Plan &P, int dir, DgTable &T) {
   const int N = P.N, Jh = P.Jh;
@@ -532,9 +541,12 @@ static int build_dir(Plan &P, int dir, DgTable &T) {
       ch += M.nq[p];
       nrmax = M.nr[p] > nrmax ? M.nr[p] : nrmax;
     }
-    for (int nt = 0; nt * DG_TN < nrmax; ++nt) items.push_back(make_int2(m, nt));
+    for (int nt = 0; nt * TN < nrmax; ++nt) items.push_back(make_int2(m, nt));
   }
   T.nchunk = ch;
+  // keep the 64-bit sums of (inverse: two parities of) K products in range (DgSum)
+  const int K = dir == 0 ? 2 * count_np(N, 0, 0) : Jh;
+  while (K >> T.guard > 1024) ++T.guard;
   T.nitems = (int)items.size();
   const long long nrows = dir == 0 ? (long long)(N + 1) * Jh : P.ncoef;
   // one allocation a direction: metadata and items (one copy), row scales, tiles
@@ -552,7 +564,7 @@ static int build_dir(Plan &P, int dir, DgTable &T) {
   T.d_tab = base + head + eb_b;
   dg_row_scale<<<(unsigned)((nrows + 7) / 8), 256>>>(dir, N, Jh, P.d_pnm, P.d_w, nrows, T.d_eb);
   DCCM_LAUNCH_CHECK();
-  dg_build<<<dim3(16, N + 1, 2), 256>>>(dir, N, Jh, DG_TN, (const DgMInfo *)T.d_mi, P.d_pnm, P.d_w, T.d_eb,
+  dg_build<<<dim3(16, N + 1, 2), 256>>>(dir, N, Jh, (const DgMInfo *)T.d_mi, P.d_pnm, P.d_w, T.d_eb,
                                         (unsigned char *)T.d_tab);
   DCCM_LAUNCH_CHECK();
   return DCCM_OK;
@@ -576,15 +588,18 @@ int build_digits(Plan &P) {
   return DCCM_OK;
 }
 
-static int launch_dg(Plan &P, int dir, int batch, int c0, int nct, double *out, cudaStream_t s) {
+template <int DIR> static int launch_kernel(const DgArgs &a, int items, cudaStream_t s) {
   static bool attr_done = false;
   if (!attr_done) {
-    DCCM_CUDA(cudaFuncSetAttribute(legendre_dg_kernel<DG_TN, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   DgShape<DG_TN>::SMEM));
-    DCCM_CUDA(cudaFuncSetAttribute(legendre_dg_kernel<DG_TN, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   DgShape<DG_TN>::SMEM));
+    DCCM_CUDA(cudaFuncSetAttribute(legendre_dg_kernel<DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
     attr_done = true;
   }
+  const int ctas = sm_count();
+  DCCM_CUDA(launch_pdl(legendre_dg_kernel<DIR>, dim3(items < ctas ? items : ctas), dim3(DG_THREADS), (size_t)DG_SMEM, s, a));
+  return DCCM_OK;
+}
+
+static int launch_dg(Plan &P, int dir, int batch, int c0, int nct, double *out, cudaStream_t s) {
   const DgTable &T = dir == 0 ? P.dinv : P.dfwd;
   DgArgs a;
   a.N = P.N;
@@ -595,6 +610,7 @@ static int launch_dg(Plan &P, int dir, int batch, int c0, int nct, double *out, 
   a.nitems = T.nitems;
   a.nchunk = T.nchunk;
   a.ldea = P.dg_ldea;
+  a.enan = 2047 + T.guard;
   a.ncoef = P.ncoef;
   a.mi = (const DgMInfo *)T.d_mi;
   a.items = T.d_items;
@@ -606,10 +622,8 @@ static int launch_dg(Plan &P, int dir, int batch, int c0, int nct, double *out, 
   a.err = P.d_err;
   a.wait_ns = tunables().wait_limit_ms > 0 ? 1000000ull * (unsigned long long)tunables().wait_limit_ms : WAIT_LIMIT_NS;
   a.withhold = tunables().tc_withhold_loads;
-  const int items = nct * T.nitems, ctas = sm_count();
-  DCCM_CUDA(launch_pdl(dir == 0 ? legendre_dg_kernel<DG_TN, 0> : legendre_dg_kernel<DG_TN, 1>, dim3(items < ctas ? items : ctas), dim3(DG_THREADS),
-                       (size_t)DgShape<DG_TN>::SMEM, s, a));
-  return DCCM_OK;
+  const int items = nct * T.nitems;
+  return dir == 0 ? launch_kernel<0>(a, items, s) : launch_kernel<1>(a, items, s);
 }
 
 int legendre_inv_f64(Plan &P, int batch, const double *spec, double *F, cudaStream_t s) {
@@ -640,7 +654,7 @@ int legendre_fwd_f64(Plan &P, int batch, const double *G, double *spec, cudaStre
     auto pack = [&](auto kernel, int wq) {
       const int per = 8 * (8 / wq);
       return launch_pdl(kernel, dim3((nc + per - 1) / per, 2 * (P.N + 1)), dim3(256), 0, s, mi, P.Jh, 2 * batch, c0, nc, G,
-                        P.dfwd.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea);
+                        P.dfwd.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea, P.dfwd.guard);
     };
     DCCM_CUDA(nq <= 1 ? pack(dg_pack_four<1>, 1) : nq <= 2 ? pack(dg_pack_four<2>, 2)
               : nq <= 4 ? pack(dg_pack_four<4>, 4) : pack(dg_pack_four<8>, 8));

@@ -60,6 +60,7 @@ struct DgTable {
   void *d_tab = nullptr;      // shared-memory images of the table tiles
   int nchunk = 0;             // A chunks per 128-column tile
   int nitems = 0;
+  int guard = 0;              // bits the A operand is scaled down by (sums of very many products)
 };
 
 struct Plan {

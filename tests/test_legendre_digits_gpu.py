@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 # (N, I, J, batch)
 SIZES = [(1, 64, 2, 1), (2, 64, 4, 3), (15, 64, 16, 1), (30, 64, 32, 2), (31, 64, 34, 63), (32, 96, 34, 64),
          (33, 96, 62, 65), (62, 128, 66, 2), (65, 192, 128, 129), (127, 256, 130, 3), (128, 384, 256, 2),
-         (257, 768, 260, 2), (300, 768, 514, 1)]
+         (257, 768, 260, 2), (300, 768, 514, 1), (21, 64, 2200, 2)]
 
 
 @pytest.mark.parametrize("N,I,J,B", SIZES)

@@ -255,7 +255,6 @@ legendre_tc_kernel(const __grid_constant__ TcLaunch L) {
         const int nrow = min(a.brows, mi.nr - nt * a.brows);
         const int amn = a.dir;  // forward A is MN-major
         const uint32_t idesc = idesc_f16kind(nrow, amn, a.nsplit == 3);
-        const int ncross = a.nsplit == 3 ? 5 : 2;
         const int ab = a.nacc == 2 ? (li & 1) : 0;
         const int ar = a.nacc == 2 ? (li >> 1) : li;  // use count of this accumulator set
         if (!mbar_wait(&acce[ab], (ar & 1) ^ 1, a.err, abort_flag, 2, L.wait_ns)) { ok = false; break; }
@@ -271,27 +270,28 @@ legendre_tc_kernel(const __grid_constant__ TcLaunch L) {
             if (!mbar_wait(&full[s], (g / NSTAGE) & 1, a.err, abort_flag, 3, L.wait_ns)) { ok = false; break; }
             tc_fence_after();
             const uint32_t As = smem_u32(stage + s * STAGE_BYTES);
-            const uint32_t Bs = As + 3 * A_SPLIT_BYTES;
             const int ksteps = min(4, (kv - q * 64 + 15) / 16);
+            // Descriptors by constant offsets (16-byte units) from the
+            // stage's two: a K step of 16 is 32 bytes along a K-major row, 16
+            // rows of an MN-major tile.  (A split, B split) of the cross
+            // terms: BF16 x 3 hi*mid, mid*hi, hi*lo, lo*hi, mid*mid; FP16
+            // hi + lo: hi*lo, lo*hi.
+            uint64_t da = smem_desc(As, amn ? 8192 : 16), db = smem_desc(As + 3 * A_SPLIT_BYTES, 16);
+            const uint64_t ka = amn ? 2048 >> 4 : 32 >> 4;
+            constexpr uint64_t A1 = A_SPLIT_BYTES >> 4, B1 = B_SPLIT_BYTES >> 4;
             for (int ks = 0; ks < ksteps; ++ks) {
-              // K step of 16: 32 bytes along a K-major row, 16 rows of an MN-major tile
-              const uint32_t ka = amn ? ks * 2048 : ks * 32;
-              const uint32_t lbo = amn ? 8192 : 16;
-              const uint32_t kb = ks * 32;
-              mma_bf16(dmain, smem_desc(As + ka, lbo), smem_desc(Bs + kb, 16), idesc, accm);
+              mma_bf16(dmain, da, db, idesc, accm);
               accm = 1;
-              // (A split, B split): BF16 x 3 hi*mid, mid*hi, hi*lo, lo*hi,
-              // mid*mid; FP16 hi + lo: hi*lo, lo*hi
-              const int pa[5] = {0, 1, 0, 2, 1};
-              const int pb[5] = {1, 0, 2, 0, 1};
-#pragma unroll
-              for (int u = 0; u < 5; ++u) {
-                if (u < ncross) {
-                  mma_bf16(dcross, smem_desc(As + pa[u] * A_SPLIT_BYTES + ka, lbo),
-                           smem_desc(Bs + pb[u] * B_SPLIT_BYTES + kb, 16), idesc, accx);
-                  accx = 1;
-                }
+              mma_bf16(dcross, da, db + B1, idesc, accx);
+              accx = 1;
+              mma_bf16(dcross, da + A1, db, idesc, 1);
+              if (a.nsplit == 3) {
+                mma_bf16(dcross, da, db + 2 * B1, idesc, 1);
+                mma_bf16(dcross, da + 2 * A1, db, idesc, 1);
+                mma_bf16(dcross, da + A1, db + B1, idesc, 1);
               }
+              da += ka;
+              db += 32 >> 4;
             }
             mma_commit(&empty[s]);
           }

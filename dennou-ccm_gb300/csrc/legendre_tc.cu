@@ -45,7 +45,7 @@ namespace sht {
 // Threads of a CTA: warp 0 (TMA), warp 1 (TMEM, MMA) and the epilogue
 // warps, 4 (narrow shape) or 8 (wide shape: two warps per TMEM lane quarter
 // share each item's epilogue).
-template <bool NARROW> constexpr int tc_epi_warps() { return NARROW ? 4 : 8; }
+template <bool NARROW> constexpr int tc_epi_warps() { return NARROW ? 4 : 16; }
 template <bool NARROW> constexpr int tc_threads() { return 64 + 32 * tc_epi_warps<NARROW>(); }
 constexpr int A_SPLIT_BYTES = 128 * 128;     // 128 rows (c) x 64 bf16 (K)
 // Two shapes of the same kernel:
@@ -338,25 +338,26 @@ legendre_tc_kernel(const __grid_constant__ TcLaunch L) {
       if (a.dir == 0) {
         const int J = 2 * a.Jh;
         const bool odd = mi.kv1 > 0;
-        for (int j0 = 16 * half; j0 < nrow; j0 += 16 * EH) {
-          // the four accumulators' columns j0..j0+15, one wait for all
-          uint32_t re[16], rx[16], ro[16], ry[16];
-          tmem_ld16_nw(tbase + j0, re);
-          tmem_ld16_nw(tbase + NT + j0, rx);
+        constexpr int CI = EH == 4 ? 8 : 16;
+        for (int j0 = CI * half; j0 < nrow; j0 += CI * EH) {
+          // the four accumulators' columns j0..j0+CI-1, one wait for all
+          uint32_t re[CI], rx[CI], ro[CI], ry[CI];
+          tmem_ld_nw(tbase + j0, re);
+          tmem_ld_nw(tbase + NT + j0, rx);
           if (odd) {
-            tmem_ld16_nw(tbase + 2 * NT + j0, ro);
-            tmem_ld16_nw(tbase + 3 * NT + j0, ry);
+            tmem_ld_nw(tbase + 2 * NT + j0, ro);
+            tmem_ld_nw(tbase + 3 * NT + j0, ry);
           }
           tmem_wait_ld();
-          float e[16], o[16];
+          float e[CI], o[CI];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
+          for (int i = 0; i < CI; ++i) {
             e[i] = __uint_as_float(re[i]) + __uint_as_float(rx[i]);
             o[i] = odd ? __uint_as_float(ro[i]) + __uint_as_float(ry[i]) : 0.f;
           }
           if (c < C2B) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
+            for (int i = 0; i < CI; ++i) {
               const int jj = nt * a.brows + j0 + i;
               if (jj < a.Jh) {
                 a.F[((long long)m * J + (a.Jh + jj)) * C2B + c] = (e[i] + o[i]) * us;
@@ -387,18 +388,19 @@ legendre_tc_kernel(const __grid_constant__ TcLaunch L) {
                 erow[2 * i] = (__uint_as_float(r0[i]) + __uint_as_float(x0[i])) * us;
                 erow[2 * i + 1] = (__uint_as_float(r1[i]) + __uint_as_float(x1[i])) * us;
               }
-            } else {  // two warps a quarter: columns k0 + 8 half .. + 7 each
-              const int k8 = k0 + 8 * half;
-              uint32_t r0[8], x0[8], r1[8], x1[8];
-              tmem_ld8_nw(tbase + k8, r0);
-              tmem_ld8_nw(tbase + NT + k8, x0);
-              tmem_ld8_nw(tbase + 2 * NT + k8, r1);
-              tmem_ld8_nw(tbase + 3 * NT + k8, x1);
+            } else {  // EH warps a quarter: columns k0 + CW half .. + CW - 1 each
+              constexpr int CW = 16 / EH;
+              const int kw = k0 + CW * half;
+              uint32_t r0[CW], x0[CW], r1[CW], x1[CW];
+              tmem_ld_nw(tbase + kw, r0);
+              tmem_ld_nw(tbase + NT + kw, x0);
+              tmem_ld_nw(tbase + 2 * NT + kw, r1);
+              tmem_ld_nw(tbase + 3 * NT + kw, x1);
               tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                erow[2 * (8 * half + i)] = (__uint_as_float(r0[i]) + __uint_as_float(x0[i])) * us;
-                erow[2 * (8 * half + i) + 1] = (__uint_as_float(r1[i]) + __uint_as_float(x1[i])) * us;
+              for (int i = 0; i < CW; ++i) {
+                erow[2 * (CW * half + i)] = (__uint_as_float(r0[i]) + __uint_as_float(x0[i])) * us;
+                erow[2 * (CW * half + i) + 1] = (__uint_as_float(r1[i]) + __uint_as_float(x1[i])) * us;
               }
             }
           }

@@ -110,6 +110,9 @@ __device__ __forceinline__ void tmem_ld8_nw(uint32_t taddr, uint32_t (&r)[8]) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld_nw(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16_nw(taddr, r); }
+__device__ __forceinline__ void tmem_ld_nw(uint32_t taddr, uint32_t (&r)[8]) { tmem_ld8_nw(taddr, r); }
+__device__ __forceinline__ void tmem_ld_nw(uint32_t taddr, uint32_t (&r)[4]) { tmem_ld4_nw(taddr, r); }
 
 }  // namespace sht
 }  // namespace dccm

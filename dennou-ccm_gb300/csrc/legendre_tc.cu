@@ -21,9 +21,9 @@
 //   A forward  G3[s][(2m+p) Jh + jj][c], MN-major (c contiguous): written
 //              split by the forward FFT;
 //   B          the pre-split Pbar tiles built at plan creation.
-// Warp roles (192 threads): warp 0 lane 0 issues the TMA loads of a stage
-// (six boxes of A and B per 64-wide K chunk); warp 1 allocates TMEM and its
-// lane 0 issues the MMAs; warps 2-5 are the epilogue (tcgen05.ld of the
+// Warp roles: warp 0 lane 0 issues the TMA loads of a stage (six boxes of A
+// and B per 64-wide K chunk); warp 1 allocates TMEM and its lane 0 issues the
+// MMAs; warps 2-17 (narrow shape 2-5) are the epilogue (tcgen05.ld of the
 // accumulators, warp w reading TMEM lanes 32 (w % 4) ..; inverse: parity
 // fold, stores coalesced along c; forward: both parities through shared
 // memory, stores coalesced along n).  Two shared-memory stages and two TMEM
@@ -43,8 +43,9 @@ namespace dccm {
 namespace sht {
 
 // Threads of a CTA: warp 0 (TMA), warp 1 (TMEM, MMA) and the epilogue
-// warps, 4 (narrow shape) or 8 (wide shape: two warps per TMEM lane quarter
-// share each item's epilogue).
+// warps, 4 (narrow shape) or 16 (wide shape: four warps per TMEM lane quarter
+// share each item's epilogue; with two T341 x 192 synthesis took 186 us, now
+// 179, the mixed pairs 57.5 -> 56.8 us at T85, 1097 -> 1090 at T341).
 template <bool NARROW> constexpr int tc_epi_warps() { return NARROW ? 4 : 16; }
 template <bool NARROW> constexpr int tc_threads() { return 64 + 32 * tc_epi_warps<NARROW>(); }
 constexpr int A_SPLIT_BYTES = 128 * 128;     // 128 rows (c) x 64 bf16 (K)

@@ -63,6 +63,10 @@ IMPLCPL_FWD_ARGS = ["xyr_MomFluxX", "xyr_MomFluxY", "xyr_HeatFlux", "xyrf_QMixFl
                     "xyz_Exner", "xyr_Exner", "xyr_VirTemp", "xyz_Height", "xyr_VelDiffCoef",
                     "xyr_TempDiffCoef", "xyr_QMixDiffCoef", "xyz_DUDt", "xyz_DVDt", "xyz_DTempDt",
                     "xyzf_DQMixDt", "xya_ImplCplCoef1", "xya_ImplCplCoef2"]
+# the profiles' and outputs' dict keys, in that order
+IMPLCPL_FWD_NAMES = ["MomFluxX", "MomFluxY", "HeatFlux", "QMixFlux", "Press", "ExnerFull", "ExnerHalf",
+                     "VirTemp", "Height", "VelDiffCoef", "TempDiffCoef", "QMixDiffCoef", "DUDt", "DVDt",
+                     "DTempDt", "DQMixDt", "ImplCplCoef1", "ImplCplCoef2"]
 
 
 class ImplCplConsts(ctypes.Structure):
@@ -221,21 +225,24 @@ def _check(st, what):
         raise DccmError(st, what)
 
 
+def _addr(a):
+    """Address of a numpy array or a torch tensor (device or host): a plain
+    int, as building a ctypes pointer object takes longer; the caller keeps
+    the array referenced."""
+    return a.data_ptr() if hasattr(a, "data_ptr") else a.ctypes.data
+
+
 def _p(a):
-    """Pointer of a numpy array or a torch tensor (device or host)."""
-    if a is None:
-        return None
-    if hasattr(a, "data_ptr"):
-        return ctypes.c_void_p(a.data_ptr())
-    return a.ctypes.data_as(ctypes.c_void_p)
+    """_addr, with None for a null pointer."""
+    return None if a is None else _addr(a)
 
 
 def _stream(s):
     if s is None:
         return None
     if hasattr(s, "cuda_stream"):
-        return ctypes.c_void_p(s.cuda_stream)
-    return ctypes.c_void_p(int(s))
+        return s.cuda_stream
+    return int(s)
 
 
 def fp64_peak(stream=None):
@@ -280,14 +287,11 @@ def DSFCM_Util_SfcBulkFlux_Get(arrays, IA, JA, IS, IE, JS, JE, device=False, str
     a_Sig1Info).  Host numpy arrays use the host entry point; torch CUDA
     tensors with device=True use the device entry point."""
     L = load()
-    a = FluxArgs()
-    keep = []
-    for n in FLUX_ARGS:
-        arr = arrays[n]
-        if n == "a_Sig1Info" and device:
-            arr = np.ascontiguousarray(np.asarray(arr.cpu() if hasattr(arr, "cpu") else arr, np.float64))
-            keep.append(arr)
-        setattr(a, n, _p(arr).value)
+    if device:
+        sig = arrays["a_Sig1Info"]
+        sig = np.ascontiguousarray(np.asarray(sig.cpu() if hasattr(sig, "cpu") else sig, np.float64))
+        arrays = {**arrays, "a_Sig1Info": sig}
+    a = FluxArgs(*[_addr(arrays[n]) for n in FLUX_ARGS])
     g = SfcGrid(IA, JA, IS, IE, JS, JE)
     if device:
         _check(L.dccm_sfc_bulk_flux_get_dev(ctypes.byref(a), ctypes.byref(g), _stream(stream)),
@@ -500,7 +504,7 @@ class ShtPlan:
     def axes(self):
         """(x_Lon, y_Lat, x_Lon_Weight, y_Lat_Weight) as SPML returns them."""
         a = [np.zeros(self.I), np.zeros(self.J), np.zeros(self.I), np.zeros(self.J)]
-        _check(load().dccm_sht_axes(self.h, *[_p(x) for x in a]), "dccm_sht_axes")
+        _check(load().dccm_sht_axes(self.h, *[_addr(x) for x in a]), "dccm_sht_axes")
         return tuple(a)
 
     def gauss(self):
@@ -614,8 +618,8 @@ class Ensemble:
 
     def _call(self, fn, a, b, batch, stream):
         ng = len(self.groups)
-        pa = (ctypes.c_void_p * ng)(*[_p(x).value for x in a])
-        pb = (ctypes.c_void_p * ng)(*[_p(x).value for x in b])
+        pa = (ctypes.c_void_p * ng)(*[_addr(x) for x in a])
+        pb = (ctypes.c_void_p * ng)(*[_addr(x) for x in b])
         nb = (ctypes.c_int * ng)(*[int(x) for x in batch])
         _check(fn(self.h, pa, pb, nb, _stream(stream)), fn.__name__)
 
@@ -653,7 +657,7 @@ class HostCopies:
         arr = (HostCopy * max(1, len(pairs)))()
         for k, (h, dv) in enumerate(pairs):
             nb = h.numel() * h.element_size() if hasattr(h, "numel") else h.nbytes
-            arr[k] = HostCopy(_p(h).value, _p(dv).value, nb)
+            arr[k] = HostCopy(_addr(h), _addr(dv), nb)
         return arr, len(pairs)
 
     def nbytes(self):
@@ -678,11 +682,11 @@ class Step:
         d = StepDesc()
         d.sht = sht.h.value if sht is not None else None
         d.nfl = int(nfl)
-        d.spec_in, d.grid, d.spec_out = (_p(x).value if x is not None else None for x in (spec_in, grid, spec_out))
+        d.spec_in, d.grid, d.spec_out = (_p(x) for x in (spec_in, grid, spec_out))
         self._keep = [sht, spec_in, grid, spec_out, flux, remaps, ensemble, ens_spec_in, ens_grid, ens_spec_out]
         if ensemble is not None:
             ng = len(ens_nfl)
-            self._ens = [(ctypes.c_void_p * ng)(*[_p(x).value for x in arrs])
+            self._ens = [(ctypes.c_void_p * ng)(*[_addr(x) for x in arrs])
                          for arrs in (ens_spec_in, ens_grid, ens_spec_out)]
             self._ens_nfl = (ctypes.c_int * ng)(*[int(x) for x in ens_nfl])
             d.ens = ensemble.h.value
@@ -693,7 +697,7 @@ class Step:
             for k, rm in enumerate(lst):
                 plan, nf, src, lds, dst, ldd = rm[:6]
                 nsub, ld2 = (rm[6], rm[7]) if len(rm) > 6 else (0, 0)
-                arr[k] = StepRemap(plan.h.value, int(nf), _p(src).value, int(lds), _p(dst).value, int(ldd),
+                arr[k] = StepRemap(plan.h.value, int(nf), _addr(src), int(lds), _addr(dst), int(ldd),
                                    int(nsub), int(ld2))
             return arr
         self._remaps = remap_array(remaps)
@@ -711,7 +715,7 @@ class Step:
             fa = FluxArgs()
             self._sig = np.ascontiguousarray(np.asarray(flux["a_Sig1Info"], np.float64))
             for n in FLUX_ARGS:
-                setattr(fa, n, self._sig.ctypes.data if n == "a_Sig1Info" else _p(flux[n]).value)
+                setattr(fa, n, self._sig.ctypes.data if n == "a_Sig1Info" else _addr(flux[n]))
             self._fa = fa
             self._fg = SfcGrid(*flux_grid)
             d.flux = ctypes.addressof(fa)
@@ -810,18 +814,7 @@ class ImplCplPlan:
         self.h = h
 
     def _args(self, prof, out):
-        a = ImplCplForwardArgs()
-        names = {"xyr_MomFluxX": "MomFluxX", "xyr_MomFluxY": "MomFluxY", "xyr_HeatFlux": "HeatFlux",
-                 "xyrf_QMixFlux": "QMixFlux", "xyr_Press": "Press", "xyz_Exner": "ExnerFull",
-                 "xyr_Exner": "ExnerHalf", "xyr_VirTemp": "VirTemp", "xyz_Height": "Height",
-                 "xyr_VelDiffCoef": "VelDiffCoef", "xyr_TempDiffCoef": "TempDiffCoef",
-                 "xyr_QMixDiffCoef": "QMixDiffCoef", "xyz_DUDt": "DUDt", "xyz_DVDt": "DVDt",
-                 "xyz_DTempDt": "DTempDt", "xyzf_DQMixDt": "DQMixDt", "xya_ImplCplCoef1": "ImplCplCoef1",
-                 "xya_ImplCplCoef2": "ImplCplCoef2"}
-        for f, n in names.items():
-            x = prof.get(n) if n in prof else out[n]
-            setattr(a, f, _p(x).value)
-        return a
+        return ImplCplForwardArgs(*[_addr(prof[n] if n in prof else out[n]) for n in IMPLCPL_FWD_NAMES])
 
     def forward(self, prof):
         """Host arrays in (synth.column_profiles layout); returns the

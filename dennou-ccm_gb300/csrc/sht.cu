@@ -102,6 +102,7 @@ static void destroy(Plan &P) {
   P.stage.release();
   P.wa_spec.release();
   if (P.stream) cudaStreamDestroy(P.stream);
+  if (P.h_err) cudaFreeHost(P.h_err);
 }
 
 static int create(Plan &P, int N, int I, int J, int precision, int max_batch) {
@@ -289,25 +290,43 @@ extern "C" int dccm_sht_status(dccm_sht_plan *p, int *device_error) {
   return DCCM_OK;
 }
 
+namespace dccm {
+namespace sht {
+// Stream and error word of the host entry points, made by the first such call.
+int host_setup(Plan &P) {
+  if (!P.h_err) DCCM_CUDA(cudaHostAlloc((void **)&P.h_err, sizeof(int), cudaHostAllocDefault));
+  if (!P.stream) DCCM_CUDA(cudaStreamCreateWithFlags(&P.stream, cudaStreamNonBlocking));
+  return DCCM_OK;
+}
+
+// End of a host entry point: the device error flag of the bounded waits and
+// the n results come back in stream order with one synchronisation (a copy of
+// the flag by itself after it took 8 us of a call: 4 bytes, a second round
+// trip).
+int host_finish(Plan &P, const double *dout, double *out, size_t n) {
+  DCCM_CUDA(cudaMemcpyAsync(P.h_err, P.d_err, sizeof(int), cudaMemcpyDeviceToHost, P.stream));
+  DCCM_CUDA(cudaMemcpyAsync(out, dout, n * sizeof(double), cudaMemcpyDeviceToHost, P.stream));
+  DCCM_CUDA(cudaStreamSynchronize(P.stream));
+  if (*P.h_err) {
+    cudaMemset(P.d_err, 0, sizeof(int));
+    return DCCM_ERR_TIMEOUT;
+  }
+  return DCCM_OK;
+}
+}  // namespace sht
+}  // namespace dccm
+
 // Host arrays: copies in, transform, copies out, checks the device error flag.
 static int host_call(dccm_sht_plan *p, const double *in, size_t in_n, double *out, size_t out_n, int batch,
                      bool inv) {
   sht::Plan &P = p->P;
-  if (!P.stream) DCCM_CUDA(cudaStreamCreateWithFlags(&P.stream, cudaStreamNonBlocking));
+  DCCM_TRY(sht::host_setup(P));
   DCCM_TRY(P.stage.ensure((in_n + out_n) * sizeof(double)));
   double *din = (double *)P.stage.ptr, *dout = din + in_n;
   DCCM_CUDA(cudaMemcpyAsync(din, in, in_n * sizeof(double), cudaMemcpyHostToDevice, P.stream));
   if (inv) DCCM_TRY(sht::inverse(P, din, dout, batch, P.stream));
   else DCCM_TRY(sht::forward(P, din, dout, batch, P.stream));
-  DCCM_CUDA(cudaMemcpyAsync(out, dout, out_n * sizeof(double), cudaMemcpyDeviceToHost, P.stream));
-  DCCM_CUDA(cudaStreamSynchronize(P.stream));
-  int e = 0;
-  DCCM_CUDA(cudaMemcpy(&e, P.d_err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (e) {
-    cudaMemset(P.d_err, 0, sizeof(int));
-    return DCCM_ERR_TIMEOUT;
-  }
-  return DCCM_OK;
+  return sht::host_finish(P, dout, out, out_n);
 }
 
 extern "C" int dccm_sht_inverse(dccm_sht_plan *p, const double *spec, double *grid, int batch) {

@@ -94,7 +94,8 @@ struct Plan {
   int *d_ea = nullptr;         // FP64 path: scale exponents of the A operand, rows of dg_ldea (in d_dig)
   int dg_ct = 0, dg_ldea = 0;
   DevBuf stage;                // host entry point staging
-  cudaStream_t stream = nullptr;
+  cudaStream_t stream = nullptr;  // of the host entry points, with h_err (host_setup)
+  int *h_err = nullptr;        // page-locked copy of d_err
   // SPML real layout (spml.cu), set up by the first call that uses it:
   int2 *d_wa_pos = nullptr;    // per spectral index k: wa positions of Re and Im (-1: none)
   int *d_wa_src = nullptr;     // per wa position l: 2 k + (0: Re, 1: Im)
@@ -129,6 +130,8 @@ int fft_multi(Plan *const *plans, const int *batch, const void *const *in, void 
               cudaStream_t s);
 int inverse(Plan &P, const double *spec, double *grid, int batch, cudaStream_t s);
 int forward(Plan &P, const double *grid, double *spec, int batch, cudaStream_t s);
+int host_setup(Plan &P);
+int host_finish(Plan &P, const double *dout, double *out, size_t n);
 int build_tiles(Plan &P);
 int build_digits(Plan &P);
 int build_fft_f64(Plan &P, std::vector<int4> &h);

@@ -172,21 +172,13 @@ extern "C" int dccm_sht_wa_xya_dev(dccm_sht_plan *p, const double *xya, double *
 static int wa_host(dccm_sht_plan *p, const double *in, size_t in_n, double *out, size_t out_n, int batch,
                    bool inv) {
   sht::Plan &P = p->P;
-  if (!P.stream) DCCM_CUDA(cudaStreamCreateWithFlags(&P.stream, cudaStreamNonBlocking));
+  DCCM_TRY(sht::host_setup(P));
   DCCM_TRY(P.stage.ensure((in_n + out_n) * sizeof(double)));
   double *din = (double *)P.stage.ptr, *dout = din + in_n;
   DCCM_CUDA(cudaMemcpyAsync(din, in, in_n * sizeof(double), cudaMemcpyHostToDevice, P.stream));
   if (inv) DCCM_TRY(sht::xya_wa(P, din, dout, batch, P.stream));
   else DCCM_TRY(sht::wa_xya(P, din, dout, batch, P.stream));
-  DCCM_CUDA(cudaMemcpyAsync(out, dout, out_n * sizeof(double), cudaMemcpyDeviceToHost, P.stream));
-  DCCM_CUDA(cudaStreamSynchronize(P.stream));
-  int e = 0;
-  DCCM_CUDA(cudaMemcpy(&e, P.d_err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (e) {
-    cudaMemset(P.d_err, 0, sizeof(int));
-    return DCCM_ERR_TIMEOUT;
-  }
-  return DCCM_OK;
+  return sht::host_finish(P, dout, out, out_n);
 }
 
 extern "C" int dccm_sht_xya_wa(dccm_sht_plan *p, const double *wa, double *xya, int batch) {

@@ -119,6 +119,19 @@ __device__ __forceinline__ double fixed_to_double(long long q, int ex) {
                                           ((unsigned long long)s << 63)));
 }
 
+// The same where every result is normal or zero: FIXED_EX_MIN <= ex <=
+// FIXED_EX_MAX (no branch).
+constexpr int FIXED_EX_MIN = -1022, FIXED_EX_MAX = 959;
+__device__ __forceinline__ double fixed_to_double_normal(long long q, int ex) {
+  const long long s = q >> 63;
+  unsigned long long m = (unsigned long long)((q ^ s) - s);
+  const int z = __clzll((long long)(m | 1));
+  m <<= z;
+  const unsigned long long mant = (m >> 11) + ((unsigned)m >> 10 & 1u);
+  const unsigned hi = (unsigned)(mant >> 32) + ((unsigned)(ex + 1085 - z) << 20) + (unsigned)(s << 31);
+  return __hiloint2double(q ? (int)hi : 0, (int)(unsigned)mant);
+}
+
 // x in units of 2^ex level-6 units, as the nearest double.
 __device__ __forceinline__ double dg_to_double(const DgSum &x, int ex) {
   const int hi = (int)(x.t >> 32);

@@ -322,14 +322,21 @@ fft_forward_kernel(int N, int J, int batch, const double *__restrict__ grid, dou
   double2 *out = reinterpret_cast<double2 *>(G + (int64_t)jj * C2B + 2 * (b0 + bl));
   const int64_t pst = (int64_t)Jh * batch;  // one parity of one m, in double2
   const double nan = __longlong_as_double(0x7FF8000000000000ll);
+  const bool normal = E < 2047 && ex >= FIXED_EX_MIN && ex <= FIXED_EX_MAX;
   for (int m = threadIdx.x / Sh::BB; m <= N; m += Sh::T) {
     const C64 a = zb[Sh::pos(m)], c = zb[Sh::pos(m ? Sh::I - m : 0)];
     // 2A = (a.x + c.x, a.y - c.y), 2B = (a.y + c.y, c.x - a.x)
     const long long ar = a.x + c.x, ai = a.y - c.y, br = a.y + c.y, bi = c.x - a.x;
-    double2 e = make_double2(fixed_to_double(ar + br, ex), fixed_to_double(ai + bi, ex));
-    double2 o = make_double2(fixed_to_double(ar - br, ex), fixed_to_double(ai - bi, ex));
+    double2 e, o;
+    if (normal) {
+      e = make_double2(fixed_to_double_normal(ar + br, ex), fixed_to_double_normal(ai + bi, ex));
+      o = make_double2(fixed_to_double_normal(ar - br, ex), fixed_to_double_normal(ai - bi, ex));
+    } else {  // results that may be subnormal or infinite, or NaN
+      e = make_double2(fixed_to_double(ar + br, ex), fixed_to_double(ai + bi, ex));
+      o = make_double2(fixed_to_double(ar - br, ex), fixed_to_double(ai - bi, ex));
+      if (E >= 2047) e = o = make_double2(nan, nan);
+    }
     if (m == 0) e.y = o.y = 0.0;
-    if (E >= 2047) e = o = make_double2(nan, m ? nan : 0.0);
     out[(int64_t)(2 * m) * pst] = e;
     out[(int64_t)(2 * m + 1) * pst] = o;
   }
@@ -352,8 +359,8 @@ fft_inverse_kernel(int N, int J, int batch, const double *__restrict__ F, double
   constexpr int KI = Sh::R1 / 2;  // N + 1 <= I / 2
   const int bl = threadIdx.x % Sh::BB, m0 = threadIdx.x / Sh::BB;
   const int64_t C2B = 2LL * batch;
+  C64 *zb = buf + (size_t)bl * Sh::LD;
   double2 a[KI], b[KI];
-  unsigned mx = 0;
 #pragma unroll
   for (int i = 0; i < KI; ++i) {
     const int m = m0 + i * Sh::T;
@@ -365,36 +372,53 @@ fft_inverse_kernel(int N, int J, int batch, const double *__restrict__ F, double
       if (m == 0) a[i].y = b[i].y = 0.0;
     }
   }
+  // their bits wait in the positions of m and I - m (frequencies above N hold
+  // zeros, the same in either form; I / 2, never used as N < I / 2, stands in
+  // for m = 0's).  The two passes over them are loops: with the values in
+  // registers and both unrolled the kernel outgrew the instruction cache (3.5
+  // of 8 cycles an instruction waited for code; T85 x 128 took 48 us, now 34,
+  // T42 x 104 15, now 12)
+  unsigned mx = 0;
 #pragma unroll
-  for (int i = 0; i < KI; ++i) mx = max(max(mx, max(mag(a[i].x), mag(a[i].y))), max(mag(b[i].x), mag(b[i].y)));
+  for (int i = 0; i < KI; ++i) {
+    const int m = m0 + i * Sh::T;
+    mx = max(max(mx, max(mag(a[i].x), mag(a[i].y))), max(mag(b[i].x), mag(b[i].y)));
+    zb[Sh::pos(m)] = {__double_as_longlong(a[i].x), __double_as_longlong(a[i].y)};
+    zb[Sh::pos(m ? Sh::I - m : Sh::I / 2)] = {__double_as_longlong(b[i].x), __double_as_longlong(b[i].y)};
+  }
   atomicMax(&smx[bl], mx);
   __syncthreads();
   const int E = max((int)(smx[bl] >> 20), 1);
-  // sum of the magnitudes in units of 2^(E - 1022 - 20), each rounded up
-  unsigned sum = 0;
-  auto units = [&](double x) {
-    const unsigned h = mag(x);
-    const int ef = (int)(h >> 20);
-    const unsigned m20 = ((h & 0xFFFFFu) | (ef ? 0x100000u : 0u)) >> 1;
-    return (m20 >> min(E - max(ef, 1), 31)) + 1u;
+  // sum of the magnitudes in units of 2^(E - 1022 - 20), rounded up: each as
+  // FP32 relative to 2^(E - 1023) (20 bits of its mantissa), a thread's sum
+  // with a margin above those and the sums' rounding errors
+  const int nm = (N + Sh::T) / Sh::T;  // m0 + i T <= N needs i < nm
+  const int hb = (E - 127) * (1 << 20);
+  auto rel = [&](long long x) {
+    return __int_as_float(max(((int)(x >> 32) & 0x7FFFFFFF) - hb, 0) << 3);
   };
-#pragma unroll
-  for (int i = 0; i < KI; ++i) sum += units(a[i].x) + units(a[i].y) + units(b[i].x) + units(b[i].y);
-  atomicAdd(&ssum[bl], sum);
+  float sum = 0.f;
+#pragma unroll 2
+  for (int i = 0; i < nm; ++i) {
+    const int m = m0 + i * Sh::T;
+    const C64 u = zb[Sh::pos(m)], w = zb[Sh::pos(m ? Sh::I - m : Sh::I / 2)];
+    sum += (rel(u.x) + rel(u.y)) + (rel(w.x) + rel(w.y));
+  }
+  atomicAdd(&ssum[bl], __float2uint_ru(sum * (524288.f + 8.f)) + 1u);
   __syncthreads();
   // sum of |Re Z| + |Im Z| over all frequencies < 2^(nbit + 1) units -> 2^62:
   // the mantissa moves by ef - E + 28 - nbit
   const int nbit = 32 - __clz((int)ssum[bl]);
   const int rb = 10 - (28 - nbit) + E;
-  C64 *zb = buf + (size_t)bl * Sh::LD;
-#pragma unroll
-  for (int i = 0; i < KI; ++i) {
+#pragma unroll 2
+  for (int i = 0; i < nm; ++i) {
     const int m = m0 + i * Sh::T;
-    const long long ar = to_fixed(a[i].x, rb), ai = to_fixed(a[i].y, rb);
-    const long long br = to_fixed(b[i].x, rb), bi = to_fixed(b[i].y, rb);
-    // frequencies above N hold zeros; I / 2 is never used (N < I / 2)
-    zb[Sh::pos(m)] = {ar - bi, ai + br};
-    zb[Sh::pos(m ? Sh::I - m : Sh::I / 2)] = m ? C64{ar + bi, br - ai} : C64{0, 0};
+    C64 &zm = zb[Sh::pos(m)], &zi = zb[Sh::pos(m ? Sh::I - m : Sh::I / 2)];
+    const C64 u = zm, w = zi;
+    const long long ar = to_fixed(__longlong_as_double(u.x), rb), ai = to_fixed(__longlong_as_double(u.y), rb);
+    const long long br = to_fixed(__longlong_as_double(w.x), rb), bi = to_fixed(__longlong_as_double(w.y), rb);
+    zm = {ar - bi, ai + br};
+    zi = m ? C64{ar + bi, br - ai} : C64{0, 0};
   }
   __syncthreads();
   const int g = threadIdx.x / Sh::T, t = threadIdx.x % Sh::T;
@@ -414,13 +438,24 @@ fft_inverse_kernel(int N, int J, int batch, const double *__restrict__ F, double
   dft<1, Sh::R1>(v);
   const int Eg = max((int)(smx[g] >> 20), 1);
   const int ex = Eg - 1075 - (28 - (32 - __clz((int)ssum[g])));
-  const double nan = __longlong_as_double(0x7FF8000000000000ll);
   double *gn = grid + ((int64_t)(b0 + g) * J + jn) * Sh::I + t;
   double *gs = grid + ((int64_t)(b0 + g) * J + js) * Sh::I + t;
+  if (Eg < 2047 && ex >= FIXED_EX_MIN && ex <= FIXED_EX_MAX) {
 #pragma unroll
-  for (int p = 0; p < Sh::R1; ++p) {
-    gn[p * Sh::N1] = Eg >= 2047 ? nan : fixed_to_double(v[p].x, ex);
-    gs[p * Sh::N1] = Eg >= 2047 ? nan : fixed_to_double(v[p].y, ex);
+    for (int p = 0; p < Sh::R1; ++p) {
+      gn[p * Sh::N1] = fixed_to_double_normal(v[p].x, ex);
+      gs[p * Sh::N1] = fixed_to_double_normal(v[p].y, ex);
+    }
+  } else {  // results that may be subnormal or infinite, or NaN
+    const double nan = __longlong_as_double(0x7FF8000000000000ll);
+#pragma unroll
+    for (int p = 0; p < Sh::R1; ++p) z[Sh::at(p * Sh::N1 + t)] = v[p];
+#pragma unroll 1
+    for (int p = 0; p < Sh::R1; ++p) {
+      const C64 u = z[Sh::at(p * Sh::N1 + t)];
+      gn[p * Sh::N1] = Eg >= 2047 ? nan : fixed_to_double(u.x, ex);
+      gs[p * Sh::N1] = Eg >= 2047 ? nan : fixed_to_double(u.y, ex);
+    }
   }
 }
 

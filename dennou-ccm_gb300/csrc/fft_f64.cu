@@ -190,6 +190,8 @@ template <int I_, int R1_, int R2_, int R3_> struct Shape {
   static constexpr int CB = 60 - clog2(RL) < 58 ? 60 - clog2(RL) : 58;
   static constexpr int THREADS = T >= 64 ? 256 : 128;
   static constexpr int BB = THREADS / T;
+  // CTAs of an SM: eight points a thread fit 80 registers, 12 or 16 take 128
+  static constexpr int MINB = (R1 == 8 && R3 > 1 ? 768 : 512) / THREADS;
   static __host__ __device__ constexpr int at(int a) { return a + a / RL + (R3 > 1 ? a / N1 : 0); }
   // stride of the row pairs' buffers, 2 (mod 8) 16-byte units
   static constexpr int LD = (at(I - 1) + 1 + 7) / 8 * 8 + 2;
@@ -255,7 +257,7 @@ __device__ __forceinline__ void pass(C64 *z, const int4 *__restrict__ tw, int t)
 }
 
 template <class Sh>
-__global__ void __launch_bounds__(Sh::THREADS, 512 / Sh::THREADS)
+__global__ void __launch_bounds__(Sh::THREADS, Sh::MINB)
 fft_forward_kernel(int N, int J, int batch, const double *__restrict__ grid, double *__restrict__ G,
                    const int4 *__restrict__ tw, int4 w0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -343,7 +345,7 @@ fft_forward_kernel(int N, int J, int batch, const double *__restrict__ grid, dou
 }
 
 template <class Sh>
-__global__ void __launch_bounds__(Sh::THREADS, 512 / Sh::THREADS)
+__global__ void __launch_bounds__(Sh::THREADS, Sh::MINB)
 fft_inverse_kernel(int N, int J, int batch, const double *__restrict__ F, double *__restrict__ grid,
                    const int4 *__restrict__ tw) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -511,15 +513,19 @@ static long long scaled(long long v, int k, bool three) {
   return (long long)(x >= 0 ? (x + d / 2) / d : -((-x + d / 2) / d));
 }
 
+// Three passes of eight points a thread where they can be had (us inverse /
+// forward, against two of 16 or 16 first): T42 x 8 8.9 / 8.2 (9.9 / 10.2), T85 x
+// 8 9.8 / 8.2 (11.9 / 10.2), T170 x 64 59 / 53 (67 / 55).  1024 points keep 16
+// first, as four passes would be needed; 192 = 12 x 4 x 4 was no faster.
 template <class F> static int with_shape(int I, F &&f) {
   switch (I) {
     case 64: return f(Shape<64, 8, 8, 1>());
     case 96: return f(Shape<96, 12, 8, 1>());
-    case 128: return f(Shape<128, 16, 8, 1>());
+    case 128: return f(Shape<128, 8, 4, 4>());
     case 192: return f(Shape<192, 12, 16, 1>());
-    case 256: return f(Shape<256, 16, 16, 1>());
+    case 256: return f(Shape<256, 8, 8, 4>());
     case 384: return f(Shape<384, 12, 8, 4>());
-    case 512: return f(Shape<512, 16, 8, 4>());
+    case 512: return f(Shape<512, 8, 8, 8>());
     case 768: return f(Shape<768, 12, 8, 8>());
     case 1024: return f(Shape<1024, 16, 8, 8>());
     default: return DCCM_ERR_UNSUPPORTED;
@@ -528,9 +534,10 @@ template <class F> static int with_shape(int I, F &&f) {
 
 }  // namespace f64
 
-// Twiddles of both directions: forward entries e^{-i theta} 2^(64 - s), such that twmul<32> scales by 2^-s, s = ceil(log2 R) (and by 2/3 in the
-// first pass of lengths with a factor 3, the odd part of 1/I); inverse
-// entries e^{+i theta} 2^62 for twmul<30>.
+// Twiddles of both directions: forward entries e^{-i theta} 2^(64 - s), such
+// that twmul<32> scales by 2^-s, s = ceil(log2 R) (and by 2/3 in the first
+// pass of lengths with a factor 3, the odd part of 1/I); inverse entries e^{+i
+// theta} 2^62 for twmul<30>.
 int build_fft_f64(Plan &P, std::vector<int4> &h) {
   using namespace f64;
   return with_shape(P.I, [&](auto sh) {

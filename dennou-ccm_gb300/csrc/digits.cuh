@@ -83,23 +83,35 @@ __device__ __forceinline__ void dg_store8(unsigned char *dst, size_t stride, con
 }
 
 // Sum of drained accumulators (levels s = 2 .. 8 of digit products, integers
-// below 2^24): t in units of level 6 (2^18 level-8 units), the two lowest
-// levels beside it in FP32 (its 24 bits reach 2^-61 of the largest product).
+// below 2^24): t in units of level 6 (2^18 level-8 units), the rest below in
+// FP32 (its 24 bits reach 2^-61 of the largest product).
 // 1.01 K 2^52 < 2^63 for K products: K < 2,000.
 struct DgSum {
   long long t;
   float l;
 };
+// Conversions to integers are the limit here (one warp instruction in eight
+// cycles), so levels 4 and 6 hand their multiples of 512 to the level above
+// in FP32, exactly, and only what is left, |.| <= 256, goes to the level
+// below: three conversions in place of five.
 __device__ __forceinline__ void dg_accumulate(DgSum &x, const unsigned (&r)[DG_SLICES]) {
-  int v[5];
+  constexpr float M = 1.5f * 4294967296.f;  // 2^32: rounds to multiples of 512
+  float v[DG_SLICES];
 #pragma unroll
-  for (int s = 0; s < 5; ++s) v[s] = __float2int_rn(__uint_as_float(r[s]));
-  x.t += v[4];
-  x.t += (long long)v[3] * (1 << 9);
-  x.t += (long long)v[2] * (1 << 18);
-  x.t += (long long)v[1] * (1 << 27);
-  x.t += (long long)v[0] << 36;
-  x.l = fmaf(__uint_as_float(r[5]), 512.f, x.l) + __uint_as_float(r[6]);
+  for (int s = 0; s < DG_SLICES; ++s) v[s] = __uint_as_float(r[s]);
+  const float h2 = __fadd_rn(__fadd_rn(v[2], M), -M), h4 = __fadd_rn(__fadd_rn(v[4], M), -M);
+  const float l2 = __fadd_rn(v[2], -h2), l4 = __fadd_rn(v[4], -h4);
+  const int i0 = __float2int_rn(v[0]);
+  const int i1 = __float2int_rn(fmaf(h2, 1.f / 512.f, v[1]));
+  const int i3 = __float2int_rn(fmaf(l2, 512.f, fmaf(h4, 1.f / 512.f, v[3])));
+  x.t += (long long)i3 * (1 << 9);
+  x.t += (long long)i1 * (1 << 27);
+  x.t += (long long)i0 << 36;
+  x.l = fmaf(l4, 262144.f, fmaf(v[5], 512.f, x.l)) + v[6];
+}
+// x 2^k in whole level-6 units, 0 <= k <= 10 and x 2^k within range
+__device__ __forceinline__ long long dg_sum_fixed(const DgSum &x, int k) {
+  return (x.t << k) + __float2int_rn(x.l * __int_as_float((k + 109) << 23));  // l 2^(k - 18)
 }
 
 // q 2^ex as the nearest double (ties away from zero).
@@ -112,6 +124,7 @@ __device__ __forceinline__ double fixed_to_double(long long q, int ex) {
   const unsigned long long mant = (m >> 11) + ((unsigned)m >> 10 & 1u);  // 53 bits, or 2^53
   const int be = ex + 63 - z + 1023;
   if ((unsigned)(be - 1) >= 2045u) {  // subnormal result or overflow
+    if (be < -60) return __longlong_as_double((long long)((unsigned long long)s << 63));
     const double r = ldexp((double)mant, be - 1075);
     return s ? -r : r;
   }
@@ -130,14 +143,6 @@ __device__ __forceinline__ double fixed_to_double_normal(long long q, int ex) {
   const unsigned long long mant = (m >> 11) + ((unsigned)m >> 10 & 1u);
   const unsigned hi = (unsigned)(mant >> 32) + ((unsigned)(ex + 1085 - z) << 20) + (unsigned)(s << 31);
   return __hiloint2double(q ? (int)hi : 0, (int)(unsigned)mant);
-}
-
-// x in units of 2^ex level-6 units, as the nearest double.
-__device__ __forceinline__ double dg_to_double(const DgSum &x, int ex) {
-  const int hi = (int)(x.t >> 32);
-  const int k = min(__clz(hi ^ (hi >> 31)) - 1, 10);  // room above t
-  const long long q = (x.t << k) + __float2int_rn(x.l * __int_as_float((k + 109) << 23));  // l 2^(k - 18)
-  return fixed_to_double(q, ex - k);
 }
 
 }  // namespace dccm

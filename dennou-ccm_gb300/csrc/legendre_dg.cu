@@ -143,6 +143,74 @@ __device__ __forceinline__ int dg_item(int k) {  // as cta_item: rounds in alter
   return (k & 1) ? (k + 1) * G - 1 - b : k * G + b;
 }
 
+__device__ __noinline__ double dg_double_any(long long q, int ex) { return fixed_to_double(q, ex); }
+
+// Bits, at most 10, that the sums S (and those in any) have room for.
+template <int EC> __device__ __forceinline__ int dg_room(const DgSum (&S)[EC], unsigned &any) {
+#pragma unroll
+  for (int x = 0; x < EC; ++x) {
+    const int hi = (int)(S[x].t >> 32);
+    any |= (unsigned)(hi ^ (hi >> 31));
+  }
+  return min(__clz((int)any) - 1, 10);
+}
+
+// The integer pipes limit this part (16 results a thread of the inverse took
+// 7,400 cycles with a range branch each and the scales loaded at the end: half
+// of an item's epilogue; T85 x 128 both ways 120 -> 111 us without them).
+// put(x, conv) for x < EC, where conv(q, x) is the double of q units of 2^-up
+// at level 6, given the scale exponents of the table's rows: without branches
+// where all results are normal.
+template <int EC, class Put>
+__device__ __forceinline__ void dg_results(const int (&eb)[EC], int E, int up, int enan, Put put) {
+  const int e0 = E - 1022 - 52 - up;
+  bool normal = E < enan;
+#pragma unroll
+  for (int x = 0; x < EC; ++x) normal = normal && e0 + eb[x] >= FIXED_EX_MIN && e0 + eb[x] <= FIXED_EX_MAX;
+  if (normal) {
+#pragma unroll
+    for (int x = 0; x < EC; ++x) put(x, [&](long long q, int k) { return fixed_to_double_normal(q, e0 + eb[k]); });
+  } else {  // rows of the table near the poles at large m, extreme or non-finite operands
+#pragma unroll
+    for (int x = 0; x < EC; ++x)
+      put(x, [&](long long q, int k) {
+        return E < enan ? dg_double_any(q, e0 + eb[k]) : __longlong_as_double(0x7FF8000000000000ll);
+      });
+  }
+}
+
+// A CTA's items in order, with the table entries of the current one in
+// registers: they are loaded an item ahead (the first before the wait for the
+// kernel before, a chain of loads of 1 us), their place in the list two ahead.
+// Read through the table at each use, that is anew after every wait and copy,
+// T341 x 192 took 538 / 638 us with its pack (inverse / forward), now 520 / 616.
+struct DgWalk {
+  int k, it, ct, m, nt;
+  DgMInfo mi;
+  int2 next, after;
+  DgMInfo minext;
+
+  __device__ __forceinline__ static int2 entry(const DgArgs &a, int it) {
+    return it < a.nct * a.nitems ? __ldg(a.items + it / a.nct) : make_int2(0, 0);
+  }
+  __device__ __forceinline__ explicit DgWalk(const DgArgs &a) : k(-1), next(entry(a, dg_item(0))), after(entry(a, dg_item(1))) {
+    minext = a.mi[next.x];
+  }
+  // the next item, if there is one
+  __device__ __forceinline__ bool step(const DgArgs &a) {
+    it = dg_item(++k);
+    if (it >= a.nct * a.nitems) return false;
+    ct = it % a.nct;
+    m = next.x;
+    nt = next.y;
+    mi = minext;
+    next = after;
+    after = entry(a, dg_item(k + 2));
+    minext = a.mi[next.x];
+    return true;
+  }
+};
+
 template <int DIR>
 __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid_constant__ DgArgs a) {
   constexpr int NSTAGE = DG_NSTAGE, NACC = DG_NACC;
@@ -179,7 +247,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const int nitems = a.nct * a.nitems;
+  DgWalk w(a);  // (tables: nothing that the kernel before writes)
   pdl_wait();
   pdl_trigger();
 
@@ -188,23 +256,23 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
     if (lane == 0 && !a.withhold) {
       int g = 0;
       bool ok = true;
-      for (int k = 0, it = dg_item(0); it < nitems && ok; it = dg_item(++k)) {
-        const int2 w = a.items[it / a.nct];
-        const int ct = it % a.nct, m = w.x, nt = w.y;
-        const DgMInfo &mi = a.mi[m];
+      while (ok && w.step(a)) {
+        const int ct = w.ct, nt = w.nt;
+        const DgMInfo &mi = w.mi;
         // rows of the column tile that hold data (whole groups of 8)
         const int rows = min(128, ((2 * a.batch - a.c0 - ct * 128) + 7) & ~7);
         for (int p = 0; p < 2 && ok; ++p) {
-          if (nt * TN >= mi.nr[p]) continue;
-          const int ntw = min(TN, mi.nr[p] - nt * TN);
-          const unsigned char *Bt =
-              a.B + mi.tab[p] + (long long)nt * TN * mi.nq[p] * (DG_SLICES * DG_ROW);
-          for (int q = 0; q < mi.nq[p]; ++q, ++g) {
+          const int nr = p ? mi.nr[1] : mi.nr[0], nq = p ? mi.nq[1] : mi.nq[0];
+          if (nt * TN >= nr) continue;
+          const int ntw = min(TN, nr - nt * TN);
+          const uint32_t bb = (uint32_t)(DG_SLICES * DG_ROW * ntw);
+          const unsigned char *Bt = a.B + (p ? mi.tab[1] : mi.tab[0]) + (long long)nt * TN * nq * (DG_SLICES * DG_ROW);
+          const unsigned char *At = a.A + ((long long)ct * a.nchunk + (p ? mi.ch[1] : mi.ch[0])) * DG_A_BYTES;
+          for (int q = 0; q < nq; ++q, ++g) {
             const int s = g % NSTAGE;
             if (!mbar_wait(&empty[s], ((g / NSTAGE) & 1) ^ 1, a.err, abort_flag, 1, a.wait_ns)) { ok = false; break; }
             unsigned char *As = stage + s * DG_STAGE;
-            const unsigned char *Ag = a.A + ((long long)ct * a.nchunk + mi.ch[p] + q) * DG_A_BYTES;
-            const uint32_t bb = (uint32_t)(DG_SLICES * DG_ROW * ntw);
+            const unsigned char *Ag = At + (long long)q * DG_A_BYTES;
             mbar_arrive_tx(&full[s], (uint32_t)(DG_SLICES * DG_ROW * rows) + bb);
             bulk_load(As + DG_A_BYTES, Bt + (long long)q * bb, bb, &full[s]);
             if (rows == 128) {
@@ -227,26 +295,26 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
     if (lane == 0) {
       int g = 0, seg = 0;
       bool ok = true;
-      for (int k = 0, it = dg_item(0); it < nitems && ok; it = dg_item(++k)) {
-        const int2 w = a.items[it / a.nct];
-        const int m = w.x, nt = w.y;
-        const DgMInfo &mi = a.mi[m];
+      while (ok && w.step(a)) {
+        const int nt = w.nt;
+        const DgMInfo &mi = w.mi;
         for (int p = 0; p < 2 && ok; ++p) {
-          if (nt * TN >= mi.nr[p]) continue;
-          const int ntw = min(TN, mi.nr[p] - nt * TN);
-          for (int q0 = 0; q0 < mi.nq[p] && ok; q0 += DG_KB, ++seg) {
+          const int nr = p ? mi.nr[1] : mi.nr[0], nq = p ? mi.nq[1] : mi.nq[0], kv = p ? mi.kv[1] : mi.kv[0];
+          if (nt * TN >= nr) continue;
+          const int ntw = min(TN, nr - nt * TN);
+          for (int q0 = 0; q0 < nq && ok; q0 += DG_KB, ++seg) {
             const int set = seg % NACC;
             if (!mbar_wait(&acce[set], ((seg / NACC) & 1) ^ 1, a.err, abort_flag, 2, a.wait_ns)) { ok = false; break; }
             tc_fence_after();
             const uint32_t acc = tmem + set * 256;
             int first = 0;  // 0 until the accumulators have been written
-            for (int q = q0; q < min(mi.nq[p], q0 + DG_KB); ++q, ++g) {
+            for (int q = q0; q < min(nq, q0 + DG_KB); ++q, ++g) {
               const int s = g % NSTAGE;
               if (!mbar_wait(&full[s], (g / NSTAGE) & 1, a.err, abort_flag, 3, a.wait_ns)) { ok = false; break; }
               tc_fence_after();
               const uint32_t As = smem_u32(stage + s * DG_STAGE);
               const uint64_t da = dg_desc(As), db = dg_desc(As + DG_A_BYTES);
-              const int ks = min(2, (mi.kv[p] - q * DG_CHUNK + 15) / 16);
+              const int ks = min(2, (kv - q * DG_CHUNK + 15) / 16);
               if (ntw == TN) dg_mma<TN>(acc, da, db, ks, first);
               else dg_mma<16>(acc, da, db, ks, first);
               first = 1;
@@ -271,14 +339,15 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
     const int C2B = 2 * a.batch;
     int seg = 0;
     bool dead = false;
-    for (int k = 0, it = dg_item(0); it < nitems && !dead; it = dg_item(++k)) {
-      const int2 w = a.items[it / a.nct];
-      const int ct = it % a.nct, m = w.x, nt = w.y;
-      const DgMInfo &mi = a.mi[m];
+    while (!dead && w.step(a)) {
+      const int ct = w.ct, m = w.m, nt = w.nt;
+      const DgMInfo &mi = w.mi;
       const int c = a.c0 + ct * 128 + row;
       const bool live = c < C2B;
+      const int r0 = nt * TN + j0;  // first row of the table
       // inverse: both parities' sums; forward: the current parity's
       DgSum sum[DIR == 0 ? 2 : 1][EC];
+      int E = 0, ex[EC];  // scale exponents of A's column and the table's rows
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
         DgSum(&S)[EC] = sum[DIR == 0 ? p : 0];
@@ -286,6 +355,15 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
         for (int x = 0; x < EC; ++x) S[x] = DgSum{0, 0.f};
         if (nt * TN >= mi.nr[p]) continue;
         const int ntw = min(TN, mi.nr[p] - nt * TN);
+        const int nx = live ? mi.nv[p] - r0 : 0;  // columns k of the tile with a result
+        // loaded ahead of the sums they scale
+        if ((DIR == 1 || p == 0) && nx > 0) {
+          E = a.ea[(long long)(DIR == 0 ? m : 2 * m + p) * a.ldea + c];
+          // forward: n = m + p + 2 (r0 + x)
+          const short *eb = a.eb + mi.eb[p] + (DIR == 0 ? r0 : p + 2 * r0);
+#pragma unroll
+          for (int x = 0; x < EC; ++x) ex[x] = x < nx ? eb[DIR == 0 ? x : 2 * x] : 0;
+        }
         for (int q0 = 0; q0 < mi.nq[p]; q0 += DG_KB, ++seg) {
           const int set = seg % NACC;
           if (!mbar_wait(&accf[set], (seg / NACC) & 1, a.err, abort_flag, 4, a.wait_ns)) {
@@ -312,37 +390,31 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
           mbar_arrive(&acce[set]);
         }
         if (dead) break;
-        if (DIR == 1 && live && j0 < ntw) {
-          // column k of the tile is n = m + p + 2 (nt TN + k)
-          const int E = a.ea[(long long)(2 * m + p) * a.ldea + c];
-          const long long id0 = mi.eb[p] + p + 2 * (nt * TN + j0);
-          double *dst = a.out + ((long long)(c >> 1) * a.ncoef + id0) * 2 + (c & 1);
-#pragma unroll
-          for (int x = 0; x < EC; ++x)
-            if (nt * TN + j0 + x < mi.nv[p]) {
-              double v = dg_to_double(S[x], E - 1022 + a.eb[id0 + 2 * x] - 52);
-              if (E >= a.enan) v = __longlong_as_double(0x7FF8000000000000ll);
-              dst[4 * x] = (m == 0 && (c & 1)) ? 0.0 : v;
-            }
+        if (DIR == 1 && nx > 0) {
+          double *dst = a.out + ((long long)(c >> 1) * a.ncoef + mi.eb[p] + p + 2 * r0) * 2 + (c & 1);
+          const bool zero = m == 0 && (c & 1);
+          unsigned any = 0;
+          const int up = dg_room(S, any);
+          dg_results<EC>(ex, E, up, a.enan, [&](int x, auto conv) {
+            const double v = conv(dg_sum_fixed(S[x], up), x);
+            if (x < nx) dst[4 * x] = zero ? 0.0 : v;
+          });
         }
       }
-      if (DIR == 0 && !dead && live) {
-        const int E = a.ea[(long long)m * a.ldea + c];
-        const int jb = nt * TN + j0;
-        const short *eb = a.eb + mi.eb[0] + jb;
-        double *Fn = a.out + ((long long)m * 2 * a.Jh + a.Jh + jb) * C2B + c;      // latitude Jh + jj
-        double *Fs = a.out + ((long long)m * 2 * a.Jh + a.Jh - 1 - jb) * C2B + c;  // its mirror
-#pragma unroll
-        for (int x = 0; x < EC; ++x)
-          if (jb + x < a.Jh) {
-            const int ex = E - 1022 + eb[x] - 52;
-            const DgSum &e = sum[0][x], &o = sum[DIR == 0][x];
-            double fn = dg_to_double(DgSum{e.t + o.t, e.l + o.l}, ex);
-            double fs = dg_to_double(DgSum{e.t - o.t, e.l - o.l}, ex);
-            if (E >= a.enan) fn = fs = __longlong_as_double(0x7FF8000000000000ll);
-            Fn[(long long)x * C2B] = fn;
-            Fs[-(long long)x * C2B] = fs;
+      if (DIR == 0 && !dead && live && r0 < a.Jh) {
+        double *Fn = a.out + ((long long)m * 2 * a.Jh + a.Jh + r0) * C2B + c;      // latitude Jh + jj
+        double *Fs = a.out + ((long long)m * 2 * a.Jh + a.Jh - 1 - r0) * C2B + c;  // its mirror
+        unsigned any = 0;
+        dg_room(sum[0], any);
+        const int up = dg_room(sum[DIR == 0], any) - 1;  // for e + o and e - o
+        dg_results<EC>(ex, E, up, a.enan, [&](int x, auto conv) {
+          const long long e = dg_sum_fixed(sum[0][x], up), o = dg_sum_fixed(sum[DIR == 0][x], up);
+          const double n = conv(e + o, x), s = conv(e - o, x);
+          if (r0 + x < a.Jh) {
+            Fn[(long long)x * C2B] = n;
+            Fs[-(long long)x * C2B] = s;
           }
+        });
       }
     }
   }
@@ -633,7 +705,10 @@ int legendre_inv_f64(Plan &P, int batch, const double *spec, double *F, cudaStre
     const int k = nct - t < P.dg_ct ? nct - t : P.dg_ct;
     const int b0 = 64 * t, nb = batch - b0 < 64 * k ? batch - b0 : 64 * k;
     // lanes a (m, field-level): 2 units of 8 for every 16 coefficients
-    if (P.N < 128)
+    if (P.N >= 64 && P.N < 128)
+      DCCM_CUDA(launch_pdl(dg_pack_spec<16>, dim3((nb + 15) / 16, P.N + 1), dim3(256), 0, s, mi, P.N, (long long)P.ncoef,
+                           (const double2 *)spec, b0, nb, P.dinv.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea));
+    else if (P.N < 128)
       DCCM_CUDA(launch_pdl(dg_pack_spec<8>, dim3((nb + 31) / 32, P.N + 1), dim3(256), 0, s, mi, P.N, (long long)P.ncoef,
                            (const double2 *)spec, b0, nb, P.dinv.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea));
     else

@@ -25,6 +25,7 @@
 // sets at k = 1 (:199, :237, :272), as the reference does: the coupler
 // replaces U, V, T and the vapour tracer there with the surface solution
 // before the backward sweep (atm/dccm_atm_mod.f90:832-835).
+#include <algorithm>
 #include <new>
 
 #include "common.cuh"
@@ -34,7 +35,10 @@
 struct dccm_implcpl {
   int ncol = 0, kmax = 0, ncmax = 0, ih2o = 1;
   dccm_implcpl_consts k;
-  double *d_mtx = nullptr;  // UV, Temp, QMix: each (ncol, kmax, -1:1)
+  // kmax x ncol each: the diagonals M(k,0) of UV, Temp and QMix after the
+  // forward sweep (M(k,-1) is then 1 and M(k,1) 0), and that sweep's shared
+  // factors G, 1/Exner_f and the mass term
+  double *d_mtx = nullptr;
   dccm::DevBuf stage;       // host entry points
   cudaStream_t stream = nullptr;
 };
@@ -45,7 +49,7 @@ namespace implcpl {
 struct Fwd {
   const double *MomX, *MomY, *Heat, *QFlx, *P, *Ef, *Eh, *Tv, *Z, *Kv, *Kt, *Kq;
   double *DU, *DV, *DT, *DQ, *C1, *C2;
-  double *uv, *tm, *qm;
+  double *mtx;  // M(k,0) of UV, Temp and QMix
   double *G, *IEF, *Mass;  // per (level, column) factors shared by the systems (geo_kernel)
   long long ncol;
   int kmax, ncmax, ih2o;
@@ -60,8 +64,7 @@ struct Fwd {
 // the model top down builds each level's row (:188-308) and eliminates it
 // at once (:380-405), carrying the eliminated M(k+1,0) and right-hand sides
 // of the level above; the eliminated matrix and tendencies are written
-// once.  The level inputs are fetched LV levels ahead into registers, so
-// the loads of a chunk overlap while the serial elimination runs.
+// once.  The next level's inputs are fetched while one is eliminated.
 //
 // With the couplings' magnitudes l = -M(k,-1), u = -M(k,1) and a = -M(k+1,0),
 // all positive in an ordinary column, the elimination
@@ -74,14 +77,18 @@ struct Fwd {
 // The top and bottom rows, and rows where a coupling is zero, negative, not
 // finite or beyond 2^+-100, take the reference's form in FP64 (a warp
 // decides as one).  FP64 was the sweeps' limit (67 operations a column and
-// level forward, 21 backward; now 12 and 8): 32,768 columns x 32 levels forward
-// 174 -> 95 us, backward 71 -> 35 us; 131,072 x 48 849 -> 397 and 253 -> 172 us.
+// level forward, 21 backward; now 12 and 8): with these, forward sweeps of
+// 32,768 columns x 32 levels took 95 us (174 in FP64), backward 35 (71).
 // What is left is the sum of three pipes' work (the ALU's about as long as
-// FP64's) with five warps a scheduler; two levels fetched ahead at 102
-// registers and five CTAs an SM beat four at 128 (95 against 99, 397 against
-// 401 us).
-constexpr int LV = 2;   // forward sweep: levels fetched ahead
-constexpr int LVB = 8;  // backward sweep
+// FP64's).  The level after the current one is always being fetched: 95 -> 75
+// us, 131,072 x 48 397 -> 324, against two levels fetched together ahead of
+// their use (five CTAs an SM at 102 registers or four at 128).  The backward
+// sweep fetches LVB ahead in the same way (FP64 pipe 66 % busy; with eight
+// unrolled and one copy of the code for each matrix a quarter of its cycles
+// waited for instructions: 131,072 x 48 172 -> 150 us); its CTAs are of 64
+// threads, so that its three kinds of block spread evenly (32,768 x 32 35 -> 33).
+constexpr int GL = 2;   // levels a thread of geo_kernel
+constexpr int LVB = 2;  // backward sweep: levels fetched ahead
 
 // positive, exponent field in [lo, hi]
 __device__ __forceinline__ bool pos_in(double x, unsigned lo, unsigned hi) {
@@ -98,26 +105,45 @@ __device__ __forceinline__ bool usual(double x) { return pos_in(x, 923, 1123); }
 // j = 1..kmax-1 (the transfer coefficient of :182-195 is K(j) G(j)), the
 // reciprocal Exner function 1 / Exner_f(j) at full level j (0-based index,
 // the temperature rows of :222-260), and the mass term of that level's row.
+// A thread takes GL levels of a column (131,072 x 48: forward sweep 333 us with
+// one, 324 with two, 326 with four, which has too few threads at 8,192).
 __global__ void __launch_bounds__(256) geo_kernel(const Fwd a) {
-  const long long n = a.ncol;
+  pdl_trigger();
+  const long long n = a.ncol, K = a.kmax;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= n * a.kmax) return;
-  const int j = (int)(t / n);
-  const long long c = t - j * n;
-  const double P0 = a.P[c + n * j];
-  a.Mass[t] = (P0 - a.P[c + n * (j + 1)]) * a.inv_g2dt;
-  a.IEF[t] = fx::rcp_d(a.Ef[c + n * j]);
-  if (j >= 1) {
-    const double Tv = a.Tv[c + n * j], dz = a.Z[c + n * j] - a.Z[c + n * (j - 1)];
-    double g;
-    if (a.fast && usual(P0) && usual(Tv) && usual(dz)) {
-      using namespace fx;
-      const UF d = mul(mul(from_double(Tv), a.uGasR), from_double(dz));
-      g = to_double(mul(from_double(P0), rcp(norm(d))));
-    } else {
-      g = P0 * fx::rcp_d(a.GasR * Tv * dz);
+  const int j0 = (int)(t / n) * GL;
+  const long long c = t % n;
+  if (j0 >= K) return;
+  double P[GL + 1], Z[GL + 1], Tv[GL], Ef[GL];
+#pragma unroll
+  for (int i = 0; i <= GL; ++i) {
+    const int j = j0 + i;
+    P[i] = j <= K ? a.P[c + n * j] : 1.0;
+    Z[i] = j >= 1 && j <= K ? a.Z[c + n * (j - 1)] : 0.0;  // full level j - 1
+    if (i < GL) {
+      Tv[i] = j >= 1 && j < K ? a.Tv[c + n * j] : 1.0;
+      Ef[i] = j < K ? a.Ef[c + n * j] : 1.0;
     }
-    a.G[t] = g;
+  }
+#pragma unroll
+  for (int i = 0; i < GL; ++i) {
+    const int j = j0 + i;
+    if (j >= K) break;
+    const long long o = c + n * j;
+    a.Mass[o] = (P[i] - P[i + 1]) * a.inv_g2dt;
+    a.IEF[o] = fx::rcp_d(Ef[i]);
+    if (j >= 1) {
+      const double dz = Z[i + 1] - Z[i];
+      double g;
+      if (a.fast && usual(P[i]) && usual(Tv[i]) && usual(dz)) {
+        using namespace fx;
+        const UF d = mul(mul(from_double(Tv[i]), a.uGasR), from_double(dz));
+        g = to_double(mul(from_double(P[i]), rcp(norm(d))));
+      } else {
+        g = P[i] * fx::rcp_d(a.GasR * Tv[i] * dz);
+      }
+      a.G[o] = g;
+    }
   }
 }
 
@@ -144,7 +170,6 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
   const unsigned warp = __activemask();
   const long long n = a.ncol;
   const int K = a.kmax;
-  const long long mstr = n * K;
   const double *__restrict__ Kd = SYS == 0 ? a.Kv : (SYS == 1 ? a.Kt : a.Kq);
   const double *__restrict__ fl[NR];
   double *__restrict__ out[NR];
@@ -160,7 +185,7 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
     fl[0] = a.QFlx + n * (long long)(K + 1) * tracer;
     out[0] = a.DQ + n * (long long)K * tracer;
   }
-  double *mat = SYS == 0 ? a.uv : (SYS == 1 ? a.tm : a.qm);
+  double *mat = a.mtx + SYS * n * K;
   const bool store_mat = SYS != 2 || tracer == 0;
   // values at level k carried from the previous (upper) iteration
   double flk[NR];
@@ -173,120 +198,115 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
   // Cp Exner_h), 1 / a
   UF upU{1ull << 63, 0}, qU{1ull << 63, 0};
   bool upv = false, qv = false;
-  for (int k0 = K; k0 >= 1; k0 -= LV) {
-    // fetch half level k-1 and full level k-1 of the next LV levels
-    double Mm[LV], Gm[LV], Kdm[LV], Ehm[LV], Iefm[LV], flm[LV][NR];
-#pragma unroll
-    for (int i = 0; i < LV; ++i) {
-      const int k = k0 - i;
-      if (k >= 1) {
-        Mm[i] = a.Mass[c + n * (k - 1)];
-        if (k > 1) {
-          Gm[i] = a.G[c + n * (k - 1)];
-          Kdm[i] = Kd[c + n * (k - 1)];
-          if (SYS == 1) {
-            Ehm[i] = a.Eh[c + n * (k - 1)];
-            Iefm[i] = a.IEF[c + n * (k - 2)];
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < NR; ++r) flm[i][r] = fl[r][c + n * (k - 1)];
+  // half level k-1 and full level k-1 of the coming level k
+  double Mn = 0.0, Gn = 0.0, Kdn = 0.0, Ehn = 0.0, Iefn = 0.0, fln[NR];
+  auto fetch = [&](int k) {
+    if (k < 1) return;
+    Mn = a.Mass[c + n * (k - 1)];
+    if (k > 1) {
+      Gn = a.G[c + n * (k - 1)];
+      Kdn = Kd[c + n * (k - 1)];
+      if (SYS == 1) {
+        Ehn = a.Eh[c + n * (k - 1)];
+        Iefn = a.IEF[c + n * (k - 2)];
       }
     }
 #pragma unroll
-    for (int i = 0; i < LV; ++i) {
-      const int k = k0 - i;
-      if (k < 1) break;
-      const double ief_km = SYS == 1 && k > 1 ? Iefm[i] : 0.0;
-      // transfer coefficient of half level k-1 (SYS 1: times Cp Exner_h)
-      UF lowU{1ull << 63, 0};
-      bool lv = false;
-      if (k > 1) {
-        lv = a.fast && usual(Kdm[i]) && usual(Gm[i]);
-        if (SYS == 1) lv = lv && usual(Ehm[i]) && usual(ief_km);
-        lowU = fx::mul(fx::from_double(Kdm[i]), fx::from_double(Gm[i]));
-        if (SYS == 1) lowU = fx::mul(fx::mul(lowU, a.uCp), fx::from_double(Ehm[i]));
-        lowU = fx::norm(lowU);
-      }
-      double b[NR], re[NR], m0e;
+    for (int r = 0; r < NR; ++r) fln[r] = fl[r][c + n * (k - 1)];
+  };
+  fetch(K);
+#pragma unroll 1
+  for (int k = K; k >= 1; --k) {
+    const double Mm = Mn, Gm = Gn, Kdm = Kdn, Ehm = Ehn;
+    double flm[NR];
 #pragma unroll
-      for (int r = 0; r < NR; ++r) b[r] = flm[i][r] - flk[r];
-      bool done = false;
-      if (__all_sync(warp, lv && upv && qv && usual(Mm[i]))) {
-        // row k: its diagonal mass + l' + u', the couplings l and u (SYS 1: the
-        // couplings with their own level's Exner function, l' and u' with k's)
-        UF mU = fx::from_double(Mm[i]), l = lowU, u = upU, l0 = lowU, u0 = upU;
-        if (SYS == 1) {
-          const UF ik = fx::from_double(ief_k);
-          mU = fx::mul(mU, a.uCp);
-          l0 = fx::mul(lowU, ik);
-          u0 = fx::mul(upU, ik);
-          l = fx::norm(fx::mul(lowU, fx::from_double(ief_km)));
-          u = fx::mul(upU, fx::from_double(ief_k1));
-        }
-        const UF cU = fx::mul(u, qU);
-        UF dU;
-        if (__all_sync(warp, fx::sub(fx::sum3(mU, l0, u0), cU, dU))) {
-          const UF iU = fx::rcp(l);
-          qU = fx::mul(l, fx::rcp(dU));
-          const double il = fx::to_double(iU), cc = fx::to_double(cU);
-          m0e = negd(fx::to_double(fx::mul(dU, iU)));
+    for (int r = 0; r < NR; ++r) flm[r] = fln[r];
+    const double ief_km = SYS == 1 && k > 1 ? Iefn : 0.0;
+    fetch(k - 1);
+    // transfer coefficient of half level k-1 (SYS 1: times Cp Exner_h)
+    UF lowU{1ull << 63, 0};
+    bool lv = false;
+    if (k > 1) {
+      lv = a.fast && usual(Kdm) && usual(Gm);
+      if (SYS == 1) lv = lv && usual(Ehm) && usual(ief_km);
+      lowU = fx::mul(fx::from_double(Kdm), fx::from_double(Gm));
+      if (SYS == 1) lowU = fx::mul(fx::mul(lowU, a.uCp), fx::from_double(Ehm));
+      lowU = fx::norm(lowU);
+    }
+    double b[NR], re[NR], m0e;
 #pragma unroll
-          for (int r = 0; r < NR; ++r) re[r] = fma(cc, rp[r], -b[r]) * il;
-          done = true;
-        }
+    for (int r = 0; r < NR; ++r) b[r] = flm[r] - flk[r];
+    bool done = false;
+    if (__all_sync(warp, lv && upv && qv && usual(Mm))) {
+      // row k: its diagonal mass + l' + u', the couplings l and u (SYS 1: the
+      // couplings with their own level's Exner function, l' and u' with k's)
+      UF mU = fx::from_double(Mm), l = lowU, u = upU, l0 = lowU, u0 = upU;
+      if (SYS == 1) {
+        const UF ik = fx::from_double(ief_k);
+        mU = fx::mul(mU, a.uCp);
+        l0 = fx::mul(lowU, ik);
+        u0 = fx::mul(upU, ik);
+        l = fx::norm(fx::mul(lowU, fx::from_double(ief_km)));
+        u = fx::mul(upU, fx::from_double(ief_k1));
       }
-      if (!done) {
-        // row k as the reference builds (:182-256) and eliminates it; +0
-        // where it assigns 0
-        const double tkm = k > 1 ? Kdm[i] * Gm[i] : 0.0, tck = Kdk * Gk;
-        double mm, m0, mp;
-        if constexpr (SYS != 1) {
-          m0 = Mm[i] + tkm + tck;
-          mm = k > 1 ? -tkm : 0.0;
-          mp = k < K ? -tck : 0.0;
-          if (k == 1) tc1 = tck;
-        } else {
-          const double ehm = k > 1 ? a.CpDry * Ehm[i] * tkm : 0.0, ehk = a.CpDry * Ehk * tck;
-          m0 = a.CpDry * Mm[i] + ehm * ief_k + ehk * ief_k;
-          mm = k > 1 ? -(ehm * ief_km) : 0.0;
-          mp = k < K ? -(ehk * ief_k1) : 0.0;
-          if (k == 1) {
-            dfadt1 = ehk * ief_k;  // DFADT1 = Cp Exner_h(1) TTC(1) / Exner_f(1)
-            dfadt2 = mp;           // DFADT2 = -Cp Exner_h(1) TTC(1) / Exner_f(2)
-          }
-        }
-        const Row w = eliminate_fp64(k == K, mm, m0, mp, m0p, b[0], b[NR - 1], rp[0], rp[NR - 1]);
-        m0e = w.m0;
-        re[0] = w.r[0];
-        if (NR == 2) re[NR - 1] = w.r[1];
-        qU = fx::rcp(fx::from_double(negd(m0e)));
-      }
-      qv = pos_in(negd(m0e), 723, 1323);
-      upU = lowU;
-      upv = lv;
+      const UF cU = fx::mul(u, qU);
+      UF dU;
+      if (__all_sync(warp, fx::sub(fx::sum3(mU, l0, u0), cU, dU))) {
+        const UF iU = fx::rcp(l);
+        qU = fx::mul(l, fx::rcp(dU));
+        const double il = fx::to_double(iU), cc = fx::to_double(cU);
+        m0e = negd(fx::to_double(fx::mul(dU, iU)));
 #pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        if (k == 1) c2[r] = b[r];  // ImplCplCoef2 starts from the level-1 divergence (:310-313)
-        out[r][c + n * (k - 1)] = re[r];
-        rp[r] = re[r];
-        if (k == 2) r_2[r] = re[r];
-        flk[r] = flm[i][r];
+        for (int r = 0; r < NR; ++r) re[r] = fma(cc, rp[r], -b[r]) * il;
+        done = true;
       }
-      if (store_mat) {
-        mat[c + n * (k - 1)] = 1.0;
-        mat[c + n * (k - 1) + mstr] = m0e;
-        mat[c + n * (k - 1) + 2 * mstr] = 0.0;
+    }
+    if (!done) {
+      // row k as the reference builds (:182-256) and eliminates it; +0
+      // where it assigns 0
+      const double tkm = k > 1 ? Kdm * Gm : 0.0, tck = Kdk * Gk;
+      double mm, m0, mp;
+      if constexpr (SYS != 1) {
+        m0 = Mm + tkm + tck;
+        mm = k > 1 ? -tkm : 0.0;
+        mp = k < K ? -tck : 0.0;
+        if (k == 1) tc1 = tck;
+      } else {
+        const double ehm = k > 1 ? a.CpDry * Ehm * tkm : 0.0, ehk = a.CpDry * Ehk * tck;
+        m0 = a.CpDry * Mm + ehm * ief_k + ehk * ief_k;
+        mm = k > 1 ? -(ehm * ief_km) : 0.0;
+        mp = k < K ? -(ehk * ief_k1) : 0.0;
+        if (k == 1) {
+          dfadt1 = ehk * ief_k;  // DFADT1 = Cp Exner_h(1) TTC(1) / Exner_f(1)
+          dfadt2 = mp;           // DFADT2 = -Cp Exner_h(1) TTC(1) / Exner_f(2)
+        }
       }
-      if (k == 2) m0_2 = m0e;
-      m0p = m0e;
-      ief_k1 = ief_k;
-      ief_k = ief_km;
-      if (k > 1) {
-        Kdk = Kdm[i];
-        Gk = Gm[i];
-        if (SYS == 1) Ehk = Ehm[i];
-      }
+      const Row w = eliminate_fp64(k == K, mm, m0, mp, m0p, b[0], b[NR - 1], rp[0], rp[NR - 1]);
+      m0e = w.m0;
+      re[0] = w.r[0];
+      if (NR == 2) re[NR - 1] = w.r[1];
+      qU = fx::rcp(fx::from_double(negd(m0e)));
+    }
+    qv = pos_in(negd(m0e), 723, 1323);
+    upU = lowU;
+    upv = lv;
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      if (k == 1) c2[r] = b[r];  // ImplCplCoef2 starts from the level-1 divergence (:310-313)
+      out[r][c + n * (k - 1)] = re[r];
+      rp[r] = re[r];
+      if (k == 2) r_2[r] = re[r];
+      flk[r] = flm[r];
+    }
+    if (store_mat) mat[c + n * (k - 1)] = m0e;
+    if (k == 2) m0_2 = m0e;
+    m0p = m0e;
+    ief_k1 = ief_k;
+    ief_k = ief_km;
+    if (k > 1) {
+      Kdk = Kdm;
+      Gk = Gm;
+      if (SYS == 1) Ehk = Ehm;
     }
   }
   // coupling coefficients (:342-375); DFADUV1 = -DFADUV2 = TC(1)
@@ -309,7 +329,8 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
   }
 }
 
-__global__ void __launch_bounds__(128, 5) forward_kernel(const Fwd a) {
+__global__ void __launch_bounds__(128, 4) forward_kernel(const Fwd a) {
+  pdl_wait();
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= a.ncol) return;
   if (blockIdx.y == 0) forward_column<0>(a, c, 0);
@@ -320,12 +341,12 @@ __global__ void __launch_bounds__(128, 5) forward_kernel(const Fwd a) {
 // Back substitution (:407-420) and the division by 2 dt (:53-61), one
 // thread per (column, matrix): blockIdx.y 0 = momentum (U and V), 1 =
 // temperature, 2 = the tracers; one reciprocal of M(k,0) per level serves
-// every right-hand side of the matrix, and levels are fetched LVB at a time
-// ahead of the serial chains.  M(k,-1) is 1 after the forward sweep and is
+// every right-hand side of the matrix, and the next LVB levels are fetched
+// while the chains run through the current ones.  M(k,-1) is 1 after the forward sweep and is
 // not read; the reciprocals and the products with 1 / (2 dt) run on the
 // integer pipes.
 struct Bwd {
-  const double *uv, *tm, *qm;
+  const double *mtx;  // M(k,0) of UV, Temp and QMix
   double *DU, *DV, *DT, *DQ;
   long long ncol;
   int kmax, ncmax;
@@ -334,63 +355,63 @@ struct Bwd {
 };
 
 template <int NR>
-__device__ __forceinline__ void backward_chains(const double *__restrict__ mat, double *const *x, long long c,
+__device__ __forceinline__ void backward_chains(const double *__restrict__ mat, double *x0, double *x1, long long c,
                                                 long long n, int K, double inv_2dt, fx::UF u2dt) {
-  const long long mstr = n * K;
+  double *x[2] = {x0, x1};
   double v[NR];
+  double xs[LVB][NR], m0[LVB];
+  auto load = [&](int k0) {
 #pragma unroll
-  for (int r = 0; r < NR; ++r) {
-    v[r] = x[r][c];
-    x[r][c] = fx::scale_d(v[r], u2dt, inv_2dt);
-  }
-  for (int k0 = 2; k0 <= K; k0 += LVB) {
-    double xs[LVB][NR], m0[LVB];
-#pragma unroll
-    for (int i = 0; i < LVB; ++i) {
-      const int k = k0 + i;
-      if (k <= K) {
-        const long long o = c + n * (k - 1);
+    for (int i = 0; i < LVB; ++i)
+      if (k0 + i <= K) {
+        const long long o = c + n * (k0 + i - 1);
 #pragma unroll
         for (int r = 0; r < NR; ++r) xs[i][r] = x[r][o];
-        m0[i] = mat[o + mstr];
+        m0[i] = mat[o];
       }
-    }
+  };
+#pragma unroll
+  for (int r = 0; r < NR; ++r) v[r] = x[r][c];
+  load(2);
+#pragma unroll
+  for (int r = 0; r < NR; ++r) x[r][c] = fx::scale_d(v[r], u2dt, inv_2dt);
+#pragma unroll 1
+  for (int k0 = 2; k0 <= K; k0 += LVB) {
+    double ys[LVB][NR], p0[LVB];
 #pragma unroll
     for (int i = 0; i < LVB; ++i) {
-      const int k = k0 + i;
-      if (k > K) break;
-      const double im = fx::rcp_d(m0[i]);
+      p0[i] = m0[i];
+#pragma unroll
+      for (int r = 0; r < NR; ++r) ys[i][r] = xs[i][r];
+    }
+    load(k0 + LVB);
+#pragma unroll
+    for (int i = 0; i < LVB; ++i) {
+      if (k0 + i > K) break;
+      const long long o = c + n * (k0 + i - 1);
+      const double im = fx::rcp_d(p0[i]);
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
-        v[r] = (xs[i][r] - v[r]) * im;
-        x[r][c + n * (k - 1)] = fx::scale_d(v[r], u2dt, inv_2dt);
+        v[r] = (ys[i][r] - v[r]) * im;
+        x[r][o] = fx::scale_d(v[r], u2dt, inv_2dt);
       }
     }
   }
 }
 
-__global__ void __launch_bounds__(128) backward_kernel(const Bwd a) {
+__global__ void __launch_bounds__(64, 16) backward_kernel(const Bwd a) {
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= a.ncol) return;
   const long long n = a.ncol;
-  const int K = a.kmax;
-  if (blockIdx.y == 0) {
-    double *x[2] = {a.DU, a.DV};
-    backward_chains<2>(a.uv, x, c, n, K, a.inv_2dt, a.u2dt);
-  } else if (blockIdx.y == 1) {
-    double *x[1] = {a.DT};
-    backward_chains<1>(a.tm, x, c, n, K, a.inv_2dt, a.u2dt);
-  } else {
-    // tracers in pairs (one reciprocal per level for both)
-    for (int t = 0; t < a.ncmax; t += 2) {
-      if (t + 1 < a.ncmax) {
-        double *x[2] = {a.DQ + n * (long long)K * t, a.DQ + n * (long long)K * (t + 1)};
-        backward_chains<2>(a.qm, x, c, n, K, a.inv_2dt, a.u2dt);
-      } else {
-        double *x[1] = {a.DQ + n * (long long)K * t};
-        backward_chains<1>(a.qm, x, c, n, K, a.inv_2dt, a.u2dt);
-      }
-    }
+  const int K = a.kmax, y = blockIdx.y;
+  const double *mat = a.mtx + y * n * K;
+  // tracers in pairs (one reciprocal per level for both)
+  const int nx = y == 0 ? 2 : y == 1 ? 1 : a.ncmax;
+  for (int t = 0; t < nx; t += 2) {
+    double *x0 = y == 0 ? a.DU : y == 1 ? a.DT : a.DQ + n * (long long)K * t;
+    double *x1 = y == 0 ? a.DV : x0 + n * (long long)K;
+    if (t + 1 < nx) backward_chains<2>(mat, x0, x1, c, n, K, a.inv_2dt, a.u2dt);
+    else backward_chains<1>(mat, x0, nullptr, c, n, K, a.inv_2dt, a.u2dt);
   }
 }
 
@@ -413,9 +434,7 @@ extern "C" int dccm_implcpl_create(int ncol, int kmax, int ncmax, int index_h2ov
   p->ncmax = ncmax;
   p->ih2o = index_h2ovap;
   p->k = *consts;
-  // the three matrices (3 diagonals each), then the forward sweep's shared
-  // factors G, 1/Exner_f and the mass term (kmax x ncol each)
-  const cudaError_t e = cudaMalloc(&p->d_mtx, (size_t)(3 * 3 + 3) * kmax * ncol * sizeof(double));
+  const cudaError_t e = cudaMalloc(&p->d_mtx, (size_t)6 * kmax * ncol * sizeof(double));
   if (e != cudaSuccess) {
     set_cuda_error(e);
     delete p;
@@ -435,7 +454,7 @@ extern "C" int dccm_implcpl_destroy(dccm_implcpl *p) {
   return DCCM_OK;
 }
 
-static size_t mstride(const dccm_implcpl *p) { return (size_t)3 * p->kmax * p->ncol; }
+static size_t mstride(const dccm_implcpl *p) { return (size_t)p->kmax * p->ncol; }
 
 // A constant the integer arithmetic takes: positive, within 2^+-100.
 static bool ordinary(double x) { return x > 0x1p-100 && x < 0x1p100; }
@@ -468,9 +487,7 @@ extern "C" int dccm_implcpl_forward_dev(dccm_implcpl *p, const dccm_implcpl_forw
   f.DQ = a->xyzf_DQMixDt;
   f.C1 = a->xya_ImplCplCoef1;
   f.C2 = a->xya_ImplCplCoef2;
-  f.uv = p->d_mtx;
-  f.tm = p->d_mtx + mstride(p);
-  f.qm = p->d_mtx + 2 * mstride(p);
+  f.mtx = p->d_mtx;
   f.ncol = p->ncol;
   f.kmax = p->kmax;
   f.ncmax = p->ncmax;
@@ -480,18 +497,17 @@ extern "C" int dccm_implcpl_forward_dev(dccm_implcpl *p, const dccm_implcpl_forw
   f.GasR = p->k.GasRDry;
   f.inv_g2dt = 1.0 / (p->k.Grav * (2.0 * p->k.DelTime));
   f.G = p->d_mtx + 3 * mstride(p);
-  f.IEF = f.G + (size_t)p->kmax * p->ncol;
-  f.Mass = f.IEF + (size_t)p->kmax * p->ncol;
+  f.IEF = f.G + mstride(p);
+  f.Mass = f.IEF + mstride(p);
   f.fast = ordinary(f.CpDry) && ordinary(f.GasR);
   f.uCp = fx::uf(f.fast ? f.CpDry : 1.0);
   f.uGasR = fx::uf(f.fast ? f.GasR : 1.0);
-  const long long nk = (long long)p->ncol * p->kmax;
+  const long long nk = (long long)p->ncol * ((p->kmax + implcpl::GL - 1) / implcpl::GL);
   implcpl::geo_kernel<<<(unsigned)((nk + 255) / 256), 256, 0, as_stream(stream)>>>(f);
   DCCM_LAUNCH_CHECK();
   const int threads = 128;
-  implcpl::forward_kernel<<<dim3((unsigned)((p->ncol + threads - 1) / threads), 2 + p->ncmax), threads, 0,
-                            as_stream(stream)>>>(f);
-  DCCM_LAUNCH_CHECK();
+  DCCM_CUDA(launch_pdl(implcpl::forward_kernel, dim3((unsigned)((p->ncol + threads - 1) / threads), 2 + p->ncmax),
+                       dim3(threads), 0, as_stream(stream), f));
   return DCCM_OK;
 }
 
@@ -500,9 +516,7 @@ extern "C" int dccm_implcpl_backward_dev(dccm_implcpl *p, double *xyz_DUDt, doub
   DCCM_NVTX_FUNC();
   if (!p || !xyz_DUDt || !xyz_DVDt || !xyz_DTempDt || !xyzf_DQMixDt) return DCCM_ERR_INVALID_ARG;
   implcpl::Bwd b;
-  b.uv = p->d_mtx;
-  b.tm = p->d_mtx + mstride(p);
-  b.qm = p->d_mtx + 2 * mstride(p);
+  b.mtx = p->d_mtx;
   b.DU = xyz_DUDt;
   b.DV = xyz_DVDt;
   b.DT = xyz_DTempDt;
@@ -513,7 +527,7 @@ extern "C" int dccm_implcpl_backward_dev(dccm_implcpl *p, double *xyz_DUDt, doub
   b.inv_2dt = 1.0 / (2.0 * p->k.DelTime);
   // an exponent that sends every product to the FP64 form where 1 / (2 dt) is not ordinary
   b.u2dt = ordinary(b.inv_2dt) ? fx::uf(b.inv_2dt) : fx::UF{0, 0};
-  const int threads = 128;
+  const int threads = 64;
   implcpl::backward_kernel<<<dim3((unsigned)((p->ncol + threads - 1) / threads), 3), threads, 0,
                              as_stream(stream)>>>(b);
   DCCM_LAUNCH_CHECK();
@@ -634,7 +648,12 @@ extern "C" int dccm_implcpl_matrices(dccm_implcpl *p, double *uv, double *temp, 
   DCCM_NVTX_FUNC();
   if (!p) return DCCM_ERR_INVALID_ARG;
   double *h[3] = {uv, temp, qmix};
+  const size_t n = mstride(p);
   for (int i = 0; i < 3; ++i)
-    if (h[i]) DCCM_CUDA(cudaMemcpy(h[i], p->d_mtx + i * mstride(p), mstride(p) * sizeof(double), cudaMemcpyDeviceToHost));
+    if (h[i]) {
+      DCCM_CUDA(cudaMemcpy(h[i] + n, p->d_mtx + i * n, n * sizeof(double), cudaMemcpyDeviceToHost));
+      std::fill(h[i], h[i] + n, 1.0);
+      std::fill(h[i] + 2 * n, h[i] + 3 * n, 0.0);
+    }
   return DCCM_OK;
 }

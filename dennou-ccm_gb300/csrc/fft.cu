@@ -250,6 +250,7 @@ __device__ __forceinline__ void warp_fft_inv(float2 (&v)[R], const float2 *tw, c
 constexpr int FFT_MAXG = 8;
 struct FftGroup {
   int N, J, batch, BB, lbb, R, W, blk0, C2Bp;  // BB row pairs per CTA, lbb = log2(BB), W warps per row pair
+  int ahead;         // forward: rows prefetched for the CTA this far on (0: none)
   const void *in;
   void *out;
   const float2 *tw, *twl;
@@ -837,6 +838,23 @@ __global__ void __launch_bounds__(512, 2) fft_multi_kernel(const __grid_constant
   const int nby = (G.batch + G.BB - 1) / G.BB;
   const int Jh = G.J / 2;
   const int by = FWD ? lb % nby : lb / Jh, jj = FWD ? lb / nby : lb % Jh;
+  if (FWD && (RFIX == 0 || RFIX >= 16) && G.ahead) {
+    // The rows of the CTA that starts `ahead` after this one, from HBM into
+    // L2: with two row pairs a warp a CTA comes back to memory between them,
+    // and 32 warps an SM do not hide that (T341 x 192 analysis 594 -> 540 us,
+    // T170 x 200 144 -> 138; 150 and more ahead, 557 us and up).  Rows of one
+    // warp in a launch of their own have more CTAs an SM: T85 x 512 75.7 and
+    // 75.4 us, and the question alone costs T85 x 128 0.3 us; an ensemble of
+    // lengths has not (members of T21 to T85 821 -> 803 us).
+    const int ln = lb + G.ahead;
+    const int jn = ln / nby, bn = ln % nby * G.BB, I = 32 * G.R;
+    const int bl = threadIdx.x >> 1;
+    if (jn < Jh && bl < G.BB && bn + bl < G.batch) {
+      const double *row = static_cast<const double *>(G.in) +
+                          ((long long)(bn + bl) * G.J + ((threadIdx.x & 1) ? Jh + jn : Jh - 1 - jn)) * I;
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(row), "r"(I * 8) : "memory");
+    }
+  }
   if constexpr (RFIX > 0) {
     dispatch_case<RFIX, RMAX, FWD>(G, jj, by, st);
   } else {
@@ -933,6 +951,8 @@ int fft_multi(Plan *const *plans, const int *batch, const void *const *in, void 
     G.out = out[g];
     G.tw = P.d_tw32;
     G.twl = P.d_twl32;
+    // bulk prefetches take 16-byte aligned rows
+    G.ahead = fwd && rp == 2 && reinterpret_cast<uintptr_t>(in[g]) % 16 == 0 ? 16 : 0;
     G.nsplit = P.nsplit;
     G.cexp = P.d_cexp ? P.d_cexp + P.max_batch : nullptr;
     if (fwd && P.nsplit == 2)

@@ -211,7 +211,11 @@ struct DgWalk {
   }
 };
 
-template <int DIR>
+// position of Re (im = 0) or Im s_n^m in SPML's real layout of a field-level
+__device__ __forceinline__ long long wa_at(int n, int m, int im) { return (long long)n * (n + 1) + (im ? -m : m); }
+
+// WA: forward results in SPML's real layout.
+template <int DIR, bool WA>
 __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid_constant__ DgArgs a) {
   constexpr int NSTAGE = DG_NSTAGE, NACC = DG_NACC;
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
@@ -393,11 +397,18 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
         if (DIR == 1 && nx > 0) {
           double *dst = a.out + ((long long)(c >> 1) * a.ncoef + mi.eb[p] + p + 2 * r0) * 2 + (c & 1);
           const bool zero = m == 0 && (c & 1);
+          const int nn = m + p + 2 * r0;  // n of the first result
+          if constexpr (WA) dst = a.out + (long long)(c >> 1) * (a.N + 1) * (a.N + 1) + wa_at(nn, m, c & 1);
           unsigned any = 0;
           const int up = dg_room(S, any);
           dg_results<EC>(ex, E, up, a.enan, [&](int x, auto conv) {
             const double v = conv(dg_sum_fixed(S[x], up), x);
-            if (x < nx) dst[4 * x] = zero ? 0.0 : v;
+            if constexpr (WA) {
+              // n (n + 1) grows by 2 x (2 nn + 1 + 2 x) over 2 x degrees
+              if (x < nx && !zero) dst[2 * x * (2 * nn + 1 + 2 * x)] = v;
+            } else if (x < nx) {
+              dst[4 * x] = zero ? 0.0 : v;
+            }
           });
         }
       }
@@ -432,7 +443,8 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
 // parities and for re and im), then write the digits; a lane takes 8
 // coefficients of one parity (n0 + p, n0 + p + 2, ...).  Whole chunks are
 // written, zeros past the last coefficient.
-template <int G>
+// WA: the spectra are in SPML's real layout (spml.cu).
+template <int G, bool WA>
 __global__ void __launch_bounds__(256)
 dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const double2 *__restrict__ spec, int b0, int nb,
              int nchunk, unsigned char *__restrict__ A, int *__restrict__ ea, int ldea) {
@@ -445,6 +457,11 @@ dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const doub
   const int b = b0 + (live ? bl : 0);
   const DgMInfo &mi = mi_[m];
   const double2 *src = spec + (long long)b * ncoef + idx_mn(N, m, m);
+  const double *wa = reinterpret_cast<const double *>(spec) + (long long)b * (N + 1) * (N + 1);
+  auto coefficient = [&](int n) {
+    if constexpr (WA) return make_double2(__ldg(wa + wa_at(n, m, 0)), m ? __ldg(wa + wa_at(n, m, 1)) : 0.0);
+    else return __ldg(src + (n - m));
+  };
   const int nu = 4 * max(mi.nq[0], mi.nq[1]);  // units of 8 a parity, both parities side by side
   unsigned mx = 0;
   double2 v[8];
@@ -452,7 +469,7 @@ dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const doub
     const int n0 = m + 16 * (t >> 1) + (t & 1);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      v[e] = live && n0 + 2 * e <= N ? __ldg(src + (n0 - m) + 2 * e) : make_double2(0.0, 0.0);
+      v[e] = live && n0 + 2 * e <= N ? coefficient(n0 + 2 * e) : make_double2(0.0, 0.0);
       mx = max(mx, max(dg_mag(v[e].x), dg_mag(v[e].y)));
     }
   }
@@ -470,7 +487,7 @@ dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const doub
     const int n0 = m + 16 * u + p;
     if (!keep) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = n0 + 2 * e <= N ? __ldg(src + (n0 - m) + 2 * e) : make_double2(0.0, 0.0);
+      for (int e = 0; e < 8; ++e) v[e] = n0 + 2 * e <= N ? coefficient(n0 + 2 * e) : make_double2(0.0, 0.0);
     }
     unsigned char *img = A + ((long long)ct * nchunk + mi.ch[p] + (u >> 2)) * DG_A_BYTES;
     unsigned long long q[8];
@@ -660,18 +677,19 @@ int build_digits(Plan &P) {
   return DCCM_OK;
 }
 
-template <int DIR> static int launch_kernel(const DgArgs &a, int items, cudaStream_t s) {
+template <int DIR, bool WA> static int launch_kernel(const DgArgs &a, int items, cudaStream_t s) {
   static bool attr_done = false;
   if (!attr_done) {
-    DCCM_CUDA(cudaFuncSetAttribute(legendre_dg_kernel<DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
+    DCCM_CUDA(cudaFuncSetAttribute(legendre_dg_kernel<DIR, WA>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
     attr_done = true;
   }
   const int ctas = sm_count();
-  DCCM_CUDA(launch_pdl(legendre_dg_kernel<DIR>, dim3(items < ctas ? items : ctas), dim3(DG_THREADS), (size_t)DG_SMEM, s, a));
+  DCCM_CUDA(launch_pdl(legendre_dg_kernel<DIR, WA>, dim3(items < ctas ? items : ctas), dim3(DG_THREADS), (size_t)DG_SMEM, s,
+                       a));
   return DCCM_OK;
 }
 
-static int launch_dg(Plan &P, int dir, int batch, int c0, int nct, double *out, cudaStream_t s) {
+static int launch_dg(Plan &P, int dir, int batch, int c0, int nct, double *out, bool wa, cudaStream_t s) {
   const DgTable &T = dir == 0 ? P.dinv : P.dfwd;
   DgArgs a;
   a.N = P.N;
@@ -695,31 +713,33 @@ static int launch_dg(Plan &P, int dir, int batch, int c0, int nct, double *out, 
   a.wait_ns = tunables().wait_limit_ms > 0 ? 1000000ull * (unsigned long long)tunables().wait_limit_ms : WAIT_LIMIT_NS;
   a.withhold = tunables().tc_withhold_loads;
   const int items = nct * T.nitems;
-  return dir == 0 ? launch_kernel<0>(a, items, s) : launch_kernel<1>(a, items, s);
+  if (dir == 0) return launch_kernel<0, false>(a, items, s);
+  return wa ? launch_kernel<1, true>(a, items, s) : launch_kernel<1, false>(a, items, s);
 }
 
-int legendre_inv_f64(Plan &P, int batch, const double *spec, double *F, cudaStream_t s) {
+int legendre_inv_f64(Plan &P, int batch, const double *spec, double *F, cudaStream_t s, bool wa) {
   const int nct = (2 * batch + 127) / 128;
   const DgMInfo *mi = (const DgMInfo *)P.dinv.d_mi;
   for (int t = 0; t < nct; t += P.dg_ct) {
     const int k = nct - t < P.dg_ct ? nct - t : P.dg_ct;
     const int b0 = 64 * t, nb = batch - b0 < 64 * k ? batch - b0 : 64 * k;
+    auto pack = [&](auto kernel, int g) {
+      return launch_pdl(kernel, dim3((nb + 256 / g - 1) / (256 / g), P.N + 1), dim3(256), 0, s, mi, P.N, (long long)P.ncoef,
+                        (const double2 *)spec, b0, nb, P.dinv.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea);
+    };
     // lanes a (m, field-level): 2 units of 8 for every 16 coefficients
-    if (P.N >= 64 && P.N < 128)
-      DCCM_CUDA(launch_pdl(dg_pack_spec<16>, dim3((nb + 15) / 16, P.N + 1), dim3(256), 0, s, mi, P.N, (long long)P.ncoef,
-                           (const double2 *)spec, b0, nb, P.dinv.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea));
-    else if (P.N < 128)
-      DCCM_CUDA(launch_pdl(dg_pack_spec<8>, dim3((nb + 31) / 32, P.N + 1), dim3(256), 0, s, mi, P.N, (long long)P.ncoef,
-                           (const double2 *)spec, b0, nb, P.dinv.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea));
+    if (wa)
+      DCCM_CUDA(P.N < 64 ? pack(dg_pack_spec<8, true>, 8) : P.N < 128 ? pack(dg_pack_spec<16, true>, 16)
+                                                                       : pack(dg_pack_spec<32, true>, 32));
     else
-      DCCM_CUDA(launch_pdl(dg_pack_spec<32>, dim3((nb + 7) / 8, P.N + 1), dim3(256), 0, s, mi, P.N, (long long)P.ncoef,
-                           (const double2 *)spec, b0, nb, P.dinv.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea));
-    DCCM_TRY(launch_dg(P, 0, batch, 128 * t, k, F, s));
+      DCCM_CUDA(P.N < 64 ? pack(dg_pack_spec<8, false>, 8) : P.N < 128 ? pack(dg_pack_spec<16, false>, 16)
+                                                                        : pack(dg_pack_spec<32, false>, 32));
+    DCCM_TRY(launch_dg(P, 0, batch, 128 * t, k, F, false, s));
   }
   return DCCM_OK;
 }
 
-int legendre_fwd_f64(Plan &P, int batch, const double *G, double *spec, cudaStream_t s) {
+int legendre_fwd_f64(Plan &P, int batch, const double *G, double *spec, cudaStream_t s, bool wa) {
   const int nct = (2 * batch + 127) / 128;
   const int nq = (P.Jh + DG_CHUNK - 1) / DG_CHUNK;
   const DgMInfo *mi = (const DgMInfo *)P.dfwd.d_mi;
@@ -733,7 +753,7 @@ int legendre_fwd_f64(Plan &P, int batch, const double *G, double *spec, cudaStre
     };
     DCCM_CUDA(nq <= 1 ? pack(dg_pack_four<1>, 1) : nq <= 2 ? pack(dg_pack_four<2>, 2)
               : nq <= 4 ? pack(dg_pack_four<4>, 4) : pack(dg_pack_four<8>, 8));
-    DCCM_TRY(launch_dg(P, 1, batch, c0, k, spec, s));
+    DCCM_TRY(launch_dg(P, 1, batch, c0, k, spec, wa, s));
   }
   return DCCM_OK;
 }

@@ -118,8 +118,9 @@ int fft_inverse_f64(const Plan &P, int batch, const double *F, double *grid, cud
 int fft_forward_f64(const Plan &P, int batch, const double *grid, double *G, cudaStream_t s);
 int fft_inverse(const Plan &P, int batch, bool fp32, const void *F, double *grid, cudaStream_t s);
 int fft_forward(const Plan &P, int batch, bool fp32, const double *grid, void *G, cudaStream_t s);
-int legendre_inv_f64(Plan &P, int batch, const double *spec, double *F, cudaStream_t s);
-int legendre_fwd_f64(Plan &P, int batch, const double *G, double *spec, cudaStream_t s);
+// wa: spectra in SPML's real layout (spml.cu)
+int legendre_inv_f64(Plan &P, int batch, const double *spec, double *F, cudaStream_t s, bool wa = false);
+int legendre_fwd_f64(Plan &P, int batch, const double *G, double *spec, cudaStream_t s, bool wa = false);
 int legendre_inv_tc(Plan &P, int batch, const double *spec, float *F, cudaStream_t s);
 int legendre_fwd_tc(Plan &P, int batch, const void *G3, double *spec, cudaStream_t s);
 int legendre_tc_multi(Plan *const *plans, const int *batch, const void *const *in, void *const *out,

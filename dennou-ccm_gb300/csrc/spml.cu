@@ -13,8 +13,9 @@
 // differ by a permutation alone (no scale, no sign).  Grids are the same
 // (0:im-1, 1:jm, k) arrays, latitudes south to north.
 //
-// The entry points permute on the device (one pass each way, gathers from
-// L2-resident tables) and call the plan's transforms; the plan keeps a
+// FP64 transforms of the smaller truncations read and write this layout
+// themselves.  The others permute on the device (one pass each way, gathers
+// from L2-resident tables) and call the plan's transforms; the plan keeps a
 // spectral buffer of max_batch field-levels for the native layout, set up by
 // the first call that needs it.
 #include <string.h>
@@ -116,6 +117,14 @@ int wa_from_spec(Plan &P, const double *spec, double *wa, int batch, cudaStream_
 }
 
 int xya_wa(Plan &P, const double *wa, double *xya, int batch, cudaStream_t s) {
+  // FP64: the operand pack gathers from this layout itself, but with 8 bytes
+  // of every sector at a time (us against the pass of its own: T21 x 16 12.6 and
+  // 16.5, T42 x 104 28.0 and 30.9, T85 x 8 28.7 and 32.9; x 128 64.3 and 63.7,
+  // T170 x 64 121 and 117, T341 x 8 190 and 179).
+  if (P.precision == DCCM_SHT_FP64 && P.N < 256 && (long long)(P.N + 1) * batch <= 8192) {
+    DCCM_TRY(legendre_inv_f64(P, batch, wa, (double *)P.d_work, s, true));
+    return fft_inverse(P, batch, false, P.d_work, xya, s);
+  }
   DCCM_TRY(wa_setup(P));
   double *spec = static_cast<double *>(P.wa_spec.ptr);
   DCCM_TRY(spec_from_wa(P, wa, spec, batch, s));
@@ -123,6 +132,13 @@ int xya_wa(Plan &P, const double *wa, double *xya, int batch, cudaStream_t s) {
 }
 
 int wa_xya(Plan &P, const double *xya, double *wa, int batch, cudaStream_t s) {
+  // FP64: the products' results go to their places in this layout (T21 x 16 13.3
+  // us, 16.6 with the pass of its own, T85 x 128 55.2 and 57.6, T170 x 64 112 and
+  // 115; T341 x 48 381 and 366).
+  if (P.precision == DCCM_SHT_FP64 && P.N < 256) {
+    DCCM_TRY(fft_forward(P, batch, false, xya, P.d_work, s));
+    return legendre_fwd_f64(P, batch, (const double *)P.d_work, wa, s, true);
+  }
   DCCM_TRY(wa_setup(P));
   double *spec = static_cast<double *>(P.wa_spec.ptr);
   DCCM_TRY(forward(P, xya, spec, batch, s));

@@ -233,16 +233,15 @@ __device__ __forceinline__ void warp_fft_fwd(float2 (&v)[R], const float2 *tw, c
 
 // Inverse (unnormalised) FFT of one row held as v[k1] = Z[k1 + R brev5(lane)];
 // on return v[r] = z[32 r + lane].
-template <int R>
+template <int R, bool PRE>
 __device__ __forceinline__ void warp_fft_inv(float2 (&v)[R], const float2 *tw, const float2 *twl,
-                                             const float2 (&w)[5], int lane) {
+                                             const float2 (&tl)[R], const float2 (&w)[5], int lane) {
   constexpr int I = 32 * R;
   lane_dit<R>(v, w, lane);
 #pragma unroll
   for (int k = 1; k < R; ++k) {
-    float2 t = __ldg(twl + k * 32 + lane);
-    t.y = -t.y;
-    v[k] = cmul(v[k], t);
+    const float2 t = PRE ? tl[k] : __ldg(twl + k * 32 + lane);
+    v[k] = cmul(v[k], make_float2(t.x, -t.y));
   }
   RegDft<R>::run(v, tw, I, +1);
 }
@@ -325,7 +324,7 @@ __device__ __forceinline__ void stage_z(const FftGroup &G, int jn, int js, int b
   }
 }
 
-template <int R>
+template <int R, bool PRE>
 __device__ __forceinline__ void fft_inv_block(const FftGroup &G, int jj, int by, float *st) {
   constexpr int I = 32 * R, ZB = zs_stride<R>();
   const int J = G.J, Jh = J / 2;
@@ -333,16 +332,26 @@ __device__ __forceinline__ void fft_inv_block(const FftGroup &G, int jj, int by,
   const int b0 = by * G.BB;
   const int nb = min(G.BB, G.batch - b0);
   float2 *zs = reinterpret_cast<float2 *>(st);
-  stage_z<R>(G, jn, js, b0, nb, zs);
-  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   float2 w[5];
-  lane_twiddles<R>(G.tw, lane, true, w);
+  float2 tl[R];
+  // PRE: both twiddles loaded with the staging's data, not after it (T85 x 128
+  // synthesis 28.1 -> 25.8 us, T127 x 64 29.9 -> 29.2).  Not where every length
+  // is compiled in (T21-T85 ensemble 807 -> 813 us) and not for rows over several
+  // warps (T341 x 192 522 -> 527).
+  if constexpr (PRE) {
+    lane_twiddles<R>(G.tw, lane, true, w);
+#pragma unroll
+    for (int k = 1; k < R; ++k) tl[k] = __ldg(G.twl + k * 32 + lane);
+  }
+  stage_z<R>(G, jn, js, b0, nb, zs);
+  __syncthreads();
+  if constexpr (!PRE) lane_twiddles<R>(G.tw, lane, true, w);
   for (int bl = warp; bl < nb; bl += nw) {
     float2 v[R];
 #pragma unroll
     for (int k1 = 0; k1 < R; ++k1) v[k1] = zs[bl * ZB + k1 * ZQ + lane];
-    warp_fft_inv<R>(v, G.tw, G.twl, w, lane);
+    warp_fft_inv<R, PRE>(v, G.tw, G.twl, tl, w, lane);
     double *gn = static_cast<double *>(G.out) + ((long long)(b0 + bl) * J + jn) * I;
     double *gs = static_cast<double *>(G.out) + ((long long)(b0 + bl) * J + js) * I;
 #pragma unroll
@@ -800,7 +809,7 @@ __device__ __forceinline__ void fft_fwd_block_mwp(const FftGroup &G, int jj, int
 // Several truncation groups in one launch: CTA blockIdx.x belongs to the
 // group whose block range contains it; the group's length selects the
 // register FFT (cases up to RMAX are compiled in).
-template <int R, int RMAX, bool FWD>
+template <int R, int RMAX, bool FWD, bool ONE>
 __device__ __forceinline__ void dispatch_case(const FftGroup &G, int jj, int by, float *st) {
   if constexpr (R <= RMAX) {
     if constexpr (R == 24) {
@@ -811,7 +820,7 @@ __device__ __forceinline__ void dispatch_case(const FftGroup &G, int jj, int by,
       else fft_inv_block_mwp<R / MW_R0>(G, jj, by, st);
     } else {
       if (FWD) fft_fwd_block<R>(G, jj, by, st);
-      else fft_inv_block<R>(G, jj, by, st);
+      else fft_inv_block<R, ONE>(G, jj, by, st);
     }
   }
 }
@@ -856,18 +865,18 @@ __global__ void __launch_bounds__(512, 2) fft_multi_kernel(const __grid_constant
     }
   }
   if constexpr (RFIX > 0) {
-    dispatch_case<RFIX, RMAX, FWD>(G, jj, by, st);
+    dispatch_case<RFIX, RMAX, FWD, true>(G, jj, by, st);
   } else {
     switch (G.R) {
-      case 2: dispatch_case<2, RMAX, FWD>(G, jj, by, st); break;
-      case 3: dispatch_case<3, RMAX, FWD>(G, jj, by, st); break;
-      case 4: dispatch_case<4, RMAX, FWD>(G, jj, by, st); break;
-      case 6: dispatch_case<6, RMAX, FWD>(G, jj, by, st); break;
-      case 8: dispatch_case<8, RMAX, FWD>(G, jj, by, st); break;
-      case 12: dispatch_case<12, RMAX, FWD>(G, jj, by, st); break;
-      case 16: dispatch_case<16, RMAX, FWD>(G, jj, by, st); break;
-      case 24: dispatch_case<24, RMAX, FWD>(G, jj, by, st); break;
-      case 32: dispatch_case<32, RMAX, FWD>(G, jj, by, st); break;
+      case 2: dispatch_case<2, RMAX, FWD, false>(G, jj, by, st); break;
+      case 3: dispatch_case<3, RMAX, FWD, false>(G, jj, by, st); break;
+      case 4: dispatch_case<4, RMAX, FWD, false>(G, jj, by, st); break;
+      case 6: dispatch_case<6, RMAX, FWD, false>(G, jj, by, st); break;
+      case 8: dispatch_case<8, RMAX, FWD, false>(G, jj, by, st); break;
+      case 12: dispatch_case<12, RMAX, FWD, false>(G, jj, by, st); break;
+      case 16: dispatch_case<16, RMAX, FWD, false>(G, jj, by, st); break;
+      case 24: dispatch_case<24, RMAX, FWD, false>(G, jj, by, st); break;
+      case 32: dispatch_case<32, RMAX, FWD, false>(G, jj, by, st); break;
       default: break;
     }
   }

@@ -448,21 +448,22 @@ template <int G, bool WA>
 __global__ void __launch_bounds__(256)
 dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const double2 *__restrict__ spec, int b0, int nb,
              int nchunk, unsigned char *__restrict__ A, int *__restrict__ ea, int ldea) {
+  const int m = blockIdx.y;
+  const int nq0 = mi_[m].nq[0], nq1 = mi_[m].nq[1], ch0 = mi_[m].ch[0], ch1 = mi_[m].ch[1];
+  asm volatile("" ::"r"(nq0 + nq1 + ch0 + ch1));  // plan constants: loaded before the wait
   pdl_wait();
   pdl_trigger();
-  const int m = blockIdx.y;
   const int gl = threadIdx.x % G;
   const int bl = blockIdx.x * (256 / G) + threadIdx.x / G;  // field-level of this launch
   const bool live = bl < nb;
   const int b = b0 + (live ? bl : 0);
-  const DgMInfo &mi = mi_[m];
   const double2 *src = spec + (long long)b * ncoef + idx_mn(N, m, m);
   const double *wa = reinterpret_cast<const double *>(spec) + (long long)b * (N + 1) * (N + 1);
   auto coefficient = [&](int n) {
     if constexpr (WA) return make_double2(__ldg(wa + wa_at(n, m, 0)), m ? __ldg(wa + wa_at(n, m, 1)) : 0.0);
     else return __ldg(src + (n - m));
   };
-  const int nu = 4 * max(mi.nq[0], mi.nq[1]);  // units of 8 a parity, both parities side by side
+  const int nu = 4 * max(nq0, nq1);  // units of 8 a parity, both parities side by side
   unsigned mx = 0;
   double2 v[8];
   for (int t = gl; t < 2 * nu; t += G) {
@@ -483,13 +484,13 @@ dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const doub
   const bool keep = 2 * nu <= G;  // the values are still in registers
   for (int t = gl; t < 2 * nu; t += G) {
     const int p = t & 1, u = t >> 1;
-    if (u >= 4 * mi.nq[p]) continue;
+    if (u >= 4 * (p ? nq1 : nq0)) continue;
     const int n0 = m + 16 * u + p;
     if (!keep) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = n0 + 2 * e <= N ? coefficient(n0 + 2 * e) : make_double2(0.0, 0.0);
     }
-    unsigned char *img = A + ((long long)ct * nchunk + mi.ch[p] + (u >> 2)) * DG_A_BYTES;
+    unsigned char *img = A + ((long long)ct * nchunk + (p ? ch1 : ch0) + (u >> 2)) * DG_A_BYTES;
     unsigned long long q[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) q[e] = dg_fixed(v[e].x, E);
@@ -509,16 +510,16 @@ __global__ void __launch_bounds__(256)
 dg_pack_four(const DgMInfo *__restrict__ mi_, int Jh, int C2B, int c0, int nc, const double *__restrict__ Gf, int nchunk,
              unsigned char *__restrict__ A, int *__restrict__ ea, int ldea, int guard) {
   __shared__ unsigned smx[8][8];
+  const int mp = blockIdx.y, m = mp >> 1, p = mp & 1;
+  const int nv = mi_[m].nv[p], nq = mi_[m].nq[p], ch = mi_[m].ch[p];
+  asm volatile("" ::"r"(nv + nq + ch));  // plan constants: loaded before the wait
   pdl_wait();
   pdl_trigger();
-  const int mp = blockIdx.y, m = mp >> 1, p = mp & 1;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int c8 = lane & 7, u = lane >> 3;
   const int cl = (blockIdx.x * (8 / WQ) + warp / WQ) * 8 + c8;
   const bool live = cl < nc;
-  const DgMInfo &mi = mi_[m];
-  if (mi.nv[p] <= 0) return;  // this parity has no coefficient (uniform over the block)
-  const int nq = mi.nq[p];
+  if (nv <= 0) return;  // this parity has no coefficient (uniform over the block)
   const double *src = Gf + (long long)mp * Jh * C2B + c0 + (live ? cl : 0);
   double v[8];
   unsigned mx = 0;
@@ -548,7 +549,7 @@ dg_pack_four(const DgMInfo *__restrict__ mi_, int Jh, int C2B, int c0, int nc, c
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = j0 + e < Jh ? __ldg(src + (long long)(j0 + e) * C2B) : 0.0;
     }
-    unsigned char *img = A + ((long long)ct * nchunk + mi.ch[p] + q) * DG_A_BYTES;
+    unsigned char *img = A + ((long long)ct * nchunk + ch + q) * DG_A_BYTES;
     unsigned long long qv[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) qv[e] = dg_fixed(v[e], E);

@@ -471,8 +471,6 @@ struct PackLaunch {
 };
 
 __global__ void __launch_bounds__(128) pack_spectra_kernel(const __grid_constant__ PackLaunch L) {
-  pdl_wait();  // Apack is read by the previous step's synthesis
-  pdl_trigger();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= L.total) return;
   int gi = 0;
@@ -484,8 +482,10 @@ __global__ void __launch_bounds__(128) pack_spectra_kernel(const __grid_constant
   const int b = (int)(u2 / (2 * G.nunits));
   const int r = (int)(u2 - (long long)b * 2 * G.nunits);
   const int p = r & 1;
-  const int4 w = __ldg(G.units + (r >> 1));
+  const int4 w = __ldg(G.units + (r >> 1));  // (a plan constant: loaded before the wait)
   const int m = w.x, n0 = m + 16 * w.y;
+  pdl_wait();  // Apack is read by the previous step's synthesis
+  pdl_trigger();
   // columns 8q .. 8q+7 of this parity hold at least one coefficient, else
   // the run lies past the segment (whose rounded length covers every run
   // that starts inside it) and is not written

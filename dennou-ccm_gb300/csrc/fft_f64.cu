@@ -485,19 +485,27 @@ static void octant(unsigned num, unsigned den, long long &c, long long &s) {
   c = (long long)((cs + 2) >> 2);
   s = (long long)((sn + 2) >> 2);
 }
-// e^{2 pi i t / I} times 2^62
-static void unit_root(int t, int I, long long &c, long long &s) {
-  const int o = 8 * t / I, r = 8 * t - o * I;  // octant, remainder in 1/I of it
-  long long a, b;
-  if (o & 1) octant((unsigned)(I - r), (unsigned)I, b, a);  // the octant's mirror image
-  else octant((unsigned)r, (unsigned)I, a, b);
-  switch (o / 2) {  // quadrant
-    case 0: c = a; s = b; break;
-    case 1: c = -b; s = a; break;
-    case 2: c = -a; s = -b; break;
-    default: c = b; s = -a; break;
+// e^{2 pi i t / I} times 2^62, from cos and sin of the first octant's I / 8 + 1
+// angles (I is a multiple of 32).
+struct Roots {
+  int I;
+  std::vector<long long> c, s;
+  explicit Roots(int n) : I(n), c(n / 8 + 1), s(n / 8 + 1) {
+    for (int k = 0; k <= n / 8; ++k) octant((unsigned)(8 * k), (unsigned)n, c[k], s[k]);
   }
-}
+  void get(int t, long long &x, long long &y) const {
+    const int o = 8 * t / I, r = t - o * (I / 8);  // octant, remainder in 1/I of the circle
+    long long a, b;
+    if (o & 1) b = c[I / 8 - r], a = s[I / 8 - r];  // the octant's mirror image
+    else a = c[r], b = s[r];
+    switch (o / 2) {  // quadrant
+      case 0: x = a; y = b; break;
+      case 1: x = -b; y = a; break;
+      case 2: x = -a; y = -b; break;
+      default: x = b; y = -a; break;
+    }
+  }
+};
 static int4 words(long long c, long long s) {
   auto hi = [](long long v) { return (int)((v + 0x80000000ll) >> 32); };
   auto lo = [](long long v) {
@@ -544,13 +552,14 @@ int build_fft_f64(Plan &P, std::vector<int4> &h) {
     using Sh = decltype(sh);
     h.assign(2 * Sh::TW + 1, int4());
     const bool three = Sh::I % 3 == 0;
+    const Roots roots(Sh::I);
     for (int dir = 0; dir < 2; ++dir) {
       int4 *w = h.data() + dir * Sh::TW;
       auto fill = [&](int R, int NS, int scale, bool th) {
         for (int p = 1; p < R; ++p)
           for (int k = 0; k < NS; ++k) {
             long long c, s;
-            unit_root(p * k, R * NS, c, s);  // p k < R NS
+            roots.get(p * k * (Sh::I / (R * NS)), c, s);  // p k < R NS
             if (dir == 0) *w++ = words(scaled(c, scale - 2, th), scaled(-s, scale - 2, th));
             else *w++ = words(c, s);
           }

@@ -5,7 +5,7 @@
 // (1.05 TFLOP/s measured), and the contraction took 80 % of the plain FP64
 // transforms as an FP64 FMA loop (T341 x 192 field-levels: synthesis 10.4
 // ms, analysis 13.5 ms; T85 x 128: 209 and 340 us; with the kernels below
-// 0.56, 0.63 ms, 36 and 35 us, packs included).  Here every operand is
+// 0.52, 0.61 ms, 32 and 31 us, packs included).  Here every operand is
 // split into seven 9-bit digits (digits.cuh: the scheme of K. Ozaki, T.
 // Ogita, S. Oishi, S. Rump, "Error-free transformations of matrix
 // multiplication", Numer. Algorithms 59 (2012), with integer digits), and
@@ -39,13 +39,18 @@
 // accumulators s = i + j: a slice of A is read from shared memory once for
 // all of them.
 //
-// What bounds it (T341 x 192, parts taken out one by one): the packs 140 and
-// 250 us (the analysis pack moves 1.5 GB), the MMAs alone 277 us against 140
-// at the peak rate (short N: 7 MMAs of 32 to 224 columns a K step), draining
-// about 60 and storing 50-100 us, mostly behind the MMAs.  TN = 64 (half the
-// reads of A, 193-227 us of MMAs, but one accumulator set, whose drains the
-// MMAs then wait for) came out at 591 and 644 us against 571 and 626, and
-// 16 % slower at T85.  Sixteen epilogue warps instead of eight: 776 -> 710 us.
+// What bounds it at T341 x 192: the packs take 100 and 240 us (the analysis
+// pack moves 1.5 GB), the rest is shared memory: a K step of 16 reads 28 KB of
+// A's slices and 28 KB of B's for its 7 MMAs of 32 to 224 columns and is
+// written 35 KB by the copies, 710 cycles at 128 bytes a cycle against 450 of
+// MMAs at the peak rate; clock stamps show the MMAs of two steps issued in
+// 1,360 cycles, and 2,000 with the drains beside them.  TN = 64 (half the
+// reads of A, but one accumulator set, whose drains the MMAs then wait for)
+// came out at 591 and 644 us against 571 and 626, and 16 % slower at T85.
+// Sixteen epilogue warps instead of eight: 776 -> 710 us.  At T85 and below an
+// item is latency: the loads 0.7 us, a chunk's MMAs 0.6, draining a set 0.8,
+// the results 2-3.  Digits made by the epilogue warps in the stages, without
+// the packs, were slower everywhere (T42 x 104 26.7 / 24.1 -> 30.6 / 26.5 us).
 //
 // A work item is (m, 128 columns c, TN rows of N).  Warp 0 copies, warp 1
 // allocates TMEM and issues the MMAs, warps 2-17 drain the accumulators
@@ -609,11 +614,12 @@ dg_build(int dir, int N, int Jh, const DgMInfo *__restrict__ mi_, const double *
 
 // ------------------------------------------------------------------ host
 
-static int build_dir(Plan &P, int dir, DgTable &T) {
+// One direction's metadata; tab: bytes of its tiles.
+static void plan_dir(const Plan &P, int dir, DgTable &T, std::vector<DgMInfo> &mi, std::vector<int2> &items,
+                     long long &tab) {
   const int N = P.N, Jh = P.Jh;
-  std::vector<DgMInfo> mi(N + 1);
-  std::vector<int2> items;
-  long long tab = 0;
+  mi.resize(N + 1);
+  tab = 0;
   int ch = 0;
   for (int m = 0; m <= N; ++m) {
     DgMInfo &M = mi[m];
@@ -638,33 +644,49 @@ static int build_dir(Plan &P, int dir, DgTable &T) {
   const int K = dir == 0 ? 2 * count_np(N, 0, 0) : Jh;
   while (K >> T.guard > 1024) ++T.guard;
   T.nitems = (int)items.size();
-  const long long nrows = dir == 0 ? (long long)(N + 1) * Jh : P.ncoef;
-  // one allocation a direction: metadata and items (one copy), row scales, tiles
-  const size_t mi_b = mi.size() * sizeof(DgMInfo), it_b = items.size() * sizeof(int2);
-  const size_t head = (mi_b + it_b + 255) / 256 * 256, eb_b = ((size_t)nrows * sizeof(short) + 255) / 256 * 256;
-  std::vector<unsigned char> h(head, 0);
-  memcpy(h.data(), mi.data(), mi_b);
-  memcpy(h.data() + mi_b, items.data(), it_b);
-  DCCM_CUDA(cudaMalloc(&T.d_mem, head + eb_b + (size_t)tab));
-  DCCM_CUDA(cudaMemcpy(T.d_mem, h.data(), head, cudaMemcpyHostToDevice));
-  unsigned char *base = (unsigned char *)T.d_mem;
-  T.d_mi = base;
-  T.d_items = (int2 *)(base + mi_b);
-  T.d_eb = (short *)(base + head);
-  T.d_tab = base + head + eb_b;
-  dg_row_scale<<<(unsigned)((nrows + 7) / 8), 256>>>(dir, N, Jh, P.d_pnm, P.d_w, nrows, T.d_eb);
-  DCCM_LAUNCH_CHECK();
-  dg_build<<<dim3(16, N + 1, 2), 256>>>(dir, N, Jh, (const DgMInfo *)T.d_mi, P.d_pnm, P.d_w, T.d_eb,
-                                        (unsigned char *)T.d_tab);
-  DCCM_LAUNCH_CHECK();
-  return DCCM_OK;
 }
 
 // Tables of both directions and the A images.  The images of one launch are
 // bounded (DG_WORK_CAP); a larger batch takes several launches.
 int build_digits(Plan &P) {
-  DCCM_TRY(build_dir(P, 0, P.dinv));
-  DCCM_TRY(build_dir(P, 1, P.dfwd));
+  DgTable *T[2] = {&P.dinv, &P.dfwd};
+  std::vector<DgMInfo> mi[2];
+  std::vector<int2> items[2];
+  long long tab[2];
+  // one allocation: metadata and items of both directions (one copy), row
+  // scales, tiles
+  auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  const long long nrows[2] = {(long long)(P.N + 1) * P.Jh, (long long)P.ncoef};
+  size_t at_mi[2], at_it[2], at_eb[2], at_tab[2], at = 0;
+  for (int d = 0; d < 2; ++d) {
+    plan_dir(P, d, *T[d], mi[d], items[d], tab[d]);
+    at_mi[d] = at;
+    at_it[d] = at + mi[d].size() * sizeof(DgMInfo);
+    at = up(at_it[d] + items[d].size() * sizeof(int2));
+  }
+  std::vector<unsigned char> &h = P.h_dg;
+  h.assign(at, 0);
+  for (int d = 0; d < 2; ++d) {
+    memcpy(h.data() + at_mi[d], mi[d].data(), mi[d].size() * sizeof(DgMInfo));
+    memcpy(h.data() + at_it[d], items[d].data(), items[d].size() * sizeof(int2));
+    at_eb[d] = at;
+    at_tab[d] = at + up((size_t)nrows[d] * sizeof(short));
+    at = up(at_tab[d] + (size_t)tab[d]);
+  }
+  DCCM_CUDA(cudaMalloc(&P.d_dgmem, at));
+  unsigned char *base = (unsigned char *)P.d_dgmem;
+  DCCM_CUDA(cudaMemcpyAsync(base, h.data(), h.size(), cudaMemcpyHostToDevice));
+  for (int d = 0; d < 2; ++d) {
+    T[d]->d_mi = base + at_mi[d];
+    T[d]->d_items = (int2 *)(base + at_it[d]);
+    T[d]->d_eb = (short *)(base + at_eb[d]);
+    T[d]->d_tab = base + at_tab[d];
+    dg_row_scale<<<(unsigned)((nrows[d] + 7) / 8), 256>>>(d, P.N, P.Jh, P.d_pnm, P.d_w, nrows[d], T[d]->d_eb);
+    DCCM_LAUNCH_CHECK();
+    dg_build<<<dim3(16, P.N + 1, 2), 256>>>(d, P.N, P.Jh, (const DgMInfo *)T[d]->d_mi, P.d_pnm, P.d_w, T[d]->d_eb,
+                                            (unsigned char *)T[d]->d_tab);
+    DCCM_LAUNCH_CHECK();
+  }
   const int nch = P.dinv.nchunk > P.dfwd.nchunk ? P.dinv.nchunk : P.dfwd.nchunk;
   const size_t per = (size_t)nch * DG_A_BYTES;
   const int nct = (2 * P.max_batch + 127) / 128;

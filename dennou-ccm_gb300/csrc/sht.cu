@@ -93,10 +93,10 @@ __global__ void pnm_kernel(int N, int Jh, const double *__restrict__ mu, double 
 }
 
 static void destroy(Plan &P) {
-  void *ptrs[] = {P.d_mu,      P.d_w,        P.d_pnm,       P.d_twfx,  P.d_tw32,  P.d_twl32,
+  void *ptrs[] = {P.d_mu,      P.d_pnm,      P.d_twfx,  P.d_tw32,  P.d_twl32,
                   P.tinv.d,    P.tfwd.d,     P.tinv.d_mi,   P.tfwd.d_mi, P.tinv.d_items,
-                  P.tfwd.d_items, P.d_work,  P.d_err,       P.d_apack, P.d_punits, P.d_cexp,
-                  P.d_wa_pos, P.d_wa_src, P.d_dig,     P.dinv.d_mem, P.dfwd.d_mem};
+                  P.tfwd.d_items, P.d_work,  P.d_apack, P.d_punits, P.d_cexp,
+                  P.d_wa_pos, P.d_wa_src, P.d_dig,     P.d_dgmem};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   P.stage.release();
@@ -115,26 +115,23 @@ static int create(Plan &P, int N, int I, int J, int precision, int max_batch) {
   P.max_batch = max_batch;
   P.ncoef = (int64_t)(N + 1) * (N + 2) / 2;
   if (!fft_length_supported(I)) return DCCM_ERR_UNSUPPORTED;
-  DCCM_CUDA(cudaMalloc(&P.d_mu, J * sizeof(double)));
-  DCCM_CUDA(cudaMalloc(&P.d_w, J * sizeof(double)));
+  DCCM_CUDA(cudaMalloc(&P.d_mu, (2 * J + 1) * sizeof(double)));  // nodes, weights, error flag
+  P.d_w = P.d_mu + J;
+  P.d_err = (int *)(P.d_mu + 2 * J);
   DCCM_CUDA(cudaMalloc(&P.d_pnm, (size_t)P.ncoef * P.Jh * sizeof(double)));
-  DCCM_CUDA(cudaMalloc(&P.d_err, sizeof(int)));
   DCCM_CUDA(cudaMemset(P.d_err, 0, sizeof(int)));
   gauss_newton_kernel<<<(P.Jh + 127) / 128, 128>>>(J, P.d_mu, P.d_w);
   DCCM_LAUNCH_CHECK();
   const long long nt = (long long)(N + 1) * P.Jh;
   pnm_kernel<<<(unsigned)((nt + 127) / 128), 128>>>(N, P.Jh, P.d_mu, P.d_pnm);
   DCCM_LAUNCH_CHECK();
-  P.mu.resize(J);
-  P.w.resize(J);
-  DCCM_CUDA(cudaMemcpy(P.mu.data(), P.d_mu, J * sizeof(double), cudaMemcpyDeviceToHost));
-  DCCM_CUDA(cudaMemcpy(P.w.data(), P.d_w, J * sizeof(double), cudaMemcpyDeviceToHost));
+  // (the host's part of the tables is made while these run)
   if (precision == DCCM_SHT_FP64) {
-    std::vector<int4> tw;
+    std::vector<int4> &tw = P.h_tw;
     DCCM_TRY(build_fft_f64(P, tw));
     P.twfx0 = tw.back();
     DCCM_CUDA(cudaMalloc(&P.d_twfx, tw.size() * sizeof(int4)));
-    DCCM_CUDA(cudaMemcpy(P.d_twfx, tw.data(), tw.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    DCCM_CUDA(cudaMemcpyAsync(P.d_twfx, tw.data(), tw.size() * sizeof(int4), cudaMemcpyHostToDevice));
   } else {
     // FFT twiddles e^{-2 pi i t / I} and the per-lane table e^{-2 pi i l k / I}
     // at [k][l] (l < 32, k < I/32), rounded from FP64.
@@ -166,7 +163,13 @@ static int create(Plan &P, int N, int I, int J, int precision, int max_batch) {
   if (precision == DCCM_SHT_MIXED_FP16) DCCM_CUDA(cudaMalloc(&P.d_cexp, 2 * (size_t)max_batch * sizeof(int)));
   if (precision != DCCM_SHT_FP64) DCCM_TRY(build_tiles(P));
   else DCCM_TRY(build_digits(P));
+  std::vector<double> mw(2 * J);
+  DCCM_CUDA(cudaMemcpy(mw.data(), P.d_mu, 2 * J * sizeof(double), cudaMemcpyDeviceToHost));
+  P.mu.assign(mw.begin(), mw.begin() + J);
+  P.w.assign(mw.begin() + J, mw.end());
   DCCM_CUDA(cudaDeviceSynchronize());
+  std::vector<int4>().swap(P.h_tw);
+  std::vector<unsigned char>().swap(P.h_dg);
   return DCCM_OK;
 }
 

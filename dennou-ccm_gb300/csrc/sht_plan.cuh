@@ -53,7 +53,7 @@ struct TileTable {
 
 // FP64 path: one direction's digit tables (legendre_dg.cu).
 struct DgTable {
-  void *d_mem = nullptr;      // the allocation that holds the four arrays below
+  // (the four arrays lie in Plan::d_dgmem)
   void *d_mi = nullptr;       // per-m tile metadata
   int2 *d_items = nullptr;    // work items (m, nt) of one 128-column tile
   short *d_eb = nullptr;      // scale exponent of every table row
@@ -70,6 +70,9 @@ struct Plan {
   int64_t ncoef = 0;
   // host copies of the axes
   std::vector<double> mu, w;
+  // FP64 path, during creation: sources of copies that may be in flight
+  std::vector<int4> h_tw;
+  std::vector<unsigned char> h_dg;
   // device
   double *d_mu = nullptr, *d_w = nullptr;
   double *d_pnm = nullptr;     // FP64 Pbar(m, n, jj): [idx(m,n)][Jh]
@@ -90,6 +93,7 @@ struct Plan {
   int nsplit = 3;              // tensor-path operand splits: 3 (BF16 x 3) or 2 (FP16 hi + lo)
   int *d_cexp = nullptr;       // FP16: per field-level scale exponents, [inverse | forward][max_batch]
   DgTable dinv, dfwd;          // FP64 path: digit tables
+  void *d_dgmem = nullptr;     // and the allocation that holds both
   void *d_dig = nullptr;       // FP64 path: A operand images of up to dg_ct column tiles
   int *d_ea = nullptr;         // FP64 path: scale exponents of the A operand, rows of dg_ldea (in d_dig)
   int dg_ct = 0, dg_ldea = 0;

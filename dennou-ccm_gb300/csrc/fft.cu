@@ -373,7 +373,8 @@ template <int R> __device__ __forceinline__ float2 *eo_plane(float *st, int BB, 
 // Split the staged E/O values into G3[s][(2m + p) Jh + jj][2 b0 + c], c =
 // 2 bl + re/im.  A thread item is (m, p, FL consecutive field-levels): FL
 // float2 reads and one store of 2 FL bf16 per plane (16, 8 or 4 bytes: the
-// run starts at 2 b0 + 2 FL q in a row of C2Bp, a multiple of 8).  Values
+// run starts at 2 b0 + 2 FL q in a row of C2Bp, a multiple of 8, so the last
+// one may reach past the batch: zeros there, which no item reads).  Values
 // are split two at a time (packed conversions round each half as the
 // scalar ones do).
 template <int R, int FL>
@@ -390,8 +391,12 @@ __device__ __forceinline__ void write_g3_fl(const FftGroup &G, int jj, int b0, i
     float2 v[FL];
 #pragma unroll
     for (int i = 0; i < FL; ++i) v[i] = eo_plane<R>(st, BB, p, f0 + i)[sl];
+    if (f0 + FL > nb) {
+#pragma unroll
+      for (int i = 0; i < FL; ++i)
+        if (f0 + i >= nb) v[i] = make_float2(0.f, 0.f);
+    }
     unsigned short *o = G3 + ((size_t)(2 * m + p) * Jh + jj) * G.C2Bp + 2 * (b0 + f0);
-    const bool full = f0 + FL <= nb;
     unsigned w[3][FL];
     if (G.nsplit == 2) {
 #pragma unroll
@@ -404,24 +409,13 @@ __device__ __forceinline__ void write_g3_fl(const FftGroup &G, int jj, int b0, i
       for (int i = 0; i < FL; ++i) split3f_x2(v[i], w[0][i], w[1][i], w[2][i]);
     }
     const int ns = G.nsplit;
-    if (full) {
 #pragma unroll
-      for (int s3 = 0; s3 < 3; ++s3) {
-        if (s3 >= ns) break;
-        unsigned short *os = o + s3 * plane;
-        if constexpr (FL == 4) *reinterpret_cast<uint4 *>(os) = make_uint4(w[s3][0], w[s3][1], w[s3][2], w[s3][3]);
-        else if constexpr (FL == 2) *reinterpret_cast<uint2 *>(os) = make_uint2(w[s3][0], w[s3][1]);
-        else *reinterpret_cast<unsigned *>(os) = w[s3][0];
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < FL; ++i)
-#pragma unroll
-        for (int s3 = 0; s3 < 3; ++s3)
-          if (f0 + i < nb && s3 < ns) {
-            o[s3 * plane + 2 * i] = (unsigned short)w[s3][i];
-            o[s3 * plane + 2 * i + 1] = (unsigned short)(w[s3][i] >> 16);
-          }
+    for (int s3 = 0; s3 < 3; ++s3) {
+      if (s3 >= ns) break;
+      unsigned short *os = o + s3 * plane;
+      if constexpr (FL == 4) *reinterpret_cast<uint4 *>(os) = make_uint4(w[s3][0], w[s3][1], w[s3][2], w[s3][3]);
+      else if constexpr (FL == 2) *reinterpret_cast<uint2 *>(os) = make_uint2(w[s3][0], w[s3][1]);
+      else *reinterpret_cast<unsigned *>(os) = w[s3][0];
     }
   }
 }
@@ -928,8 +922,17 @@ int fft_multi(Plan *const *plans, const int *batch, const void *const *in, void 
   // 15.8 / 15.6 and 14.3 / 13.0, T127 x 60 33.9 / 35.0 and 30.1 / 31.3), 40
   // for rows over four warps, whose CTAs are larger (T341 x 8 74 / 77 and
   // 79 / 82 us, x 192 530 / 580 and 602 / 685; x 4 70 / 74 and 66 / 70).
-  const int WPC = (tb == 4 || tb == 8 || tb == 16) ? tb : (wmin >= 3 ? 16 : 8);
   const int rpw = tr == 1 || tr == 2 ? tr : (wt >= (wmin == 4 ? 40LL : 60LL) * sm_count() ? 2 : 1);
+  int wpc = wmin >= 3 ? 16 : 8;
+  if (wmin >= 3 && ngroups == 1) {
+    // not where the wider CTAs leave a quarter of their row pairs empty (T341 x 9
+    // 85 / 97 us with 16 warps, 78 / 95 with 8; x 5 70 / 80 and 68 / 79; T255 x 5
+    // 43 / 40 and 41 / 37), unless one holds the batch
+    const int bb16 = wmin == 4 ? 4 * rpw : 4, bb8 = bb16 / 2, b = batch[0];
+    const int s16 = (b + bb16 - 1) / bb16 * bb16, s8 = (b + bb8 - 1) / bb8 * bb8;
+    if (b > bb16 && 4 * s16 >= 5 * s8) wpc = 8;
+  }
+  const int WPC = (tb == 4 || tb == 8 || tb == 16) ? tb : wpc;
   FftLaunch L;
   memset(&L, 0, sizeof L);
   int nblk = 0, ng = 0;
@@ -938,7 +941,9 @@ int fft_multi(Plan *const *plans, const int *batch, const void *const *in, void 
     if (batch[g] <= 0) continue;
     const Plan &P = *plans[g];
     const int R = P.I / 32, W = fft_warps_per_row(R);
-    const int rp = W == 3 ? 1 : rpw;
+    // FP16 rows of 12 samples a lane lose by two (T127 x 505 analysis 216 -> 228
+    // us; BF16 x 3 181 -> 172)
+    const int rp = W == 3 || (tr == 0 && fwd && P.nsplit == 2 && R == 12) ? 1 : rpw;
     int BB = 1;
     while (2 * BB * W <= WPC * rp && fft_smem(R, 2 * BB, WPC / W) <= budget) BB *= 2;
     int lbb = 0;

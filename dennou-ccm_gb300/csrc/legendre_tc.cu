@@ -281,27 +281,39 @@ legendre_tc_kernel(const __grid_constant__ TcLaunch L) {
             tc_fence_after();
             const uint32_t As = smem_u32(stage + s * STAGE_BYTES);
             const int ksteps = min(4, (kv - q * 64 + 15) / 16);
-            // Descriptors by constant offsets (16-byte units) from the
-            // stage's two: a K step of 16 is 32 bytes along a K-major row, 16
-            // rows of an MN-major tile.  (A split, B split) of the cross
-            // terms: BF16 x 3 hi*mid, mid*hi, hi*lo, lo*hi, mid*mid; FP16
-            // hi + lo: hi*lo, lo*hi.
-            uint64_t da = smem_desc(As, amn ? 8192 : 16), db = smem_desc(As + 3 * A_SPLIT_BYTES, 16);
-            const uint64_t ka = amn ? 2048 >> 4 : 32 >> 4;
-            constexpr uint64_t A1 = A_SPLIT_BYTES >> 4, B1 = B_SPLIT_BYTES >> 4;
-            for (int ks = 0; ks < ksteps; ++ks) {
-              mma_bf16(dmain, da, db, idesc, accm);
-              accm = 1;
-              mma_bf16(dcross, da, db + B1, idesc, accx);
-              accx = 1;
-              mma_bf16(dcross, da + A1, db, idesc, 1);
-              if (a.nsplit == 3) {
+            // A K step of 16: 32 bytes along a K-major row, 16 rows of an
+            // MN-major tile.  (A split, B split) of the cross terms: BF16 x 3
+            // hi*mid, mid*hi, hi*lo, lo*hi, mid*mid; FP16 hi + lo: hi*lo, lo*hi.
+            const uint32_t lbo = amn ? 8192 : 16;
+            if (a.nsplit == 3) {
+              // descriptors by constant offsets (16-byte units) from the stage's two
+              uint64_t da = smem_desc(As, lbo), db = smem_desc(As + 3 * A_SPLIT_BYTES, 16);
+              const uint64_t ka = amn ? 2048 >> 4 : 32 >> 4;
+              constexpr uint64_t A1 = A_SPLIT_BYTES >> 4, B1 = B_SPLIT_BYTES >> 4;
+              for (int ks = 0; ks < ksteps; ++ks) {
+                mma_bf16(dmain, da, db, idesc, accm);
+                accm = 1;
+                mma_bf16(dcross, da, db + B1, idesc, accx);
+                accx = 1;
+                mma_bf16(dcross, da + A1, db, idesc, 1);
                 mma_bf16(dcross, da, db + 2 * B1, idesc, 1);
                 mma_bf16(dcross, da + 2 * A1, db, idesc, 1);
                 mma_bf16(dcross, da + A1, db + B1, idesc, 1);
+                da += ka;
+                db += 32 >> 4;
               }
-              da += ka;
-              db += 32 >> 4;
+            } else {
+              // half the MMAs: issued at that pace they hold up the loads (T341 x
+              // 1 analysis 54 us, 46 with every descriptor built anew)
+              const uint32_t Bs = As + 3 * A_SPLIT_BYTES;
+              for (int ks = 0; ks < ksteps; ++ks) {
+                const uint32_t ka = amn ? ks * 2048 : ks * 32, kb = ks * 32;
+                mma_bf16(dmain, smem_desc(As + ka, lbo), smem_desc(Bs + kb, 16), idesc, accm);
+                accm = 1;
+                mma_bf16(dcross, smem_desc(As + ka, lbo), smem_desc(Bs + B_SPLIT_BYTES + kb, 16), idesc, accx);
+                accx = 1;
+                mma_bf16(dcross, smem_desc(As + A_SPLIT_BYTES + ka, lbo), smem_desc(Bs + kb, 16), idesc, 1);
+              }
             }
             mma_commit(&empty[s]);
           }

@@ -539,8 +539,9 @@ def roofline(S, inp, groups, stage_ms, workload, fp64_peak, flux_alone=None, pro
     also report their tensor rate against the BF16 peak divided by the
     products per multiply-add (6 for BF16 x 3, 3 for FP16 hi + lo), with
     the raw fraction of the BF16 peak beside it.  The flux kernel, bound by
-    the FP64 pipe, reports its FP64 instruction rate (ncu counts per
-    column) over the measured FP64 peak.  flux_alone: the flux kernel timed
+    the FP64 and integer pipes together, reports the rate of the FP64
+    instructions it executes (ncu counts per column) over the measured FP64
+    peak, and beside it the FP64 work of the plain formulation.  flux_alone: the flux kernel timed
     alone on its full grid when the step caps its grid; its roofline is then
     taken from that time (the step's time and cap are kept beside it)."""
     hbm, bf16, src_peak = peaks()
@@ -563,18 +564,19 @@ def roofline(S, inp, groups, stage_ms, workload, fp64_peak, flux_alone=None, pro
                             "products_per_mac": products, "raw_peak": bf16, "raw_frac": tf / bf16,
                             "algorithmic_flops": fl}
         stages[n] = st
-    stages["bulk_flux"]["limiter"] = "FP64 pipe, not HBM"
+    stages["bulk_flux"]["limiter"] = "FP64 and integer pipes, not HBM"
     if flux_alone:
         stages["bulk_flux"]["launch"] = ("full grid, timed alone; in the step its grid is capped at %d CTAs "
                                          "(%.4f ms there)" % (flux_alone["step_cta_cap"], flux_alone["ms_in_step"]))
-    f64 = FLUX_FP64_INSTR_PER_COLUMN * S["ncol"]
+    f64 = FLUX_FP64_EXECUTED_FLOPS_PER_COLUMN * S["ncol"]
     tf = f64 / (stages["bulk_flux"]["ms"] / 1e3) / 1e12
     stages["bulk_flux"]["fp64"] = {"achieved": tf, "unit": "TFLOP/s", "peak": fp64_peak,
                                    "peak_source": "measured (dccm_fp64_peak)", "frac": tf / fp64_peak,
                                    "flops_per_launch": f64,
-                                   "count": "FP64 pipe work per column from ncu instruction counts (DADD + DMUL "
+                                   "plain_formulation_flops": FLUX_FP64_INSTR_PER_COLUMN * S["ncol"],
+                                   "count": "FP64 instructions executed per column from ncu counts (DADD + DMUL "
                                             "+ 2 DFMA), the same for every ice-free column",
-                                   "pipe": fp64_pipe(FLUX_FP64_PIPE_OPS_PER_COLUMN * S["ncol"],
+                                   "pipe": fp64_pipe(FLUX_FP64_EXECUTED_OPS_PER_COLUMN * S["ncol"],
                                                      stages["bulk_flux"]["ms"], fp64_peak)}
     # the remap keeps the reference's separately rounded products and sums
     # (bit-exact): one DMUL per table entry and field, and one DADD per
@@ -604,7 +606,9 @@ def roofline(S, inp, groups, stage_ms, workload, fp64_peak, flux_alone=None, pro
 
 def roofline_f64(groups, stage_ms, fp64_peak):
     """Stage rooflines of the FP64 step (the denominator of mixed / FP64):
-    FP64 flops over the measured FP64 peak, bytes over the copy bandwidth."""
+    the algorithm's FP64 flops over the measured FP64 peak (above 1: the
+    contractions run on the tensor cores as products of integer digits, the
+    FFTs in 64-bit fixed point), bytes over the copy bandwidth."""
     hbm, _, _ = peaks()
     work = stage_work_f64(groups)
     names = dccm_stages()
@@ -620,23 +624,24 @@ def roofline_f64(groups, stage_ms, fp64_peak):
     return out
 
 
-# FP64 pipe work of the flux kernel per ocean column: DADD + DMUL + 2 DFMA
-# thread instructions (ncu sass counters, c3, 45,478 columns: 1,182,428
-# DADD, 3,137,982 DMUL, 5,002,580 DFMA; the reciprocals, square roots, exp
-# and log are the kernel's own, csrc/fp64_fast.cuh).  Every column does the
-# same work when there is no sea ice (all workloads here: warps whose
-# columns all have SIceCon = 0 skip the ice physics and the merging), so
-# the per-column figure carries to every workload.
+# FP64 work of the bulk flux per ocean column in a plain FP64 formulation:
+# DADD + DMUL + 2 DFMA thread instructions (ncu sass counters of such a
+# kernel, c3, 45,478 columns: 1,182,428 DADD, 3,137,982 DMUL, 5,002,580
+# DFMA), and the same counts as FP64 pipe operations (one issue slot each).
 FLUX_FP64_INSTR_PER_COLUMN = (1182428 + 3137982 + 2 * 5002580) / 45478
-# the same counts as FP64 pipe operations (one issue slot each)
 FLUX_FP64_PIPE_OPS_PER_COLUMN = (1182428 + 3137982 + 5002580) / 45478
+# What the kernel leaves to the FP64 pipe (its reciprocals, square roots,
+# exp, log and the products around them run on the integer pipes; counters
+# of a launch of 1,036,800 ice-free columns): 13 DADD, 13 DMUL, 10 DFMA.
+FLUX_FP64_EXECUTED_OPS_PER_COLUMN = 36.0
+FLUX_FP64_EXECUTED_FLOPS_PER_COLUMN = 46.0
 
 
-# FP64 flops of the implicit-coupling sweeps per column and level, one
-# tracer (DADD + DMUL + 2 DFMA thread instructions, ncu sass counters,
-# 32768 columns x 32 levels): per 32-level column forward 3163 (shared
-# factors 502 + elimination 2661), backward 1058.
-IMPLCPL_FP64_FLOPS = {"forward": 3163 / 32, "backward": 1058 / 32}
+# FP64 flops that the implicit-coupling sweeps leave to the FP64 pipe, per
+# column and level, one tracer (DADD + DMUL + 2 DFMA thread instructions,
+# ncu sass counters, 32768 columns x 32 levels): per 32-level column forward
+# 757 (shared factors 95 + elimination 662), backward 248.
+IMPLCPL_FP64_FLOPS = {"forward": 757 / 32, "backward": 248 / 32}
 
 
 def dccm_stages():
@@ -999,7 +1004,8 @@ def implcpl_leg(args, groups, dccm, synth, torch, dev, stream, flush, fp64_peak)
     tracer), reported beside the step: forward sweep (ImplCplCoef1/2 for the
     bulk flux) and backward sweep, CUDA events, L2 flushed between runs.
     Algorithmic bytes: 12 input profiles and 4 outputs of kmax+1 levels, the
-    module-state matrices written and read back (3 x 3 x kmax), FP64."""
+    diagonals of the module-state matrices written and read back (3 x kmax;
+    the other two diagonals are constants), FP64."""
     g = max(groups, key=lambda q: q.I * q.J)
     ncol, kmax = g.I * g.J, max(2, g.nfl // 4 if len(groups) == 1 else 32)
     d = synth.column_profiles(ncol, kmax, ncmax=1, seed=7)
@@ -1025,8 +1031,8 @@ def implcpl_leg(args, groups, dccm, synth, torch, dev, stream, flush, fp64_peak)
             tf.append(e[0].elapsed_time(e[1]))
             tb.append(e[1].elapsed_time(e[2]))
     hbm, _, _ = peaks()
-    fwd_bytes = ncol * 8 * ((kmax + 1) * (9 + 1) + kmax * 2 + kmax * 4 + 8 + 3 * 3 * kmax)
-    bwd_bytes = ncol * 8 * (2 * 4 * kmax + 3 * 2 * kmax)
+    fwd_bytes = ncol * 8 * ((kmax + 1) * (9 + 1) + kmax * 2 + kmax * 4 + 8 + 3 * kmax)
+    bwd_bytes = ncol * 8 * (2 * 4 * kmax + 3 * kmax)
     f, b = float(np.mean(tf)), float(np.mean(tb))
 
     def fp64(key, ms):
@@ -1039,7 +1045,7 @@ def implcpl_leg(args, groups, dccm, synth, torch, dev, stream, flush, fp64_peak)
             "columns_per_s": ncol / ((f + b) / 1e3),
             "forward_roofline": {"bound": "hbm", "algorithmic_bytes": fwd_bytes,
                                  "achieved": fwd_bytes / (f / 1e3) / 1e9, "unit": "GB/s", "peak": hbm,
-                                 "frac": fwd_bytes / (f / 1e3) / 1e9 / hbm, "limiter": "FP64 pipe, not HBM",
+                                 "frac": fwd_bytes / (f / 1e3) / 1e9 / hbm, "limiter": "FP64 and integer pipes, not HBM",
                                  "fp64": fp64("forward", f)},
             "backward_roofline": {"bound": "hbm", "algorithmic_bytes": bwd_bytes,
                                   "achieved": bwd_bytes / (b / 1e3) / 1e9, "unit": "GB/s", "peak": hbm,

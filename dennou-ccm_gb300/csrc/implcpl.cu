@@ -85,8 +85,9 @@ struct Fwd {
 // their use (five CTAs an SM at 102 registers or four at 128).  The backward
 // sweep fetches LVB ahead in the same way (FP64 pipe 66 % busy; with eight
 // unrolled and one copy of the code for each matrix a quarter of its cycles
-// waited for instructions: 131,072 x 48 172 -> 150 us); its CTAs are of 64
-// threads, so that its three kinds of block spread evenly (32,768 x 32 35 -> 33).
+// waited for instructions: 131,072 x 48 172 -> 150 us); its CTAs are single
+// warps, so that its three kinds of block spread evenly (32,768 x 32 35 us with
+// 128 threads, 33 with 64, 31 with 32; 2,048 x 16 10.3 and 8.3).
 constexpr int GL = 2;   // levels a thread of geo_kernel
 constexpr int LVB = 2;  // backward sweep: levels fetched ahead
 
@@ -399,7 +400,7 @@ __device__ __forceinline__ void backward_chains(const double *__restrict__ mat, 
   }
 }
 
-__global__ void __launch_bounds__(64, 16) backward_kernel(const Bwd a) {
+__global__ void __launch_bounds__(32, 32) backward_kernel(const Bwd a) {
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= a.ncol) return;
   const long long n = a.ncol;
@@ -527,7 +528,7 @@ extern "C" int dccm_implcpl_backward_dev(dccm_implcpl *p, double *xyz_DUDt, doub
   b.inv_2dt = 1.0 / (2.0 * p->k.DelTime);
   // an exponent that sends every product to the FP64 form where 1 / (2 dt) is not ordinary
   b.u2dt = ordinary(b.inv_2dt) ? fx::uf(b.inv_2dt) : fx::UF{0, 0};
-  const int threads = 64;
+  const int threads = 32;
   implcpl::backward_kernel<<<dim3((unsigned)((p->ncol + threads - 1) / threads), 3), threads, 0,
                              as_stream(stream)>>>(b);
   DCCM_LAUNCH_CHECK();

@@ -34,9 +34,9 @@
 // sums start at zero and add the separately rounded products in table
 // order, which makes the result bit-identical to the reference loop
 // (:293-302); the first addition of a row, 0 + p, is p with -0 turned into
-// +0, which integer instructions give exactly without the FP64 pipe (the
-// pipe the kernel is bound by: one DMUL per entry and field, one DADD per
-// entry after the first).
+// +0, which integer instructions give exactly, and two of three products are
+// rounded on the integer pipes too (product below): the FP64 pipe does a DMUL
+// for the third and a DADD per entry after a row's first.
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -67,6 +67,55 @@ namespace remap {
 constexpr int UNSET = -2147483647;
 
 // ---------------------------------------------------------------- apply
+// A weight unpacked for mul_rn: mantissa at the top of 64 bits, exponent field
+// less the bias, sign bit.
+struct Weight {
+  unsigned h, l, sign;
+  int e;
+  double v;
+  __device__ __forceinline__ explicit Weight(double w) : v(w) {
+    const unsigned hi = (unsigned)__double2hiint(w), lo = (unsigned)__double2loint(w);
+    const int ef = (int)(hi >> 20 & 0x7FFu);
+    h = __funnelshift_l(lo, hi, 11) | 0x80000000u;
+    l = lo << 11;
+    sign = hi & 0x80000000u;
+    e = (unsigned)(ef - 1) < 2046u ? ef - 1023 : -4096;  // out of mul_rn's range
+  }
+};
+// x w rounded to nearest even, on the integer pipes where x, w and the
+// product are normal: the exact 106-bit product, what lies below the result's
+// 53 bits as a sticky bit, one addition.
+__device__ __forceinline__ double mul_rn(double x, const Weight &w) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int ex = (int)(hi >> 20 & 0x7FFu), t = ex + w.e;
+  if ((unsigned)(ex - 1) >= 2046u || (unsigned)(t - 2) > 2042u) return __dmul_rn(x, w.v);
+  const unsigned ah = __funnelshift_l(lo, hi, 11) | 0x80000000u, al = lo << 11;
+  typedef unsigned long long u64;
+  const u64 p0 = (u64)al * w.l;
+  const u64 p1 = (u64)ah * w.l + (p0 >> 32);
+  const u64 p2 = (u64)al * w.h + (unsigned)p1;
+  u64 q = (u64)ah * w.h + (p1 >> 32) + (p2 >> 32);  // [2^62, 2^64)
+  const unsigned rest = (unsigned)p2 | (unsigned)p0;
+  const int up = (int)(q >> 63);
+  if (!up) q = (q << 1) | ((unsigned)p2 >> 31);  // rest's top bit twice: it is sticky below bit 0 either way
+  q |= rest != 0;
+  q += 0x3FF + ((unsigned)q >> 11 & 1u);
+  const u64 m = (q >> 11) + ((long long)q >= 0 ? 1ull << 53 : 0);  // the sum carried out
+  const unsigned rh = (unsigned)(m >> 32) + ((unsigned)(t + up - 1) << 20);
+  return __hiloint2double((int)(rh | ((hi ^ w.sign) & 0x80000000u)), (int)(unsigned)m);
+}
+
+// Two of three products on the integer pipes, the third and the sums on the FP64
+// pipe, which had all of them and was the limit (one warp instruction in 64
+// cycles; about 35 integer instructions a product take as long on a pipe of
+// their own).  Six fields from the T85 grid, us with none, half, two thirds and
+// all of them there: to 1 degree 8.3, 7.6, 7.3, 6.9; 0.5 degree 20.6, 12.3, 12.3,
+// 12.4; 0.25 degree 67.7, 26.8, 26.8, 32.8; from T341 to 0.25 degree 98.5, 62.8,
+// 59.8, 67.7.
+__device__ __forceinline__ double product(bool integer, double x, const Weight &w) {
+  return integer ? mul_rn(x, w) : __dmul_rn(x, w.v);
+}
+
 // Thread = destination row r (lane of its slice, rows[]) x fields f0 .. f0+FC-1
 // (f0 = FC blockIdx.y).  Field f is read at src + f ld_src and written at
 // (f % nsub) ld_dst + (f / nsub) ld_dst2.  U records a round: their loads,
@@ -105,17 +154,18 @@ sell_apply(const int2 *__restrict__ slices, const int *__restrict__ rows, const 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (__double_as_longlong(q[u].y) < 0) continue;
+      const Weight w(q[u].x);
       if (u == 0 && k0 == 0) {
         // the row's first entry: 0 + p, which is p except that -0 becomes +0;
-        // done on the integer pipes (the FP64 pipe is this kernel's limit)
+        // done on the integer pipes
 #pragma unroll
         for (int f = 0; f < FC; ++f) {
-          const double pr = __dmul_rn(x[u][f], q[u].x);
+          const double pr = product((f + u) % 3 != 0, x[u][f], w);
           acc[f] = (__double_as_longlong(pr) << 1) == 0 ? 0.0 : pr;
         }
       } else {
 #pragma unroll
-        for (int f = 0; f < FC; ++f) acc[f] = __dadd_rn(acc[f], __dmul_rn(x[u][f], q[u].x));
+        for (int f = 0; f < FC; ++f) acc[f] = __dadd_rn(acc[f], product((f + u) % 3 != 0, x[u][f], w));
       }
     }
   }

@@ -524,11 +524,17 @@ def fp64_pipe(ops, ms, fp64_peak):
 
 
 def remap_pipe_ops(tables, members, fields=6):
-    """FP64 operations of the remap apply: one DMUL per table entry and
-    field, one DADD per entry and field after each destination row's first
-    (the first addition, 0 + p, is done on the integer pipes); tables are
+    """FP64 operations of the remap apply in a plain FP64 form: one DMUL per
+    table entry and field, one DADD per entry and field after each destination
+    row's first (the first addition, 0 + p, is exact without it); tables are
     (send, recv, coef) per group, each applied to fields x members columns."""
     return sum((2.0 * len(t[2]) - len(np.unique(t[1]))) * fields * m for t, m in zip(tables, members))
+
+
+def remap_executed_ops(tables, members, fields=6):
+    """What the kernel leaves to the FP64 pipe of remap_pipe_ops: a third of
+    the products (the others round on the integer pipes) and the sums."""
+    return sum((4.0 / 3.0 * len(t[2]) - len(np.unique(t[1]))) * fields * m for t, m in zip(tables, members))
 
 
 def roofline(S, inp, groups, stage_ms, workload, fp64_peak, flux_alone=None, products=6):
@@ -579,15 +585,17 @@ def roofline(S, inp, groups, stage_ms, workload, fp64_peak, flux_alone=None, pro
                                    "pipe": fp64_pipe(FLUX_FP64_EXECUTED_OPS_PER_COLUMN * S["ncol"],
                                                      stages["bulk_flux"]["ms"], fp64_peak)}
     # the remap keeps the reference's separately rounded products and sums
-    # (bit-exact): one DMUL per table entry and field, and one DADD per
-    # entry and field after each row's first (the first addition, 0 + p, is
-    # done on the integer pipes), reported beside its bytes
+    # (bit-exact): a product per table entry and field, two of three of them
+    # rounded on the integer pipes, and one DADD per entry and field after each
+    # row's first; reported beside its bytes
     rf = sum(2.0 * len(t[2]) * 6 * len(g.members) for g, t in zip(groups, S["tables"]))
-    rops = remap_pipe_ops(S["tables"], [len(g.members) for g in groups])
+    rops = remap_executed_ops(S["tables"], [len(g.members) for g in groups])
     tf = rf / (stages["remap"]["ms"] / 1e3) / 1e12
     stages["remap"]["fp64"] = {"achieved": tf, "unit": "TFLOP/s", "peak": fp64_peak,
                                "peak_source": "measured (dccm_fp64_peak)", "frac": tf / fp64_peak,
-                               "flops_per_launch": rf, "pipe": fp64_pipe(rops, stages["remap"]["ms"], fp64_peak)}
+                               "flops_per_launch": rf,
+                               "plain_formulation_ops": remap_pipe_ops(S["tables"], [len(g.members) for g in groups]),
+                               "pipe": fp64_pipe(rops, stages["remap"]["ms"], fp64_peak)}
     cq = sum(work[n][0] for n in CHAIN)
     cms = sum(stage_ms[names.index(n)] for n in CHAIN)
     ctr = [traffic.get(n) for n in CHAIN]

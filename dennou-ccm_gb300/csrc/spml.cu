@@ -116,12 +116,23 @@ int wa_from_spec(Plan &P, const double *spec, double *wa, int batch, cudaStream_
   return DCCM_OK;
 }
 
+// For calls that do not use the tables themselves: the first call on a plan
+// still sets them up, so that any later one can be captured; inside a capture
+// it goes without.
+static int wa_setup_outside_capture(Plan &P, cudaStream_t s) {
+  if (P.d_wa_pos) return DCCM_OK;
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  DCCM_CUDA(cudaStreamIsCapturing(s, &c));
+  return c == cudaStreamCaptureStatusNone ? wa_setup(P) : DCCM_OK;
+}
+
 int xya_wa(Plan &P, const double *wa, double *xya, int batch, cudaStream_t s) {
   // FP64: the operand pack gathers from this layout itself, but with 8 bytes
   // of every sector at a time (us against the pass of its own: T21 x 16 12.6 and
   // 16.5, T42 x 104 28.0 and 30.9, T85 x 8 28.7 and 32.9; x 128 64.3 and 63.7,
   // T170 x 64 121 and 117, T341 x 8 190 and 179).
   if (P.precision == DCCM_SHT_FP64 && P.N < 256 && (long long)(P.N + 1) * batch <= 8192) {
+    DCCM_TRY(wa_setup_outside_capture(P, s));
     DCCM_TRY(legendre_inv_f64(P, batch, wa, (double *)P.d_work, s, true));
     return fft_inverse(P, batch, false, P.d_work, xya, s);
   }
@@ -136,6 +147,7 @@ int wa_xya(Plan &P, const double *xya, double *wa, int batch, cudaStream_t s) {
   // us, 16.6 with the pass of its own, T85 x 128 55.2 and 57.6, T170 x 64 112 and
   // 115; T341 x 48 381 and 366).
   if (P.precision == DCCM_SHT_FP64 && P.N < 256) {
+    DCCM_TRY(wa_setup_outside_capture(P, s));
     DCCM_TRY(fft_forward(P, batch, false, xya, P.d_work, s));
     return legendre_fwd_f64(P, batch, (const double *)P.d_work, wa, s, true);
   }

@@ -35,3 +35,27 @@ def test_equals_permuted(dccm, cuda, N, I, J, batch):
     assert torch.equal(back, want_wa)
     torch.cuda.synchronize()
     assert P.status()[0] == 0
+
+
+def test_first_call_prepares_captured_calls(dccm, cuda):
+    """A first call of any size sets the plan's tables up for captured ones."""
+    torch = cuda
+    N, I, J, most = 85, 256, 128, 120  # 120 field-levels are permuted, 2 are not
+    P = dccm.ShtPlan(N, I, J, max_batch=most)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    wa = torch.randn(most, P.nwa, dtype=torch.float64, device="cuda", generator=gen)
+    grid = torch.zeros(most, J, I, dtype=torch.float64, device="cuda")
+    spec = torch.zeros(most, P.ncoef, 2, dtype=torch.float64, device="cuda")
+    st = torch.cuda.Stream()
+    P.xya_wa_dev(wa, grid, 2, st)
+    st.synchronize()
+    small = grid[:2].clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        P.xya_wa_dev(wa, grid, most, torch.cuda.current_stream())
+        P.spec_from_wa_dev(wa, spec, most, torch.cuda.current_stream())
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(grid[:2], small)
+    assert torch.equal(spec[:, 0, 0], wa[:, 0])
+    assert P.status()[0] == 0

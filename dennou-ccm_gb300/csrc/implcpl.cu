@@ -507,8 +507,8 @@ extern "C" int dccm_implcpl_forward_dev(dccm_implcpl *p, const dccm_implcpl_forw
   implcpl::geo_kernel<<<(unsigned)((nk + 255) / 256), 256, 0, as_stream(stream)>>>(f);
   DCCM_LAUNCH_CHECK();
   const int threads = 128;
-  DCCM_CUDA(launch_pdl(implcpl::forward_kernel, dim3((unsigned)((p->ncol + threads - 1) / threads), 2 + p->ncmax),
-                       dim3(threads), 0, as_stream(stream), f));
+  DCCM_CUDA(launch_dependent(implcpl::forward_kernel, dim3((unsigned)((p->ncol + threads - 1) / threads), 2 + p->ncmax),
+                             dim3(threads), 0, as_stream(stream), f));
   return DCCM_OK;
 }
 

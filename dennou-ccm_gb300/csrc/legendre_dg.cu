@@ -448,10 +448,12 @@ __global__ void __launch_bounds__(DG_THREADS, 1) legendre_dg_kernel(const __grid
 // parities and for re and im), then write the digits; a lane takes 8
 // coefficients of one parity (n0 + p, n0 + p + 2, ...).  Whole chunks are
 // written, zeros past the last coefficient.
-// WA: the spectra are in SPML's real layout (spml.cu).
-template <int G, bool WA>
+// Where the spectra lie: complex numbers read as 16-byte pairs, the same at an
+// address that is a multiple of 8 bytes only, SPML's real layout (spml.cu).
+enum SpecLayout { SPEC_PAIRS, SPEC_DOUBLES, SPEC_WA };
+template <int G, SpecLayout LAY>
 __global__ void __launch_bounds__(256)
-dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const double2 *__restrict__ spec, int b0, int nb,
+dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const double *__restrict__ spec, int b0, int nb,
              int nchunk, unsigned char *__restrict__ A, int *__restrict__ ea, int ldea) {
   const int m = blockIdx.y;
   const int nq0 = mi_[m].nq[0], nq1 = mi_[m].nq[1], ch0 = mi_[m].ch[0], ch1 = mi_[m].ch[1];
@@ -462,11 +464,12 @@ dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const doub
   const int bl = blockIdx.x * (256 / G) + threadIdx.x / G;  // field-level of this launch
   const bool live = bl < nb;
   const int b = b0 + (live ? bl : 0);
-  const double2 *src = spec + (long long)b * ncoef + idx_mn(N, m, m);
-  const double *wa = reinterpret_cast<const double *>(spec) + (long long)b * (N + 1) * (N + 1);
+  const double *src = spec + 2 * ((long long)b * ncoef + idx_mn(N, m, m));
+  const double *wa = spec + (long long)b * (N + 1) * (N + 1);
   auto coefficient = [&](int n) {
-    if constexpr (WA) return make_double2(__ldg(wa + wa_at(n, m, 0)), m ? __ldg(wa + wa_at(n, m, 1)) : 0.0);
-    else return __ldg(src + (n - m));
+    if constexpr (LAY == SPEC_WA) return make_double2(__ldg(wa + wa_at(n, m, 0)), m ? __ldg(wa + wa_at(n, m, 1)) : 0.0);
+    else if constexpr (LAY == SPEC_DOUBLES) return make_double2(__ldg(src + 2 * (n - m)), __ldg(src + 2 * (n - m) + 1));
+    else return __ldg(reinterpret_cast<const double2 *>(src) + (n - m));
   };
   const int nu = 4 * max(nq0, nq1);  // units of 8 a parity, both parities side by side
   unsigned mx = 0;
@@ -748,15 +751,18 @@ int legendre_inv_f64(Plan &P, int batch, const double *spec, double *F, cudaStre
     const int b0 = 64 * t, nb = batch - b0 < 64 * k ? batch - b0 : 64 * k;
     auto pack = [&](auto kernel, int g) {
       return launch_pdl(kernel, dim3((nb + 256 / g - 1) / (256 / g), P.N + 1), dim3(256), 0, s, mi, P.N, (long long)P.ncoef,
-                        (const double2 *)spec, b0, nb, P.dinv.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea);
+                        spec, b0, nb, P.dinv.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea);
     };
-    // lanes a (m, field-level): 2 units of 8 for every 16 coefficients
+    // lanes a (m, field-level): 2 units of 8 for every 16 coefficients; any
+    // number does for spectra at an odd multiple of 8 bytes
     if (wa)
-      DCCM_CUDA(P.N < 64 ? pack(dg_pack_spec<8, true>, 8) : P.N < 128 ? pack(dg_pack_spec<16, true>, 16)
-                                                                       : pack(dg_pack_spec<32, true>, 32));
+      DCCM_CUDA(P.N < 64 ? pack(dg_pack_spec<8, SPEC_WA>, 8) : P.N < 128 ? pack(dg_pack_spec<16, SPEC_WA>, 16)
+                                                                          : pack(dg_pack_spec<32, SPEC_WA>, 32));
+    else if (reinterpret_cast<uintptr_t>(spec) % 16 != 0)
+      DCCM_CUDA(pack(dg_pack_spec<32, SPEC_DOUBLES>, 32));
     else
-      DCCM_CUDA(P.N < 64 ? pack(dg_pack_spec<8, false>, 8) : P.N < 128 ? pack(dg_pack_spec<16, false>, 16)
-                                                                        : pack(dg_pack_spec<32, false>, 32));
+      DCCM_CUDA(P.N < 64 ? pack(dg_pack_spec<8, SPEC_PAIRS>, 8) : P.N < 128 ? pack(dg_pack_spec<16, SPEC_PAIRS>, 16)
+                                                                             : pack(dg_pack_spec<32, SPEC_PAIRS>, 32));
     DCCM_TRY(launch_dg(P, 0, batch, 128 * t, k, F, false, s));
   }
   return DCCM_OK;

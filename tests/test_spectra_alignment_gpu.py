@@ -1,0 +1,54 @@
+"""Spectra at any address that holds doubles.
+
+An FP64 plan takes spectra that start at an odd multiple of 8 bytes (a part
+of a larger array of doubles) both ways, with the results of the same values at a
+16-byte boundary: sizes on both sides of the packs' lane groups, ragged
+batches, and through an ensemble.
+"""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _moved(torch, x):
+    """x's values 8 bytes past a 16-byte boundary."""
+    store = torch.empty(x.numel() + 1, dtype=x.dtype, device=x.device)
+    y = store[1:].view(x.shape)
+    y.copy_(x)
+    assert y.data_ptr() % 16 == 8 and x.data_ptr() % 16 == 0
+    return y
+
+
+@pytest.mark.parametrize("N,I,J,batch", [(1, 64, 2, 1), (21, 64, 32, 7), (63, 192, 96, 3), (64, 192, 96, 65),
+                                         (127, 384, 192, 2), (128, 384, 192, 5)])
+def test_fp64_takes_any_double(dccm, cuda, N, I, J, batch):
+    torch = cuda
+    P = dccm.ShtPlan(N, I, J, max_batch=batch)
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    spec = torch.randn(batch, P.ncoef, 2, dtype=torch.float64, device="cuda", generator=gen)
+
+    def new(*shape):
+        return torch.full(shape, float("nan"), dtype=torch.float64, device="cuda")
+
+    want, got = new(batch, J, I), new(batch, J, I)
+    P.inverse_dev(spec, want, batch)
+    P.inverse_dev(_moved(torch, spec), got, batch)
+    assert torch.equal(got, want)
+    back, out = new(batch, P.ncoef, 2), _moved(torch, new(batch, P.ncoef, 2))
+    P.forward_dev(want, back, batch)
+    P.forward_dev(_moved(torch, want), out, batch)
+    assert torch.equal(out, back)
+    assert P.status()[0] == 0
+
+
+def test_fp64_ensemble(dccm, cuda):
+    torch = cuda
+    sizes = [(21, 64, 32, 3), (42, 128, 64, 2)]
+    E = dccm.Ensemble(sizes, dccm.SHT_FP64)
+    n = [b for *_, b in sizes]
+    spec = [torch.randn(b, (N + 1) * (N + 2) // 2, 2, dtype=torch.float64, device="cuda") for N, I, J, b in sizes]
+    grids = [[torch.zeros(b, J, I, dtype=torch.float64, device="cuda") for N, I, J, b in sizes] for _ in range(2)]
+    E.inverse_dev(spec, grids[0], n)
+    E.inverse_dev([_moved(torch, s) for s in spec], grids[1], n)
+    for a, b in zip(*grids):
+        assert torch.equal(a, b)

@@ -129,6 +129,9 @@ inline cudaError_t launch_surface(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
     if (st_ != DCCM_OK) return st_; \
   } while (0)
 
+// Address of complex numbers that kernels read or write as 16-byte pairs.
+inline bool pairs_aligned(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // Number of SMs of the current device (cached per device).

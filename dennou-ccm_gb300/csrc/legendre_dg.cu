@@ -758,7 +758,7 @@ int legendre_inv_f64(Plan &P, int batch, const double *spec, double *F, cudaStre
     if (wa)
       DCCM_CUDA(P.N < 64 ? pack(dg_pack_spec<8, SPEC_WA>, 8) : P.N < 128 ? pack(dg_pack_spec<16, SPEC_WA>, 16)
                                                                           : pack(dg_pack_spec<32, SPEC_WA>, 32));
-    else if (reinterpret_cast<uintptr_t>(spec) % 16 != 0)
+    else if (!pairs_aligned(spec))
       DCCM_CUDA(pack(dg_pack_spec<32, SPEC_DOUBLES>, 32));
     else
       DCCM_CUDA(P.N < 64 ? pack(dg_pack_spec<8, SPEC_PAIRS>, 8) : P.N < 128 ? pack(dg_pack_spec<16, SPEC_PAIRS>, 16)

@@ -574,6 +574,7 @@ int pack_spectra(Plan *const *plans, const int *batch, const double *const *spec
     if (batch[g] <= 0) continue;
     const Plan &P = *plans[g];
     if (!P.d_apack || !P.d_punits) return DCCM_ERR_UNSUPPORTED;
+    if (!pairs_aligned(spec[g])) return DCCM_ERR_INVALID_ARG;
     PackGroup &G = L.g[ng++];
     G.spec = reinterpret_cast<const double2 *>(spec[g]);
     G.units = P.d_punits;
@@ -924,6 +925,7 @@ int legendre_tc_multi(Plan *const *plans, const int *batch, const void *const *i
     a.cexp = dir == 0 ? P.d_cexp : P.d_cexp + P.max_batch;
     if (dir == 0) a.F = (float *)out[g];
     else a.spec_out = (double *)out[g];
+    if (dir == 1 && !pairs_aligned(out[g])) return DCCM_ERR_INVALID_ARG;
     L.map[ng] = T.map;
     L.amap[ng] = T.amap;
     L.start[ng] = items;

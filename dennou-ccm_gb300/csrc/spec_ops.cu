@@ -113,6 +113,7 @@ extern "C" int dccm_spec_apply_dev(int nmax, const dccm_spec_op *o, const double
   DCCM_TRY(spec::factors(nmax, o, t));
   if (batch < 0 || (batch > 0 && (!spec_in || !spec_out))) return DCCM_ERR_INVALID_ARG;
   if (batch == 0) return DCCM_OK;
+  if (!pairs_aligned(spec_in) || !pairs_aligned(spec_out)) return DCCM_ERR_INVALID_ARG;
   const int ncoef = (nmax + 1) * (nmax + 2) / 2;
   const int threads = nmax + 1 >= 256 ? 256 : ((nmax + 1 + 31) / 32) * 32;
   // U field-levels per CTA: every thread issues its U loads at once, and the

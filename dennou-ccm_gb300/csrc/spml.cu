@@ -99,6 +99,7 @@ static unsigned grid_for(long long total) {
 int spec_from_wa(Plan &P, const double *wa, double *spec, int batch, cudaStream_t s) {
   DCCM_TRY(wa_setup(P));
   if (batch <= 0) return DCCM_OK;
+  if (!pairs_aligned(spec)) return DCCM_ERR_INVALID_ARG;
   const long long L = (long long)(P.N + 1) * (P.N + 1), total = (long long)batch * P.ncoef;
   wa_to_spec_kernel<<<grid_for(total), 256, 0, s>>>(wa, L, P.d_wa_pos, P.ncoef, total,
                                                       reinterpret_cast<double2 *>(spec));
@@ -109,6 +110,7 @@ int spec_from_wa(Plan &P, const double *wa, double *spec, int batch, cudaStream_
 int wa_from_spec(Plan &P, const double *spec, double *wa, int batch, cudaStream_t s) {
   DCCM_TRY(wa_setup(P));
   if (batch <= 0) return DCCM_OK;
+  if (!pairs_aligned(spec)) return DCCM_ERR_INVALID_ARG;
   const long long L = (long long)(P.N + 1) * (P.N + 1), total = (long long)batch * L;
   spec_to_wa_kernel<<<grid_for(total), 256, 0, s>>>(reinterpret_cast<const double2 *>(spec), P.ncoef,
                                                       P.d_wa_src, L, total, wa);

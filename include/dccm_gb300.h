@@ -321,7 +321,11 @@ int dccm_sht_gauss(const dccm_sht_plan *plan, double *mu, double *w);
 /* FP64 Pbar table as computed on the GPU: pnm[idx(m,n)*(jmax/2) + jj] at
  * mu[jmax/2 + jj] (northern hemisphere), host array. */
 int dccm_sht_pnm(const dccm_sht_plan *plan, double *pnm);
-/* Device arrays, stream-ordered; batch <= max_batch field-levels. */
+/* Device arrays, stream-ordered; batch <= max_batch field-levels.  FP64
+ * plans take arrays at any multiple of 8 bytes; the spectra of mixed plans
+ * (here, in ensembles and steps) and those of dccm_sht_spec_from_wa_dev,
+ * dccm_sht_wa_from_spec_dev and dccm_spec_apply_dev are read and written as
+ * 16-byte pairs and start at a multiple of 16 (DCCM_ERR_INVALID_ARG else). */
 int dccm_sht_inverse_dev(dccm_sht_plan *plan, const double *spec, double *grid, int batch,
                          void *stream);
 int dccm_sht_forward_dev(dccm_sht_plan *plan, const double *grid, double *spec, int batch,

@@ -52,3 +52,38 @@ def test_fp64_ensemble(dccm, cuda):
     E.inverse_dev([_moved(torch, s) for s in spec], grids[1], n)
     for a, b in zip(*grids):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("prec", ["SHT_MIXED", "SHT_MIXED_FP16"])
+def test_others_refuse(dccm, cuda, prec):
+    """Kernels that take spectra as 16-byte pairs: the host refuses other
+    addresses, launches nothing on them, and the plan works on."""
+    torch = cuda
+    N, I, J, B = 42, 128, 64, 2
+    P = dccm.ShtPlan(N, I, J, getattr(dccm, prec), B)
+    E = dccm.Ensemble([(N, I, J, B)], getattr(dccm, prec))
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    spec = torch.randn(B, P.ncoef, 2, dtype=torch.float64, device="cuda", generator=gen)
+    grid = torch.zeros(B, J, I, dtype=torch.float64, device="cuda")
+    wa = torch.zeros(B, P.nwa, dtype=torch.float64, device="cuda")
+    moved = _moved(torch, spec)
+    op = dccm.spec_op(dccm.SPEC_LAPLACIAN, 1.0)
+    calls = {
+        "inverse": lambda s: P.inverse_dev(s, grid, B),
+        "forward": lambda s: P.forward_dev(grid, s, B),
+        "ensemble inverse": lambda s: E.inverse_dev([s], [grid], [B]),
+        "ensemble forward": lambda s: E.forward_dev([grid], [s], [B]),
+        "from wa": lambda s: P.spec_from_wa_dev(wa, s, B),
+        "to wa": lambda s: P.wa_from_spec_dev(s, wa, B),
+        "operator in": lambda s: dccm.spec_apply_dev(N, op, s, spec, B),
+        "operator out": lambda s: dccm.spec_apply_dev(N, op, spec, s, B),
+    }
+    keep = moved.clone()
+    for name, call in calls.items():
+        with pytest.raises(dccm.DccmError) as e:
+            call(moved)
+        assert e.value.status == -1, name
+        call(spec.clone())
+    torch.cuda.synchronize()
+    assert torch.equal(moved, keep)
+    assert P.status()[0] == 0

@@ -199,6 +199,7 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
   // Cp Exner_h), 1 / a
   UF upU{1ull << 63, 0}, qU{1ull << 63, 0};
   bool upv = false, qv = false;
+  bool efv = SYS == 1 && usual(ief_k);  // full level k's Exner function
   // half level k-1 and full level k-1 of the coming level k
   double Mn = 0.0, Gn = 0.0, Kdn = 0.0, Ehn = 0.0, Iefn = 0.0, fln[NR];
   auto fetch = [&](int k) {
@@ -226,10 +227,13 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
     fetch(k - 1);
     // transfer coefficient of half level k-1 (SYS 1: times Cp Exner_h)
     UF lowU{1ull << 63, 0};
+    const bool efm = SYS == 1 && usual(ief_km);
     bool lv = false;
     if (k > 1) {
+      // every factor of the two couplings across this half level: M(k,-1) and
+      // M(k-1,1) hold the Exner functions of both its full levels
       lv = a.fast && usual(Kdm) && usual(Gm);
-      if (SYS == 1) lv = lv && usual(Ehm) && usual(ief_km);
+      if (SYS == 1) lv = lv && usual(Ehm) && efv && efm;
       lowU = fx::mul(fx::from_double(Kdm), fx::from_double(Gm));
       if (SYS == 1) lowU = fx::mul(fx::mul(lowU, a.uCp), fx::from_double(Ehm));
       lowU = fx::norm(lowU);
@@ -304,6 +308,7 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
     m0p = m0e;
     ief_k1 = ief_k;
     ief_k = ief_km;
+    efv = efm;
     if (k > 1) {
       Kdk = Kdm;
       Gk = Gm;

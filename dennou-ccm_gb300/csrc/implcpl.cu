@@ -75,8 +75,8 @@ struct Fwd {
 // (with q = 1 / a carried: c = u q, q <- l / (M(k,0) - c)): products and reciprocals of positive numbers, which run with 64-bit
 // mantissas on the integer pipes (fx64.cuh), and a few signed sums in FP64.
 // The top and bottom rows, and rows where a coupling is zero, negative, not
-// finite or beyond 2^+-100, take the reference's form in FP64 (a warp
-// decides as one).  FP64 was the sweeps' limit (67 operations a column and
+// finite or beyond 2^+-100, take the reference's form in FP64: each column by
+// its own values, so that its results do not depend on the columns beside it.  FP64 was the sweeps' limit (67 operations a column and
 // level forward, 21 backward; now 12 and 8): with these, forward sweeps of
 // 32,768 columns x 32 levels took 95 us (174 in FP64), backward 35 (71).
 // What is left is the sum of three pipes' work (the ALU's about as long as
@@ -168,7 +168,6 @@ template <int SYS>
 __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tracer) {
   using fx::UF;
   constexpr int NR = SYS == 0 ? 2 : 1;
-  const unsigned warp = __activemask();
   const long long n = a.ncol;
   const int K = a.kmax;
   const double *__restrict__ Kd = SYS == 0 ? a.Kv : (SYS == 1 ? a.Kt : a.Kq);
@@ -242,7 +241,7 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
 #pragma unroll
     for (int r = 0; r < NR; ++r) b[r] = flm[r] - flk[r];
     bool done = false;
-    if (__all_sync(warp, lv && upv && qv && usual(Mm))) {
+    if (lv && upv && qv && usual(Mm)) {
       // row k: its diagonal mass + l' + u', the couplings l and u (SYS 1: the
       // couplings with their own level's Exner function, l' and u' with k's)
       UF mU = fx::from_double(Mm), l = lowU, u = upU, l0 = lowU, u0 = upU;
@@ -256,7 +255,7 @@ __device__ __forceinline__ void forward_column(const Fwd &a, long long c, int tr
       }
       const UF cU = fx::mul(u, qU);
       UF dU;
-      if (__all_sync(warp, fx::sub(fx::sum3(mU, l0, u0), cU, dU))) {
+      if (fx::sub(fx::sum3(mU, l0, u0), cU, dU)) {
         const UF iU = fx::rcp(l);
         qU = fx::mul(l, fx::rcp(dU));
         const double il = fx::to_double(iU), cc = fx::to_double(cU);

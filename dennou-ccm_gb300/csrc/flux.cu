@@ -7,7 +7,7 @@
 // so one thread evaluates the whole routine for one column in registers:
 // 21 FP64 reads and 42 FP64 writes per column, nothing else touches HBM.
 // Two forms of the column: fast_column, most of whose arithmetic runs on the
-// integer pipes, and flux_column, in FP64, for warps with inputs outside the
+// integer pipes, and flux_column, in FP64, for columns with inputs outside the
 // first one's ranges.  Expressions follow the reference's, except that
 // divisions not followed by a cancelling difference are products with a
 // shared reciprocal, the elementary functions are those of fx64.cuh (62 bits
@@ -351,7 +351,7 @@ __device__ __forceinline__ void flux_column(const Ptrs &p, const Geom &g, const 
 // ------------------------------------------------------- the integer path
 // The same column with most of its arithmetic on the integer pipes (fx64.cuh)
 // for columns whose inputs lie in the ranges checked by in_range, which hold
-// any atmosphere of interest; other warps take flux_column.
+// any atmosphere of interest; other columns take flux_column.
 //
 // FP64 was this kernel's limit (205 operations a column, 95 % of the pipe's
 // rate: 1,036,800 columns in 422 us, 45,478 in 33 us).  Two things take it
@@ -648,7 +648,7 @@ __global__ void __maxnreg__(REGS) bulk_flux_column(Ptrs p, Geom g, const __grid_
     FastIn in;
     const bool ok = g.fast && in_range<HOST>(p, g, h, t, c, SIceCon > 1e-12, in);
     const bool wpure = __all_sync(act, pure);
-    if (__all_sync(act, ok)) {
+    if (ok) {  // by the column's own values: its results do not depend on the columns beside it
       if (wpure) fast_column<HOST, true>(p, g, h, t, c, SIceCon, in);
       else fast_column<HOST, false>(p, g, h, t, c, SIceCon, in);
     } else if (wpure) {

@@ -31,7 +31,7 @@ __device__ __forceinline__ unsigned long long dg_fixed(double x, int E) {
   const int ef = (int)(b >> 52) & 0x7FF;
   // the 53-bit mantissa at bits 10 .. 62, moved down by E - ef + 1, rounded
   const unsigned long long m = ((b << 10) & 0x3FFFFFFFFFFFFC00ull) | (ef ? 1ull << 62 : 0ull);
-  const int r = min(E - max(ef, 1), 62);
+  const int r = min(E - max(ef, 1), 63);  // at 63 nothing is left
   const unsigned long long q = ((m >> r) + 1ull) >> 1;
   constexpr unsigned long long BIAS =
       256ull * (1ull + (1ull << 9) + (1ull << 18) + (1ull << 27) + (1ull << 36) + (1ull << 45) + (1ull << 54));

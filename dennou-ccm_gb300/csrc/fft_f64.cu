@@ -221,7 +221,7 @@ __device__ __forceinline__ long long to_fixed(double x, int rbase) {
   const int ef = (int)(b >> 52) & 0x7FF;
   const unsigned long long m = ((b << 10) & 0x3FFFFFFFFFFFFC00ull) | (ef ? 1ull << 62 : 0ull);
   int r = rbase - (ef ? ef : 1);
-  r = r > 63 ? 63 : r;
+  r = r > 64 ? 64 : r;  // at 64 nothing is left
   const long long q = (long long)(((m >> (r - 1)) + 1) >> 1);
   return (long long)b < 0 ? -q : q;
 }

@@ -85,7 +85,7 @@ __device__ __forceinline__ void dg_store8(unsigned char *dst, size_t stride, con
 // Sum of drained accumulators (levels s = 2 .. 8 of digit products, integers
 // below 2^24): t in units of level 6 (2^18 level-8 units), the rest below in
 // FP32 (its 24 bits reach 2^-61 of the largest product).
-// 1.01 K 2^52 < 2^63 for K products: K < 2,000.
+// 1.01 K 2^52 < 2^62 for K products: K < 1,000.
 struct DgSum {
   long long t;
   float l;

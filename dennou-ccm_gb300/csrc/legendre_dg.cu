@@ -150,14 +150,16 @@ __device__ __forceinline__ int dg_item(int k) {  // as cta_item: rounds in alter
 
 __device__ __noinline__ double dg_double_any(long long q, int ex) { return fixed_to_double(q, ex); }
 
-// Bits, at most 10, that the sums S (and those in any) have room for.
+// Bits, at most 10, that the sums S (and those in any) can be shifted up by to
+// stay below 2^62: the lower levels (DgSum::l, below 2^31 then) still come on
+// top, and carry a sum that lies just below a power of two over it.
 template <int EC> __device__ __forceinline__ int dg_room(const DgSum (&S)[EC], unsigned &any) {
 #pragma unroll
   for (int x = 0; x < EC; ++x) {
     const int hi = (int)(S[x].t >> 32);
     any |= (unsigned)(hi ^ (hi >> 31));
   }
-  return min(__clz((int)any) - 1, 10);
+  return min(__clz((int)any) - 2, 10);
 }
 
 // The integer pipes limit this part (16 results a thread of the inverse took
@@ -645,7 +647,7 @@ static void plan_dir(const Plan &P, int dir, DgTable &T, std::vector<DgMInfo> &m
   T.nchunk = ch;
   // keep the 64-bit sums of (inverse: two parities of) K products in range (DgSum)
   const int K = dir == 0 ? 2 * count_np(N, 0, 0) : Jh;
-  while (K >> T.guard > 1024) ++T.guard;
+  while (K >> T.guard > 512) ++T.guard;
   T.nitems = (int)items.size();
 }
 

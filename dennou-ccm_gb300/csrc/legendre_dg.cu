@@ -25,7 +25,8 @@
 // wavenumber m and parity p (n - m even / odd), folded by equatorial symmetry:
 //   inverse  D_p[c][jj] = sum_k S_p[c][k] Pbar_p[jj][k],
 //            F(jn) = D_0 + D_1, F(js) = D_0 - D_1 (added as integers);
-//   forward  D_p[c][k]  = sum_jj X_p[c][jj] ((w/2) Pbar)_p[k][jj].
+//   forward  D_p[c][k]  = sum_jj X_p[c][jj] ((w/2) Pbar)_p[k][jj],
+//            X and the table with a power of two per latitude (dg_fwd_scales).
 //
 // Both operands lie in global memory as the shared-memory image of a tile
 // (K-major rows of 32 values = 64 bytes, 64-byte swizzle), so that a stage
@@ -78,6 +79,7 @@ constexpr int TN = 32;                                         // rows of N an i
 constexpr int DG_B_BYTES = DG_SLICES * TN * DG_ROW;
 constexpr int DG_STAGE = DG_A_BYTES + DG_B_BYTES;              // 70 KB
 constexpr int DG_NSTAGE = 3;
+constexpr int DG_NONFINITE = 8192;                             // forward: scale exponent of a column with an infinity or NaN
 constexpr int DG_NACC = 2;                                     // accumulator sets (7 TN TMEM columns each)
 constexpr int DG_SMEM = 1024 + DG_NSTAGE * DG_STAGE + 256;
 
@@ -511,15 +513,21 @@ dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const doub
   }
 }
 
-// Folded Fourier coefficients G[m][p][jj][c] -> A images, one scale per
-// (m, p, c).  A warp takes 8 columns x 4 units of 8 latitudes (one chunk):
-// its loads are 64-byte runs along c, its stores whole rows of an image.
-// WQ warps share the chunks of 8 columns.
+// Exponents of a lane's eight latitudes, times 2^20 (of the high words' unit).
+__device__ __forceinline__ void dg_factors(const int *ec, int (&f)[8]) {
+  const int4 a = __ldg(reinterpret_cast<const int4 *>(ec)), b = __ldg(reinterpret_cast<const int4 *>(ec) + 1);
+  f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+}
+// Folded Fourier coefficients G[m][p][jj][c] -> A images, every latitude times
+// its factor 2^ec (dg_fwd_scales), one scale per (m, p, c).  A warp takes 8
+// columns x 4 units of 8 latitudes (one chunk): its loads are 64-byte runs along
+// c, its stores whole rows of an image.  WQ warps share the chunks of 8 columns.
 template <int WQ>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 dg_pack_four(const DgMInfo *__restrict__ mi_, int Jh, int C2B, int c0, int nc, const double *__restrict__ Gf, int nchunk,
-             unsigned char *__restrict__ A, int *__restrict__ ea, int ldea, int guard) {
-  __shared__ unsigned smx[8][8];
+             unsigned char *__restrict__ A, int *__restrict__ ea, int ldea, int guard, const int *__restrict__ ec_,
+             int ldec) {
+  __shared__ int smx[8][8];
   const int mp = blockIdx.y, m = mp >> 1, p = mp & 1;
   const int nv = mi_[m].nv[p], nq = mi_[m].nq[p], ch = mi_[m].ch[p];
   asm volatile("" ::"r"(nv + nq + ch));  // plan constants: loaded before the wait
@@ -531,15 +539,23 @@ dg_pack_four(const DgMInfo *__restrict__ mi_, int Jh, int C2B, int c0, int nc, c
   const bool live = cl < nc;
   if (nv <= 0) return;  // this parity has no coefficient (uniform over the block)
   const double *src = Gf + (long long)mp * Jh * C2B + c0 + (live ? cl : 0);
+  const int *ec = ec_ + (long long)mp * ldec;
   double v[8];
-  unsigned mx = 0;
+  int f[8];  // (loaded again for the digits: eight registers fewer meanwhile)
+  int mx = 1 << 20;  // exponents are at most 0: enough for zeros and subnormals
+  unsigned any = 0;
   for (int q = warp % WQ; q < nq; q += WQ) {
     const int j0 = q * DG_CHUNK + 8 * u;
+    dg_factors(ec + j0, f);
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = live && j0 + e < Jh ? __ldg(src + (long long)(j0 + e) * C2B) : 0.0;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) mx = max(mx, dg_mag(v[e]));
+    for (int e = 0; e < 8; ++e) {
+      any = max(any, dg_mag(v[e]));
+      mx = max(mx, (int)dg_mag(v[e]) + f[e]);
+    }
   }
+  mx = any < 0x7FF00000u ? mx >> 20 : DG_NONFINITE;
   mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
   mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
   if (WQ > 1) {
@@ -549,12 +565,13 @@ dg_pack_four(const DgMInfo *__restrict__ mi_, int Jh, int C2B, int c0, int nc, c
     for (int k = 0; k < WQ; ++k) mx = max(mx, smx[warp / WQ * WQ + k][c8]);
   }
   if (!live) return;
-  const int E = dg_exp(mx) + guard;
+  const int E = mx + guard;
   if (u == 0 && warp % WQ == 0) ea[(long long)mp * ldea + c0 + cl] = E;
   const int ct = cl / 128, row = cl % 128;
   const bool keep = nq <= WQ;
   for (int q = warp % WQ; q < nq; q += WQ) {
     const int j0 = q * DG_CHUNK + 8 * u;
+    dg_factors(ec + j0, f);
     if (!keep) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = j0 + e < Jh ? __ldg(src + (long long)(j0 + e) * C2B) : 0.0;
@@ -562,35 +579,62 @@ dg_pack_four(const DgMInfo *__restrict__ mi_, int Jh, int C2B, int c0, int nc, c
     unsigned char *img = A + ((long long)ct * nchunk + ch + q) * DG_A_BYTES;
     unsigned long long qv[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) qv[e] = dg_fixed(v[e], E);
+    for (int e = 0; e < 8; ++e) qv[e] = dg_fixed(v[e], E - (f[e] >> 20));
     dg_store8(img + dg_unit(row, u), DG_A_SLICE, qv);
   }
 }
 
 // ------------------------------------------------------------------ tables
-// Scale exponent of every table row: inverse rows (m, jj) over all n;
-// forward rows (m, n) over all latitudes of (w/2) Pbar.  The stored value is
-// E - 1022: the row's entries are below 2^eb.  One warp per row.
-__global__ void dg_row_scale(int dir, int N, int Jh, const double *__restrict__ pnm, const double *__restrict__ w,
-                             long long nrows, short *__restrict__ eb) {
+// Inverse: scale exponent of every table row (m, jj) over all n.  The stored
+// value is E - 1022: the row's entries are below 2^eb.  One warp per row.
+__global__ void dg_inv_scales(int N, int Jh, const double *__restrict__ pnm, long long nrows, short *__restrict__ eb) {
   const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (r >= nrows) return;
   unsigned mx = 0;
-  if (dir == 0) {
-    const int m = (int)(r / Jh), jj = (int)(r % Jh);
-    for (int n = m + lane; n <= N; n += 32) mx = max(mx, dg_mag(pnm[idx_mn(N, m, n) * Jh + jj]));
-  } else {
-    for (int jj = lane; jj < Jh; jj += 32) mx = max(mx, dg_mag((0.5 * w[Jh + jj]) * pnm[r * Jh + jj]));
-  }
+  const int m = (int)(r / Jh), jj = (int)(r % Jh);
+  for (int n = m + lane; n <= N; n += 32) mx = max(mx, dg_mag(pnm[idx_mn(N, m, n) * Jh + jj]));
   mx = __reduce_max_sync(0xffffffffu, mx);
   if (lane == 0) eb[r] = (short)(dg_exp(mx) - 1022);
+}
+
+// Forward: factors 2^ec of the latitudes, 2^-ec of them on the table, such
+// that every latitude's largest entry of (w/2) Pbar over the degrees of one (m, p)
+// lies in [2^7, 2^8) (ec < 0: entries are at most sqrt(2 N + 1) / 2); then the scale exponent of every row (m, n) over the
+// latitudes.  Towards the poles the entries of large m fall by hundreds of orders
+// of magnitude, and the Fourier coefficients need not: without the factors the
+// largest coefficient set the scale although its products count for nothing, and
+// a field non-zero near the poles alone lost whole wavenumbers (T85: from m =
+// 40 on).  With them the scale is that of the largest product of the (m, p).
+// Block (m, p); ec[(2 m + p) ldec + jj] times 2^20, zero past the last latitude.
+__global__ void __launch_bounds__(256)
+dg_fwd_scales(const DgMInfo *__restrict__ mi_, int N, int Jh, const double *__restrict__ pnm, const double *__restrict__ w,
+              int *__restrict__ ec_, int ldec, short *__restrict__ eb) {
+  const int mp = blockIdx.x, m = mp >> 1, p = mp & 1;
+  const int nv = mi_[m].nv[p];
+  int *ec = ec_ + (long long)mp * ldec;
+  const double *tab = pnm + (idx_mn(N, m, m) + p) * Jh;  // row k (n = m + p + 2 k) at 2 k Jh
+  for (int jj = threadIdx.x; jj < ldec; jj += blockDim.x) {
+    unsigned mx = 0;
+    if (jj < Jh)
+      for (int k = 0; k < nv; ++k) mx = max(mx, dg_mag((0.5 * w[Jh + jj]) * tab[2LL * k * Jh + jj]));
+    ec[jj] = jj < Jh && nv > 0 ? (dg_exp(mx) - 1030) * (1 << 20) : 0;
+  }
+  __syncthreads();
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  for (int k = warp; k < nv; k += blockDim.x / 32) {
+    int mx = -4096;
+    for (int jj = lane; jj < Jh; jj += 32) mx = max(mx, dg_exp(dg_mag((0.5 * w[Jh + jj]) * tab[2LL * k * Jh + jj])) - (ec[jj] >> 20));
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) eb[mi_[m].eb[p] + p + 2 * k] = (short)(mx - 1022);
+  }
 }
 
 // Table tiles: thread = (m, p, row of N, unit of 8 along K).
 __global__ void __launch_bounds__(256)
 dg_build(int dir, int N, int Jh, const DgMInfo *__restrict__ mi_, const double *__restrict__ pnm,
-         const double *__restrict__ w, const short *__restrict__ eb, unsigned char *__restrict__ B) {
+         const double *__restrict__ w, const short *__restrict__ eb, const int *__restrict__ ec, int ldec,
+         unsigned char *__restrict__ B) {
   const int m = blockIdx.y, p = blockIdx.z;
   const DgMInfo &mi = mi_[m];
   const int nu = 4 * mi.nq[p];
@@ -604,11 +648,13 @@ dg_build(int dir, int N, int Jh, const DgMInfo *__restrict__ mi_, const double *
     for (int e = 0; e < 8; ++e) {
       const int k = 8 * ug + e;
       double x = 0.0;
+      int Ek = 1;
       if (r < mi.nv[p] && k < mi.kv[p]) {
         if (dir == 0) x = pnm[idx_mn(N, m, m + p + 2 * k) * Jh + r];
         else x = (0.5 * w[Jh + k]) * pnm[idx_mn(N, m, m + p + 2 * r) * Jh + k];
+        Ek = dir == 0 ? E : E + (ec[(2 * m + p) * ldec + k] >> 20);
       }
-      q[e] = dg_fixed(x, E);
+      q[e] = dg_fixed(x, Ek);
     }
     const int nt = r / TN, ntw = min(TN, mi.nr[p] - nt * TN);
     unsigned char *tile = B + mi.tab[p] +
@@ -662,7 +708,8 @@ int build_digits(Plan &P) {
   // scales, tiles
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
   const long long nrows[2] = {(long long)(P.N + 1) * P.Jh, (long long)P.ncoef};
-  size_t at_mi[2], at_it[2], at_eb[2], at_tab[2], at = 0;
+  const int ldec = (P.Jh + DG_CHUNK - 1) / DG_CHUNK * DG_CHUNK;
+  size_t at_mi[2], at_it[2], at_eb[2], at_tab[2], at_ec, at = 0;
   for (int d = 0; d < 2; ++d) {
     plan_dir(P, d, *T[d], mi[d], items[d], tab[d]);
     at_mi[d] = at;
@@ -678,6 +725,8 @@ int build_digits(Plan &P) {
     at_tab[d] = at + up((size_t)nrows[d] * sizeof(short));
     at = up(at_tab[d] + (size_t)tab[d]);
   }
+  at_ec = at;
+  at += (size_t)2 * (P.N + 1) * ldec * sizeof(int);
   DCCM_CUDA(cudaMalloc(&P.d_dgmem, at));
   unsigned char *base = (unsigned char *)P.d_dgmem;
   DCCM_CUDA(cudaMemcpyAsync(base, h.data(), h.size(), cudaMemcpyHostToDevice));
@@ -686,10 +735,15 @@ int build_digits(Plan &P) {
     T[d]->d_items = (int2 *)(base + at_it[d]);
     T[d]->d_eb = (short *)(base + at_eb[d]);
     T[d]->d_tab = base + at_tab[d];
-    dg_row_scale<<<(unsigned)((nrows[d] + 7) / 8), 256>>>(d, P.N, P.Jh, P.d_pnm, P.d_w, nrows[d], T[d]->d_eb);
+    T[d]->d_ec = d == 0 ? nullptr : (int *)(base + at_ec);
+    if (d == 0)
+      dg_inv_scales<<<(unsigned)((nrows[d] + 7) / 8), 256>>>(P.N, P.Jh, P.d_pnm, nrows[d], T[d]->d_eb);
+    else
+      dg_fwd_scales<<<2 * (P.N + 1), 256>>>((const DgMInfo *)T[d]->d_mi, P.N, P.Jh, P.d_pnm, P.d_w, T[d]->d_ec, ldec,
+                                            T[d]->d_eb);
     DCCM_LAUNCH_CHECK();
     dg_build<<<dim3(16, P.N + 1, 2), 256>>>(d, P.N, P.Jh, (const DgMInfo *)T[d]->d_mi, P.d_pnm, P.d_w, T[d]->d_eb,
-                                            (unsigned char *)T[d]->d_tab);
+                                            T[d]->d_ec, ldec, (unsigned char *)T[d]->d_tab);
     DCCM_LAUNCH_CHECK();
   }
   const int nch = P.dinv.nchunk > P.dfwd.nchunk ? P.dinv.nchunk : P.dfwd.nchunk;
@@ -728,7 +782,7 @@ static int launch_dg(Plan &P, int dir, int batch, int c0, int nct, double *out, 
   a.nitems = T.nitems;
   a.nchunk = T.nchunk;
   a.ldea = P.dg_ldea;
-  a.enan = 2047 + T.guard;
+  a.enan = dir == 0 ? 2047 : DG_NONFINITE;
   a.ncoef = P.ncoef;
   a.mi = (const DgMInfo *)T.d_mi;
   a.items = T.d_items;
@@ -780,7 +834,8 @@ int legendre_fwd_f64(Plan &P, int batch, const double *G, double *spec, cudaStre
     auto pack = [&](auto kernel, int wq) {
       const int per = 8 * (8 / wq);
       return launch_pdl(kernel, dim3((nc + per - 1) / per, 2 * (P.N + 1)), dim3(256), 0, s, mi, P.Jh, 2 * batch, c0, nc, G,
-                        P.dfwd.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea, P.dfwd.guard);
+                        P.dfwd.nchunk, (unsigned char *)P.d_dig, P.d_ea, P.dg_ldea, P.dfwd.guard,
+                        (const int *)P.dfwd.d_ec, nq * DG_CHUNK);
     };
     DCCM_CUDA(nq <= 1 ? pack(dg_pack_four<1>, 1) : nq <= 2 ? pack(dg_pack_four<2>, 2)
               : nq <= 4 ? pack(dg_pack_four<4>, 4) : pack(dg_pack_four<8>, 8));

@@ -53,10 +53,11 @@ struct TileTable {
 
 // FP64 path: one direction's digit tables (legendre_dg.cu).
 struct DgTable {
-  // (the four arrays lie in Plan::d_dgmem)
+  // (the arrays lie in Plan::d_dgmem)
   void *d_mi = nullptr;       // per-m tile metadata
   int2 *d_items = nullptr;    // work items (m, nt) of one 128-column tile
   short *d_eb = nullptr;      // scale exponent of every table row
+  int *d_ec = nullptr;      // forward: exponent of every latitude's factor
   void *d_tab = nullptr;      // shared-memory images of the table tiles
   int nchunk = 0;             // A chunks per 128-column tile
   int nitems = 0;

@@ -7,7 +7,7 @@
 // at 2^-62 of it below), and Q in seven balanced digits of 9 bits,
 //   a = 2^(E-1030) sum_{i=1..7} d_i 2^(-9 (i-1)),  |d_i| <= 256,
 // every one an FP16 number exactly.  Products of digits are integers of at
-// most 2^16, so FP32 accumulation of up to 2^24 / 2^16 of them is exact.
+// most 2^16, so FP32 accumulation of them is exact up to a sum of 2^24.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -82,8 +82,8 @@ __device__ __forceinline__ void dg_store8(unsigned char *dst, size_t stride, con
   put(6, low);
 }
 
-// Sum of drained accumulators (levels s = 2 .. 8 of digit products, integers
-// below 2^24): t in units of level 6 (2^18 level-8 units), the rest below in
+// Sum of drained accumulators (levels s = 2 .. 8 of digit products, 2 .. 5
+// integers below 2^24): t in units of level 6 (2^18 level-8 units), the rest below in
 // FP32 (its 24 bits reach 2^-61 of the largest product).
 // 1.01 K 2^52 < 2^62 for K products: K < 1,000.
 struct DgSum {

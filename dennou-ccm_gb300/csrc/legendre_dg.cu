@@ -12,14 +12,19 @@
 // the products d_i(a) d_j(b) of equal weight, s = i + j = 2 .. 8, are
 // summed in one FP32 accumulator per s: integers below 2^24, so the sums
 // are exact.  28 MMAs take the place of an FP64 FMA; the products left out
-// (s >= 9) are below 2^-60 of (largest |a|) (largest |b|), well under the
-// rounding errors of an FP64 sum.
+// (s >= 9) are below 2^-60 of (largest |a|) (largest |b|).  Errors are thus
+// relative to the largest product of a contraction (one m, parity and
+// field-level; synthesis: of the row of the table), where they are well under
+// the rounding errors of an FP64 sum; a result far smaller than that has fewer
+// correct digits than an FP64 sum of its own products would give it.
 //
-// Exactness: an accumulator takes at most DG_KB = 128 values of K before it
-// is drained, so levels s = 2, 3 (one and two products of at most 2^16 a
-// value) stay within 2^24 whatever the data; levels 4 and 5 do for any data
-// because the table's lower digits average 128 in magnitude; from level 6
-// on (below 2^-52 of the largest product) a rounding would not be seen.
+// Exactness: an accumulator takes at most 96 values of K (DG_KB chunks) before
+// it is drained, so levels s = 2 and 3 (one and two products of at most 2^16 a
+// value) stay within 2^24 whatever the tables, and levels 4 and 5 whatever the
+// data, by the digits that the tables have (0.94 of 2^24 at most; with 128
+// values level 5 could reach 1.2: a unit of it is 2^-43 of the largest product.
+// A drain more an item of the T341 analysis: 2,597 -> 2,612 us both ways); from
+// level 6 on (below 2^-52 of the largest product) a rounding would not be seen.
 //
 // As the mixed path (legendre_tc.cu) the contractions run per zonal
 // wavenumber m and parity p (n - m even / odd), folded by equatorial symmetry:
@@ -68,7 +73,7 @@ namespace dccm {
 namespace sht {
 
 constexpr int DG_CHUNK = 32;                                   // K of a stage
-constexpr int DG_KB = 4;                                       // chunks an accumulator takes (128 values of K)
+constexpr int DG_KB = 3;                                       // chunks an accumulator takes (96 values of K)
 constexpr int DG_ROW = 2 * DG_CHUNK;                           // bytes of a K-major row of a chunk
 constexpr int DG_A_SLICE = 128 * DG_ROW;                       // 8 KB
 constexpr int DG_A_BYTES = DG_SLICES * DG_A_SLICE;             // 56 KB

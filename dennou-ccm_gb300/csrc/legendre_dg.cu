@@ -705,6 +705,10 @@ static void plan_dir(const Plan &P, int dir, DgTable &T, std::vector<DgMInfo> &m
 // Tables of both directions and the A images.  The images of one launch are
 // bounded (DG_WORK_CAP); a larger batch takes several launches.
 int build_digits(Plan &P) {
+  // set here and not by the first launch of a process: it holds for the
+  // device and context that the plan is made in
+  for (auto kernel : {legendre_dg_kernel<0, false>, legendre_dg_kernel<1, false>, legendre_dg_kernel<1, true>})
+    DCCM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
   DgTable *T[2] = {&P.dinv, &P.dfwd};
   std::vector<DgMInfo> mi[2];
   std::vector<int2> items[2];
@@ -765,11 +769,6 @@ int build_digits(Plan &P) {
 }
 
 template <int DIR, bool WA> static int launch_kernel(const DgArgs &a, int items, cudaStream_t s) {
-  static bool attr_done = false;
-  if (!attr_done) {
-    DCCM_CUDA(cudaFuncSetAttribute(legendre_dg_kernel<DIR, WA>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
-    attr_done = true;
-  }
   const int ctas = sm_count();
   DCCM_CUDA(launch_pdl(legendre_dg_kernel<DIR, WA>, dim3(items < ctas ? items : ctas), dim3(DG_THREADS), (size_t)DG_SMEM, s,
                        a));

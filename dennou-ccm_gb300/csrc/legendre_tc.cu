@@ -865,17 +865,26 @@ static int build_pack(Plan &P) {
   return DCCM_OK;
 }
 
+template <bool NARROW> static size_t tc_smem_bytes() {
+  return 1024 + (size_t)TcShape<NARROW>::NSTAGE * TcShape<NARROW>::STAGE_BYTES + 128 + EP_BYTES;
+}
+
 // Called after d_work exists (the forward A map points into it).
 int build_tiles(Plan &P) {
+  // set here and not by the first launch of a process: they hold for the
+  // device and context that the plan is made in
+  DCCM_CUDA(cudaFuncSetAttribute(legendre_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)tc_smem_bytes<false>()));
+  DCCM_CUDA(cudaFuncSetAttribute(legendre_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)tc_smem_bytes<true>()));
+  DCCM_CUDA(cudaFuncSetAttribute(legendre_tc_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared));
   DCCM_TRY(build_pack(P));
   DCCM_TRY(build_one(P, 0, P.tinv));
   DCCM_TRY(build_one(P, 1, P.tfwd));
   return DCCM_OK;
 }
 
-template <bool NARROW> static size_t tc_smem_bytes() {
-  return 1024 + (size_t)TcShape<NARROW>::NSTAGE * TcShape<NARROW>::STAGE_BYTES + 128 + EP_BYTES;
-}
 
 // One persistent launch over ngroups plans (truncation groups) of one
 // direction: dir 0 (inverse) reads the plan's packed spectra (pack_spectra
@@ -885,17 +894,7 @@ template <bool NARROW> static size_t tc_smem_bytes() {
 int legendre_tc_multi(Plan *const *plans, const int *batch, const void *const *in, void *const *out,
                       int ngroups, int dir, cudaStream_t s) {
   (void)in;
-  static bool attr_done = false;
   if (ngroups < 1 || ngroups > MAXG) return DCCM_ERR_UNSUPPORTED;
-  if (!attr_done) {
-    DCCM_CUDA(cudaFuncSetAttribute(legendre_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)tc_smem_bytes<false>()));
-    DCCM_CUDA(cudaFuncSetAttribute(legendre_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)tc_smem_bytes<true>()));
-    DCCM_CUDA(cudaFuncSetAttribute(legendre_tc_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                   (int)cudaSharedmemCarveoutMaxShared));
-    attr_done = true;
-  }
   TcLaunch L;
   memset(&L, 0, sizeof L);
   int ntmax = 64, ng = 0, items = 0;

@@ -12,9 +12,10 @@
 // Rows pair up as in fft.cu: z = g(jn) + i g(js), one complex transform of
 // length I = R1 R2 (R3) by T = I / R1 threads.  A row pair has one scale:
 //   forward  the largest magnitude of the pair sits at 2^CB; every pass
-//            of radix R is followed by its twiddles times 2^-ceil(log2 R),
-//            so nothing overflows (|Z| <= sum |z|) and a pass rounds once,
-//            below 2^-53 of the row's r.m.s. for noise-like rows;
+//            of radix R is followed by its twiddles times 2^-ceil(log2 R)
+//            (12: times 2/3 2^-3), so nothing overflows (|Z| <= sum |z|) and
+//            a pass rounds once, below 2^-53 of the row's r.m.s. for
+//            noise-like rows and below 2^-52 for a single value;
 //   inverse  every partial sum of the transform is bounded by the sum S of
 //            the input magnitudes, so the inputs are scaled with S at 2^62
 //            and no pass scales: roundings are a few 2^-62 S.
@@ -184,10 +185,12 @@ template <int I_, int R1_, int R2_, int R3_> struct Shape {
   static constexpr int N1 = I / R1, N2 = N1 / R2;  // N2 = R3
   static constexpr int T = N1;                     // threads a row pair
   static constexpr int RL = R3 > 1 ? R3 : R2;      // last radix
-  static constexpr int S1 = clog2(R1), S2 = R3 > 1 ? clog2(R2) : 0;
-  // forward: components of the input below 2^CB, so that R1 2^(CB + 1/2) and
-  // the fold of four results of the last pass stay below 2^63
-  static constexpr int CB = 60 - clog2(RL) < 58 ? 60 - clog2(RL) : 58;
+  // forward: bits that a pass scales down by (R1 = 12: with the 2/3 of 1/I)
+  static constexpr int S1 = R1 == 12 ? 3 : clog2(R1), S2 = R3 > 1 ? clog2(R2) : 0;
+  // forward: components of the input at most (1 - 2^-53) 2^CB, so that R1 2^(CB +
+  // 1/2) and the fold of four results of the last pass, 4 RL (1 - 2^-53) 2^CB
+  // and a few units of rounding, stay below 2^63
+  static constexpr int CB = 61 - clog2(RL) < 58 ? 61 - clog2(RL) : 58;
   static constexpr int THREADS = T >= 64 ? 256 : 128;
   static constexpr int BB = THREADS / T;
   // CTAs of an SM: eight points a thread fit 80 registers, 12 or 16 take 128

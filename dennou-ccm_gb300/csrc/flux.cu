@@ -439,7 +439,8 @@ __device__ __forceinline__ SlotOut fast_slot(const Geom &g, const FastCol &k, do
   constexpr long long a0 = (long long)(b0.m / 273 * 128 + b0.m % 273 * 128 / 273),
                       a1 = (long long)(b1.m / 273 * 128 + b1.m % 273 * 128 / 273);
   const u64 b = mulhi(rts.m, ocean ? b0.m : b1.m);
-  const UF ex = exp_fix((ocean ? a0 : a1) - (long long)(b << 1 >> (ts.e - 7)));
+  // (b / Ts reaches 48 at 128 K, beyond a signed word; the difference is within 26)
+  const UF ex = exp_fix((long long)((u64)(ocean ? a0 : a1) - (b << 1 >> (ts.e - 7))));
   const UF qs = norm(mul(mul(k.rps, uf(Es0 * (MolWtWet / MolWtDry))), ex));
   o.QSat = to_double(qs);
   // bulk Richardson number; an exact zero becomes 2^-200 (unstable branch, as Ri = 0)

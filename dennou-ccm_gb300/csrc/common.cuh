@@ -65,8 +65,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 int greatest_priority();
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                              Args &&...args) {
+inline cudaError_t launch_attr(bool dependent, bool urgent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                               cudaStream_t s, Args &&...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -74,11 +74,11 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
   unsigned n = 0;
-  if (!tunables().serial) {
+  if (dependent) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n++].val.programmaticStreamSerializationAllowed = 1;
   }
-  if (tunables().prio == 1) {
+  if (urgent) {
     attr[n].id = cudaLaunchAttributePriority;
     attr[n++].val.priority = greatest_priority();
   }
@@ -87,40 +87,28 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// The same outside the transform chain: dependent on the previous kernel, at
-// the stream's own priority whatever the "prio" knob.
+// A kernel of the transform chain: dependent on the previous one (unless the
+// "serial" knob is set), at the device's greatest priority with the "prio"
+// knob at 1.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                              Args &&...args) {
+  return launch_attr(!tunables().serial, tunables().prio == 1, kernel, grid, block, smem, s, std::forward<Args>(args)...);
+}
+
+// The same outside the transform chain, at the stream's own priority.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                     Args &&...args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = tunables().serial ? 0 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  return launch_attr(!tunables().serial, false, kernel, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
-// Launch of a surface-branch kernel (remap, flux): at the device's greatest
-// priority with the "prio" knob at 2, else an ordinary launch.
+// A surface-branch kernel (remap, flux): at the device's greatest priority with
+// the "prio" knob at 2, else an ordinary launch.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_surface(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                   Args &&...args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributePriority;
-  attr[0].val.priority = greatest_priority();
-  cfg.attrs = attr;
-  cfg.numAttrs = tunables().prio == 2 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  return launch_attr(false, tunables().prio == 2, kernel, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
 #define DCCM_TRY(expr)           \

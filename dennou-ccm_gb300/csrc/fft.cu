@@ -912,16 +912,13 @@ int fft_multi(Plan *const *plans, const int *batch, const void *const *in, void 
     wt += (long long)plans[g]->Jh * batch[g] * W;
   }
   // Defaults where the knobs are 0.  Rows over three or four warps: 16 warps
-  // a CTA, so that a G3 run is wider (inverse / forward with their Legendre
-  // steps, 16 against 8 warps: T255 x 16 58 / 58 and 60 / 61 us, x 300 529 /
-  // 588 and 541 / 664 us; T341 x 4 66 / 70 and 66 / 73 us).  Two row pairs a
-  // warp halve the warps and widen the runs once the launch has warps for
-  // two waves: 60 an SM (T21 x 700 18.7 / 15.5 with two, 17.9 / 16.4 us with
-  // one; T63 x 200 24.2 / 23.9 and 24.9 / 23.7; T85 x 512 79.6 / 78.6 and
-  // 84.6 / 82.2; T170 x 40 41.6 / 41.5 and 43.4 / 44.3; below, T42 x 104
-  // 15.8 / 15.6 and 14.3 / 13.0, T127 x 60 33.9 / 35.0 and 30.1 / 31.3), 40
-  // for rows over four warps, whose CTAs are larger (T341 x 8 74 / 77 and
-  // 79 / 82 us, x 192 530 / 580 and 602 / 685; x 4 70 / 74 and 66 / 70).
+  // a CTA, so that a G3 run is wider (forward, 16 against 8 warps: T255 x 300
+  // 588 and 664 us, T341 x 4 70 and 73).  Two row pairs a warp halve the warps
+  // and widen the runs once the launch has warps for two waves: 60 an SM
+  // (forward, two against one: T85 x 512 78.6 and 82.2 us, T170 x 40 41.5 and
+  // 44.3; below, T42 x 104 15.6 and 13.0, T127 x 60 35.0 and 31.3), 40 for
+  // rows over four warps, whose CTAs are larger (T341 x 8 77 and 82, x 192 580
+  // and 685; x 4 74 and 70).
   const int rpw = tr == 1 || tr == 2 ? tr : (wt >= (wmin == 4 ? 40LL : 60LL) * sm_count() ? 2 : 1);
   int wpc = wmin >= 3 ? 16 : 8;
   if (wmin >= 3 && ngroups == 1) {
@@ -941,8 +938,10 @@ int fft_multi(Plan *const *plans, const int *batch, const void *const *in, void 
     if (batch[g] <= 0) continue;
     const Plan &P = *plans[g];
     const int R = P.I / 32, W = fft_warps_per_row(R);
-    // FP16 rows of 12 samples a lane lose by two (T127 x 505 analysis 216 -> 228
-    // us; BF16 x 3 181 -> 172)
+    // FP16 rows of 12 samples a lane lose by two (T127 analysis, one / two: x 100
+    // 57.5 / 61.7 us, x 192 95 / 100, x 320 154 / 163, x 505 210 / 224; BF16 x 3
+    // 47 / 50, 74 / 74, 117 / 117, 179 / 175; FP16 rows of 6 and 8 do not: T85 x
+    // 512 103 / 101, T63 x 505 65 / 62)
     const int rp = W == 3 || (tr == 0 && fwd && P.nsplit == 2 && R == 12) ? 1 : rpw;
     int BB = 1;
     while (2 * BB * W <= WPC * rp && fft_smem(R, 2 * BB, WPC / W) <= budget) BB *= 2;

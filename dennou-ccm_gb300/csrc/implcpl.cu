@@ -76,10 +76,12 @@ struct Fwd {
 // mantissas on the integer pipes (fx64.cuh), and a few signed sums in FP64.
 // The top and bottom rows, and rows where a coupling is zero, negative, not
 // finite or beyond 2^+-100, take the reference's form in FP64: each column by
-// its own values, so that its results do not depend on the columns beside it.  FP64 was the sweeps' limit (67 operations a column and
-// level forward, 21 backward; now 12 and 8): with these, forward sweeps of
-// 32,768 columns x 32 levels took 95 us (174 in FP64), backward 35 (71).
-// What is left is the sum of three pipes' work (the ALU's about as long as
+// its own values, so that its results do not depend on the columns beside it.
+// FP64 was the sweeps' limit (67 operations a column and level forward, 21
+// backward; now 12 and 8): with these, forward sweeps of 32,768 columns x 32
+// levels took 95 us (174 in FP64), backward 35 (71); with one column in seven
+// without diffusion aloft forward 216 (218 with every row in FP64), 2,048 x 16
+// 36 (34).  What is left is the sum of three pipes' work (the ALU's about as long as
 // FP64's).  The level after the current one is always being fetched: 95 -> 75
 // us, 131,072 x 48 397 -> 324, against two levels fetched together ahead of
 // their use (five CTAs an SM at 102 registers or four at 128).  The backward

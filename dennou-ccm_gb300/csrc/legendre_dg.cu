@@ -5,7 +5,7 @@
 // (1.05 TFLOP/s measured), and the contraction took 80 % of the plain FP64
 // transforms as an FP64 FMA loop (T341 x 192 field-levels: synthesis 10.4
 // ms, analysis 13.5 ms; T85 x 128: 209 and 340 us; with the kernels below
-// 0.52, 0.61 ms, 32 and 31 us, packs included).  Here every operand is
+// 0.53, 0.61 ms, 39 and 35 us, packs included).  Here every operand is
 // split into seven 9-bit digits (digits.cuh: the scheme of K. Ozaki, T.
 // Ogita, S. Oishi, S. Rump, "Error-free transformations of matrix
 // multiplication", Numer. Algorithms 59 (2012), with integer digits), and
@@ -52,11 +52,8 @@
 // MMAs at the peak rate; clock stamps show the MMAs of two steps issued in
 // 1,360 cycles, and 2,000 with the drains beside them.  TN = 64 (half the
 // reads of A, but one accumulator set, whose drains the MMAs then wait for)
-// came out at 591 and 644 us against 571 and 626, and 16 % slower at T85.
-// Sixteen epilogue warps instead of eight: 776 -> 710 us.  At T85 and below an
-// item is latency: the loads 0.7 us, a chunk's MMAs 0.6, draining a set 0.8,
-// the results 2-3.  Digits made by the epilogue warps in the stages, without
-// the packs, were slower everywhere (T42 x 104 26.7 / 24.1 -> 30.6 / 26.5 us).
+// is 3 % slower there and 16 % at T85.  At T85 and below an item is latency:
+// the loads 0.7 us, a chunk's MMAs 0.6, draining a set 0.8, the results 2-3.
 //
 // A work item is (m, 128 columns c, TN rows of N).  Warp 0 copies, warp 1
 // allocates TMEM and issues the MMAs, warps 2-17 drain the accumulators
@@ -197,7 +194,7 @@ __device__ __forceinline__ void dg_results(const int (&eb)[EC], int E, int up, i
 // registers: they are loaded an item ahead (the first before the wait for the
 // kernel before, a chain of loads of 1 us), their place in the list two ahead.
 // Read through the table at each use, that is anew after every wait and copy,
-// T341 x 192 took 538 / 638 us with its pack (inverse / forward), now 520 / 616.
+// T341 x 192 took 3 % longer.
 struct DgWalk {
   int k, it, ct, m, nt;
   DgMInfo mi;

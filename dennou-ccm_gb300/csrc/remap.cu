@@ -108,10 +108,11 @@ __device__ __forceinline__ double mul_rn(double x, const Weight &w) {
 // Two of three products on the integer pipes, the third and the sums on the FP64
 // pipe, which had all of them and was the limit (one warp instruction in 64
 // cycles; about 35 integer instructions a product take as long on a pipe of
-// their own).  Six fields from the T85 grid, us with none, half, two thirds and
-// all of them there: to 1 degree 8.3, 7.6, 7.3, 6.9; 0.5 degree 20.6, 12.3, 12.3,
-// 12.4; 0.25 degree 67.7, 26.8, 26.8, 32.8; from T341 to 0.25 degree 98.5, 62.8,
-// 59.8, 67.7.
+// their own).  Six fields from the T85 grid, us a launch back to back with none,
+// half, two thirds and all of them there: to 0.5 degree 20.6, 12.3, 12.3, 12.4;
+// 0.25 degree 67.7, 26.8, 26.8, 32.8; from T341 to 0.25 degree 98.5, 62.8, 59.8,
+// 67.7.  To 1 degree a launch in a graph takes 6.8 with none and 5.5 with two
+// thirds (an empty one 2.1); a call from the host takes longer than either.
 __device__ __forceinline__ double product(bool integer, double x, const Weight &w) {
   return integer ? mul_rn(x, w) : __dmul_rn(x, w.v);
 }

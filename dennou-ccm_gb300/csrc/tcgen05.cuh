@@ -94,7 +94,7 @@ __device__ __forceinline__ void tmem_ld16_nw(uint32_t taddr, uint32_t (&r)[16]) 
       : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// Named barrier of the four epilogue warps (threads 64..191).
+// Named barrier of the mixed kernel's epilogue warps (NTHREADS threads from 64 on).
 template <int NTHREADS> __device__ __forceinline__ void epi_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(NTHREADS) : "memory");
 }

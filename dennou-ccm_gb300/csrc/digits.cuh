@@ -24,14 +24,14 @@ __device__ __forceinline__ int dg_exp(unsigned maxmag) {
   return e < 1 ? 1 : e;
 }
 
-// Q of x for scale exponent E (at least that of the vector), with 256 added
-// to every digit so that they come off as plain bit fields.
+// Q of x for scale exponent E (at least that of the vector; 0 for an x beyond
+// it), with 256 added to every digit so that they come off as plain bit fields.
 __device__ __forceinline__ unsigned long long dg_fixed(double x, int E) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const int ef = (int)(b >> 52) & 0x7FF;
   // the 53-bit mantissa at bits 10 .. 62, moved down by E - ef + 1, rounded
   const unsigned long long m = ((b << 10) & 0x3FFFFFFFFFFFFC00ull) | (ef ? 1ull << 62 : 0ull);
-  const int r = min(E - max(ef, 1), 63);  // at 63 nothing is left
+  const unsigned r = min((unsigned)(E - max(ef, 1)), 63u);  // at 63 nothing is left
   const unsigned long long q = ((m >> r) + 1ull) >> 1;
   constexpr unsigned long long BIAS =
       256ull * (1ull + (1ull << 9) + (1ull << 18) + (1ull << 27) + (1ull << 36) + (1ull << 45) + (1ull << 54));

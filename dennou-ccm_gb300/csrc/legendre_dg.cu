@@ -477,6 +477,9 @@ dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const doub
     else if constexpr (LAY == SPEC_DOUBLES) return make_double2(__ldg(src + 2 * (n - m)), __ldg(src + 2 * (n - m) + 1));
     else return __ldg(reinterpret_cast<const double2 *>(src) + (n - m));
   };
+  // Im s_n^0 does not enter the synthesis, whatever it holds: not the scale
+  // either (its digits are then any, and its column is not read)
+  const unsigned im_mag = m ? 0x7FFFFFFFu : 0u;
   const int nu = 4 * max(nq0, nq1);  // units of 8 a parity, both parities side by side
   unsigned mx = 0;
   double2 v[8];
@@ -485,7 +488,7 @@ dg_pack_spec(const DgMInfo *__restrict__ mi_, int N, long long ncoef, const doub
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       v[e] = live && n0 + 2 * e <= N ? coefficient(n0 + 2 * e) : make_double2(0.0, 0.0);
-      mx = max(mx, max(dg_mag(v[e].x), dg_mag(v[e].y)));
+      mx = max(mx, max(dg_mag(v[e].x), (unsigned)__double2hiint(v[e].y) & im_mag));
     }
   }
 #pragma unroll
